@@ -161,13 +161,15 @@ int mpkg_plan_wave_ctas(int n, const int *ptr, const int *col, const double *val
  * (l*N + row0[m]) * nrhs, row0[m] = n[0] + ... + n[m-1], each row's nrhs
  * values contiguous; level 0 is the input.  Entries are accumulated with
  * FP32 FMA in CSR order.  tune = MPKG_BATCH_TUNE times every kernel
- * configuration (lanes per row x vector width, L2 group size, CTAs per SM,
- * and for nrhs a multiple of 4 the kernel that stages each CTA's window of
- * the previous level in shared memory) on these matrices at plan time and
- * keeps the fastest; MPKG_BATCH_DEFAULT takes the first configuration
- * untimed, MPKG_BATCH_STAGED / MPKG_BATCH_STAGED2 / MPKG_BATCH_STAGED4 the
- * staged kernel at one, two or four CTAs per SM untimed (EINVAL when nrhs
- * is not a multiple of 4).  All configurations give the same bits. */
+ * configuration (lanes per row x vector width, group size, CTAs per SM, and
+ * for nrhs a multiple of 4 the kernel that stages each CTA's window of the
+ * previous level, and the packed matrix, in shared memory) on these matrices
+ * at plan time and keeps the fastest; MPKG_BATCH_DEFAULT takes one untimed:
+ * the staged kernel at one CTA per SM when nrhs is a multiple of 4 and its
+ * windows reach three quarters of the entries, else the CSR kernel;
+ * MPKG_BATCH_STAGED / MPKG_BATCH_STAGED2 / MPKG_BATCH_STAGED4 the staged
+ * kernel at one, two or four CTAs per SM untimed (EINVAL when nrhs is not a
+ * multiple of 4).  All configurations give the same bits. */
 enum {
   MPKG_BATCH_DEFAULT = 0,
   MPKG_BATCH_TUNE = 1,

@@ -21,6 +21,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -1703,20 +1704,51 @@ inline TmKernel tm_kernel_ptr(int value_type, int w) {
 // lanes, each holding VW consecutive right-hand sides (vector loads);
 // entries are accumulated with single-precision FMA in CSR order.
 // ------------------------------------------------------------------------
+// A (group, CTA) unit of the packed batched form.  Its blob, for nw warps:
+// per warp its first slice (nw + 1) and the first chunk of its stream
+// (nw + 1), the slices' pairs, the slices' row ids (-1: none), padded to 16
+// bytes (`head`), then the streams of entries in whole chunks.  Shared memory
+// holds the zero row, the warps' rings (not in the resident form), the
+// window and the staged part of the blob.
+struct BatchUnit {
+  int nslice;
+  int blob16;         // start of the blob, in 16-byte words
+  int head;           // bytes
+  int head_at;        // its place in shared memory, past the window
+  int staged;         // bytes of the blob in shared memory: the head (resident form: and the streams), or 0
+  int iv0, ivh, iv1;  // window intervals: the CTA's own rows, then its neighbours'
+  int win_rows;       // rows of the window
+};
+
+constexpr int kBatchIntervals = 32;  // intervals of columns (a bulk copy each; one across the own rows is cut in up to three)
+constexpr int kBatchZero = 512;      // bytes of shared memory for the zero row
+
 struct BatchArgs {
   long N;                      // rows of all matrices
   int nrhs, nlevel, nblk, ngroup;
-  uint32_t base, stall;
+  uint32_t stall;
   const int *ptr, *col;        // block-diagonal CSR (global columns)
   const float *val;
   float *vb;                   // (nlevel + 1) * N * nrhs, level 0 = input
   const int *row_lo;           // ngroup * (nblk + 1)
   const int *dep_ptr;          // ngroup * nblk + 1: CTA b of group g waits for
   const int *dep_idx;          // dep_idx[dep_ptr[g*nblk+b] ..), the other CTAs owning its columns
-  unsigned int *flags;
+  unsigned int *flags;         // per CTA: last level published, on from the call before (modulo 2^32)
   int *err;
-  const int *win;              // staged form: ngroup * nblk pairs [w0, w1) of previous-level rows in smem
+  // packed form (batch_pack_kernel), per (group, CTA) u = g * nblk + b:
+  const BatchUnit *unit;
+  const int4 *iv;              // window intervals: first row, rows, byte offset in shared memory
+  const unsigned char *blob;   // the units' heads and streams
 };
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void cp_async_wait_group() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
 
 template <int VW>
 struct VecF;
@@ -1753,16 +1785,17 @@ __global__ void __launch_bounds__(256) batch_kernel(BatchArgs a) {
   __syncthreads();
   const int b = blockIdx.x, nrhs = LPR * VW;
   const int lane = (int)threadIdx.x % LPR, rpp = (int)blockDim.x / LPR;
+  const unsigned base = a.flags[b];  // where the last call left every flag
   for (int g = 0; g < a.ngroup; g++) {
     const int r0 = a.row_lo[(size_t)g * (a.nblk + 1) + b], r1 = a.row_lo[(size_t)g * (a.nblk + 1) + b + 1];
-    const unsigned tag = a.base + (unsigned)g * (unsigned)(a.nlevel + 1);
+    const unsigned tag = base + (unsigned)g * (unsigned)(a.nlevel + 1);
     const int dlo = a.dep_ptr[(size_t)g * a.nblk + b], dhi = a.dep_ptr[(size_t)g * a.nblk + b + 1];
     for (int l = 1; l <= a.nlevel; l++) {
       if (l > 1) {  // the CTAs owning this range's columns have published level l-1 of group g
         for (int k = dlo + (int)threadIdx.x; k < dhi; k += blockDim.x) {
           const int c = a.dep_idx[k];
           long spins = 0;
-          while (ld_acquire(a.flags + c) < tag + (unsigned)(l - 1) + a.stall) {
+          while ((int)(ld_acquire(a.flags + c) - (tag + (unsigned)(l - 1) + a.stall)) < 0) {
             if (++spins > kSpinLimit || *((volatile int *)a.err)) {
               atomicCAS(a.err, 0, kErrTimeout);
               s_abort = 1;
@@ -1814,41 +1847,109 @@ __global__ void __launch_bounds__(256) batch_kernel(BatchArgs a) {
       }
     }
   }
+  if (threadIdx.x == 0) a.flags[b] = base + (unsigned)a.ngroup * (unsigned)(a.nlevel + 1);
 }
 
-// The batched rows with the previous level staged in shared memory.  Per
-// (group, level) the CTA copies rows [w0, w1) of the previous level (its
-// own rows and the halo its columns reach, as far as the window holds)
-// with one bulk copy on an mbarrier; an entry whose column falls in the
-// window reads shared memory, any other reads global memory through the
-// same generic load.  Rows of the window that no row of the CTA reads may
-// be stale: they are never used.  Same rows, CSR order and FMAs as
-// batch_kernel, so the same bits.
-template <int LPR, int VW>
-__global__ void __launch_bounds__(1024) batch_stage_kernel(BatchArgs a) {
-  extern __shared__ __align__(128) float bs_win[];
+// The batched rows with the previous level in shared memory and the matrix
+// streamed past it.  Per (group, level) the CTA copies the rows of the
+// previous level that its columns reach (up to kBatchIntervals intervals of
+// rows, a bulk copy each) into its window, then computes its rows in slices
+// of 32 / LPR rows, LPR lanes of four right-hand sides per row.  The CTA's
+// rows are sorted by length, so the rows of a slice advance together, and an
+// entry is a (value, byte offset of its column's row in shared memory) pair,
+// two entries to a 16-byte word, [pair][row] within a slice.  Every warp has
+// its slices, dealt out in equal shares, and their entries as one stream:
+// per two entries one shared-memory load, per entry one for its vector row
+// and four FMAs.  When every CTA has room for its streams (RES) they are
+// copied once per call with the head, in one bulk copy; else each warp copies
+// its stream at every level through a ring of its own (cp.async, kBpRing
+// chunks in flight, started before the wait for the neighbours).
+// Padding is (-0, the zero row): fma(-0, +0, s) = s exactly, so the sums are
+// batch_kernel's FP32 FMA chains in CSR order, bit for bit.  Slices with a
+// column outside the window (bit 31 of the offset, then the column itself)
+// read it from global memory.  Window rows that no row of the CTA reads may
+// be stale: they are never used.
+//
+// What bounds it: the shared-memory pipe (128 bytes a clock and SM).  Per two
+// entries of 8 rows at 16 right-hand sides a warp takes 2 of its cycles for
+// the entry words, 8 for the vector rows (more where two rows of a quarter
+// warp meet in their banks, which the plan keeps rare) and 1 for the copy in.
+// 48 matrices (stencils and random banded, 375 K rows, 4.8 M entries), 16
+// right-hand sides, 6 levels: 138 us at four CTAs per SM, 134 at one or two,
+// against 220 for the CSR rows read from L2 into the same window; 6 matrices
+// of 300-3000 rows, 4 right-hand sides, 4 levels (resident): 21 against 47.
+// Two ring chunks measure as three do (139 and 142 us at two CTAs per SM)
+// and leave room for one group instead of two at four CTAs (142 and 167).
+constexpr int kBpRing = 2;  // chunks in flight per warp
+__host__ __device__ constexpr int bp_chunk_pairs(int lpr) { return lpr == 1 ? 2 : lpr == 2 ? 4 : lpr; }
+__host__ __device__ constexpr int bp_chunk_bytes(int lpr) { return bp_chunk_pairs(lpr) * (32 / lpr) * 16; }
+
+template <int LPR, bool RES>
+__global__ void __launch_bounds__(1024) batch_pack_kernel(BatchArgs a) {
+  extern __shared__ __align__(128) unsigned char bp_smem[];
   __shared__ int s_abort;
-  __shared__ __align__(8) unsigned long long s_bar;
+  __shared__ __align__(8) unsigned long long s_bar_w, s_bar_m;
+  constexpr int kRows = 32 / LPR;  // rows per slice
+  constexpr int kPairs = bp_chunk_pairs(LPR), kChunk = bp_chunk_bytes(LPR);
+  constexpr int nrhs = LPR * 4;
   if (threadIdx.x == 0) {
     s_abort = 0;
-    mbar_init(&s_bar);
+    mbar_init(&s_bar_w);
+    mbar_init(&s_bar_m);
   }
+  if (threadIdx.x < nrhs) reinterpret_cast<float *>(bp_smem)[threadIdx.x] = 0.f;  // the zero row
   __syncthreads();
-  unsigned phase = 0;
-  const int b = blockIdx.x, nrhs = LPR * VW;
-  const int lane = (int)threadIdx.x % LPR, rpp = (int)blockDim.x / LPR;
+  unsigned phase_w = 0, phase_m = 0;
+  const int b = blockIdx.x;
+  const unsigned base = a.flags[b];  // where the last call left every flag
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int rl = lane / LPR, ch = lane % LPR;
+  const unsigned char *wl = bp_smem + 16 * ch;
+  unsigned char *ring = bp_smem + kBatchZero + warp * kBpRing * kChunk;
   for (int g = 0; g < a.ngroup; g++) {
-    const int r0 = a.row_lo[(size_t)g * (a.nblk + 1) + b], r1 = a.row_lo[(size_t)g * (a.nblk + 1) + b + 1];
-    const unsigned tag = a.base + (unsigned)g * (unsigned)(a.nlevel + 1);
-    const int dlo = a.dep_ptr[(size_t)g * a.nblk + b], dhi = a.dep_ptr[(size_t)g * a.nblk + b + 1];
-    const int w0 = a.win[2 * ((size_t)g * a.nblk + b)], w1 = a.win[2 * ((size_t)g * a.nblk + b) + 1];
-    const unsigned wn = (unsigned)(w1 - w0);
+    const size_t u = (size_t)g * a.nblk + b;
+    const BatchUnit un = a.unit[u];
+    if (un.nslice == 0) continue;  // no rows here: nobody waits for this CTA
+    const unsigned tag = base + (unsigned)g * (unsigned)(a.nlevel + 1);
+    const int dlo = a.dep_ptr[u], dhi = a.dep_ptr[u + 1];
+    const unsigned char *blob = a.blob + 16 * (size_t)un.blob16;
+    unsigned char *head_s = bp_smem + un.head_at;
+    const int *head = reinterpret_cast<const int *>(un.staged ? head_s : blob);
+    if (un.staged) {  // warp ranges, slice lengths and row ids (RES: the streams too), once per group
+      if (threadIdx.x == 0) {
+        asm volatile("fence.proxy.async;" ::: "memory");
+        mbar_expect(&s_bar_m, (unsigned)un.staged);
+        bulk_g2s(head_s, blob, (unsigned)un.staged, &s_bar_m);
+      }
+      if (!tr_wait(&s_bar_m, phase_m, a.err)) return;
+      phase_m ^= 1u;
+    }
+    const int sl0 = head[warp], sl1 = head[warp + 1];
+    const int ch0 = head[nw + 1 + warp], nch = head[nw + 2 + warp] - ch0;  // chunks of this warp's stream
+    const int *pairs = head + 2 * (nw + 1);
+    const int *ids = pairs + un.nslice;
+    const unsigned char *stream = blob + un.head + (size_t)ch0 * kChunk + 16 * lane;
+    if (RES) ring = head_s + un.head + ch0 * kChunk;
+    auto fetch = [&](int c, int slot) {
+      if (RES) return;
+      if (c < nch) {
+#pragma unroll
+        for (int t = 0; t < kChunk / 512; t++)
+          cp_async16(ring + slot * kChunk + 512 * t + 16 * lane, stream + (size_t)c * kChunk + 512 * t);
+      }
+      cp_async_commit();
+    };
+    auto copy = [&](const float *src, const int4 iv) {  // first row, rows, byte offset in shared memory
+      bulk_g2s(bp_smem + iv.z, src + (size_t)iv.x * nrhs, (unsigned)iv.y * (unsigned)nrhs * 4u, &s_bar_w);
+    };
+#pragma unroll
+    for (int c = 0; c < kBpRing; c++) fetch(c, c);
     for (int l = 1; l <= a.nlevel; l++) {
       if (l > 1) {  // the CTAs owning this range's columns have published level l-1 of group g
         for (int k = dlo + (int)threadIdx.x; k < dhi; k += blockDim.x) {
           const int c = a.dep_idx[k];
           long spins = 0;
-          while (ld_acquire(a.flags + c) < tag + (unsigned)(l - 1) + a.stall) {
+          while ((int)(ld_acquire(a.flags + c) - (tag + (unsigned)(l - 1) + a.stall)) < 0) {
             if (++spins > kSpinLimit || *((volatile int *)a.err)) {
               atomicCAS(a.err, 0, kErrTimeout);
               s_abort = 1;
@@ -1858,62 +1959,94 @@ __global__ void __launch_bounds__(1024) batch_stage_kernel(BatchArgs a) {
           }
         }
         __syncthreads();
-        if (s_abort) return;
+        if (s_abort) {
+          cp_async_wait_all();
+          return;
+        }
       }
       const float *src = a.vb + (size_t)(l - 1) * a.N * nrhs;
-      if (wn > 0) {
-        if (threadIdx.x == 0) {
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier reads of the window first
-          const unsigned bytes = wn * (unsigned)nrhs * 4u;
-          mbar_expect(&s_bar, bytes);
-          bulk_g2s(bs_win, src + (size_t)w0 * nrhs, bytes, &s_bar);
+      if (un.iv1 > un.iv0) {
+        if (warp == 0) {
+          // the CTA's reads of the window and the acquired rows come before
+          // the copies (generic before async proxy)
+          asm volatile("fence.proxy.async;" ::: "memory");
+          if (l == 1 && lane == 0) mbar_expect(&s_bar_w, (unsigned)un.win_rows * (unsigned)nrhs * 4u);
+          __syncwarp();
+          for (int k = (l == 1 ? un.iv0 : un.ivh) + lane; k < un.iv1; k += 32) copy(src, a.iv[k]);
         }
-        if (!tr_wait(&s_bar, phase, a.err)) return;
-        phase ^= 1u;
+        if (!tr_wait(&s_bar_w, phase_w, a.err)) {
+          cp_async_wait_all();
+          return;
+        }
+        phase_w ^= 1u;
       }
-      const float *gl = src + lane * VW;
-      const float *wl = bs_win + lane * VW;
-      float *dst = a.vb + (size_t)l * a.N * nrhs + lane * VW;
-      for (int i = r0 + (int)threadIdx.x / LPR; i < r1; i += rpp) {
-        float acc[VW];
-#pragma unroll
-        for (int u = 0; u < VW; u++) acc[u] = 0.0f;
-        const int q0 = __ldg(a.ptr + i), q1 = __ldg(a.ptr + i + 1);
-        int q = q0;
-        for (; q + 4 <= q1; q += 4) {
-          const float *xp[4];
-          float v[4], xv[4][VW];
-#pragma unroll
-          for (int u = 0; u < 4; u++) {
-            const int c = __ldg(a.col + q + u);
-            v[u] = __ldg(a.val + q + u);
-            const unsigned o = (unsigned)(c - w0);
-            xp[u] = o < wn ? wl + (size_t)o * nrhs : gl + (size_t)c * nrhs;
+      const float *gl = src + 4 * ch;
+      float *dst = a.vb + (size_t)l * a.N * nrhs + 4 * ch;
+      int c = 0, slot = 0, in = 0;  // chunk of the stream, its ring slot, pairs of it used
+      const unsigned char *e = ring + rl * 16;
+      for (int sl = sl0; sl < sl1; sl++) {
+        const int np = pairs[sl];  // negative: a column outside the window
+        const int row = ids[sl * kRows + rl];
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        auto mac = [&](unsigned vbits, const float4 &x) {
+          const float v = __uint_as_float(vbits);
+          acc.x = __fmaf_rn(v, x.x, acc.x);
+          acc.y = __fmaf_rn(v, x.y, acc.y);
+          acc.z = __fmaf_rn(v, x.z, acc.z);
+          acc.w = __fmaf_rn(v, x.w, acc.w);
+        };
+        for (int left = abs(np); left > 0; left--) {
+          if (!RES && in == 0) {  // a new chunk: its copies are done, and the other lanes' too
+            cp_async_wait_group<kBpRing - 1>();
+            __syncwarp();
           }
-#pragma unroll
-          for (int u = 0; u < 4; u++) VecF<VW>::ld(xp[u], xv[u]);
-#pragma unroll
-          for (int u = 0; u < 4; u++)
-#pragma unroll
-            for (int w = 0; w < VW; w++) acc[w] = __fmaf_rn(v[u], xv[u][w], acc[w]);
+          const uint4 w = *reinterpret_cast<const uint4 *>(e);
+          float4 x0, x1;
+          if (np >= 0) {
+            x0 = *reinterpret_cast<const float4 *>(wl + w.y);
+            x1 = *reinterpret_cast<const float4 *>(wl + w.w);
+          } else {
+            x0 = (int)w.y < 0 ? *reinterpret_cast<const float4 *>(gl + (size_t)(w.y & 0x7FFFFFFFu) * nrhs)
+                              : *reinterpret_cast<const float4 *>(wl + w.y);
+            x1 = (int)w.w < 0 ? *reinterpret_cast<const float4 *>(gl + (size_t)(w.w & 0x7FFFFFFFu) * nrhs)
+                              : *reinterpret_cast<const float4 *>(wl + w.w);
+          }
+          e += kRows * 16;
+          mac(w.x, x0);
+          mac(w.z, x1);
+          if (!RES && ++in == kPairs) {  // the chunk is used up: the next one of its slot
+            __syncwarp();
+            fetch(c + kBpRing, slot);
+            c++;
+            slot++;
+            in = 0;
+            if (slot == kBpRing) {
+              slot = 0;
+              e = ring + rl * 16;
+            }
+          }
         }
-        for (; q < q1; q++) {
-          float x0[VW];
-          const int c = __ldg(a.col + q);
-          const float v0 = __ldg(a.val + q);
-          const unsigned o = (unsigned)(c - w0);
-          VecF<VW>::ld(o < wn ? wl + (size_t)o * nrhs : gl + (size_t)c * nrhs, x0);
+        if (row >= 0) __stcs(reinterpret_cast<float4 *>(dst + (size_t)row * nrhs), acc);
+      }
+      if (l < a.nlevel) {  // the next level's first chunks
+        __syncwarp();
 #pragma unroll
-          for (int u = 0; u < VW; u++) acc[u] = __fmaf_rn(v0, x0[u], acc[u]);
-        }
-        VecF<VW>::st(dst + (size_t)i * nrhs, acc);
+        for (int t = 0; t < kBpRing; t++) fetch(t, t);
       }
       __syncthreads();  // rows written and the window read; the release store is cumulative
       if (threadIdx.x == 0) {
         asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.flags + b), "r"(tag + (unsigned)l) : "memory");
+        if (l < a.nlevel && un.iv1 > un.iv0) {
+          // the next level's own rows, while the neighbours finish theirs:
+          // the release above has ordered the CTA's writes before the copies
+          asm volatile("fence.proxy.async;" ::: "memory");
+          mbar_expect(&s_bar_w, (unsigned)un.win_rows * (unsigned)nrhs * 4u);
+          for (int k = un.iv0; k < un.ivh; k++) copy(a.vb + (size_t)l * a.N * nrhs, a.iv[k]);
+        }
       }
     }
   }
+  if (threadIdx.x == 0) a.flags[b] = base + (unsigned)a.ngroup * (unsigned)(a.nlevel + 1);
 }
 
 // One pdmpk batch of every rank (Buffers::DoComp, pdmpk/buffers.cc:76-97):
@@ -2071,8 +2204,11 @@ struct mpkg_plan {
   BatchArgs batch{};
   int batch_lpr = 0, batch_vw = 0, batch_nmat = 0;
   int batch_threads = 256;   // CTA size of the persistent launch
-  bool batch_staged = false; // batch_stage_kernel: previous level windowed in shared memory
+  bool batch_staged = false; // batch_pack_kernel: previous level windowed in shared memory
+  bool batch_resident = false;  // ... and the matrix in shared memory for the whole call
   size_t batch_smem = 0;     // its window bytes per CTA
+  std::vector<void *> batch_owned;  // device arrays of the current configuration
+  long batch_bytes = 0;             // ... and their size, part of device_bytes
   long batch_group_bytes = 0;
   double batch_tune_ms = 0.0;
   int batch_candidates = 0;
@@ -2369,16 +2505,15 @@ typedef void (*BatchKernel)(BatchArgs);
 
 BatchKernel batch_kernel_for(int lpr, int vw) {
 #define MPKG_BK(L, V) if (lpr == L && vw == V) return batch_kernel<L, V>;
-  MPKG_BK(1, 1) MPKG_BK(2, 1) MPKG_BK(4, 1) MPKG_BK(8, 1) MPKG_BK(16, 1) MPKG_BK(32, 1)
-  MPKG_BK(1, 2) MPKG_BK(2, 2) MPKG_BK(4, 2) MPKG_BK(8, 2) MPKG_BK(16, 2) MPKG_BK(32, 2)
+  MPKG_BK(1, 1) MPKG_BK(2, 1) MPKG_BK(1, 2)
   MPKG_BK(1, 4) MPKG_BK(2, 4) MPKG_BK(4, 4) MPKG_BK(8, 4) MPKG_BK(16, 4) MPKG_BK(32, 4)
 #undef MPKG_BK
   return nullptr;
 }
 
-BatchKernel batch_stage_kernel_for(int lpr, int vw) {
-#define MPKG_BK(L, V) if (lpr == L && vw == V) return batch_stage_kernel<L, V>;
-  MPKG_BK(1, 4) MPKG_BK(2, 4) MPKG_BK(4, 4) MPKG_BK(8, 4) MPKG_BK(16, 4) MPKG_BK(32, 4)
+BatchKernel batch_pack_kernel_for(int lpr, bool resident) {
+#define MPKG_BK(L) if (lpr == L) return resident ? batch_pack_kernel<L, true> : batch_pack_kernel<L, false>;
+  MPKG_BK(1) MPKG_BK(2) MPKG_BK(4) MPKG_BK(8) MPKG_BK(16) MPKG_BK(32)
 #undef MPKG_BK
   return nullptr;
 }
@@ -2391,96 +2526,396 @@ struct BatchHost {
   std::vector<long> mat_row0;  // nmat + 1
 };
 
+// A batch configuration's CTA row ranges, dependencies and, for the packed
+// form, the packed matrix.
+struct BatchLayout {
+  int ngroup = 0;
+  std::vector<int> row_lo, dptr, didx;
+  std::vector<BatchUnit> unit;
+  std::vector<int4> iv;
+  std::unique_ptr<uint4[]> blob;
+  size_t blob_words = 0;
+  long far = 0;          // entries outside their CTA's window
+  bool resident = false; // every unit's streams have room beside its window
+};
+
+// Runs fn(0..count-1) on all host threads, the caller's among them; false
+// when a call threw (out of memory).
+template <typename F>
+bool host_parallel(int count, F &&fn) {
+  const int nth = (int)std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+  std::atomic<int> next{0};
+  std::atomic<bool> ok{true};
+  auto work = [&] {
+    try {
+      for (int q; ok && (q = next.fetch_add(1)) < count;) fn(q);
+    } catch (const std::exception &) {
+      ok = false;
+    }
+  };
+  std::vector<std::thread> pool;
+  try {
+    for (int t = 1; t < nth && t < count; t++) pool.emplace_back(work);
+  } catch (const std::exception &) {  // no more threads: the caller's thread does the rest
+  }
+  work();
+  for (auto &th : pool) th.join();
+  return ok;
+}
+
 // Groups of consecutive matrices within `budget` bytes (matrix + two
 // levels of vectors); per group, CTA row ranges of equal nonzeros and the
-// CTAs owning each range's columns.  With cap_rows > 0, also each (group,
-// CTA)'s window [w0, w1) of previous-level rows for shared memory: the span
-// of its columns when that fits cap_rows rows, else cap_rows rows around
-// its own rows (columns beyond are read from global memory).
-void batch_layout(const BatchHost &h, int nrhs, long budget, int grid, long cap_rows, std::vector<int> *row_lo,
-                  std::vector<int> *dptr, std::vector<int> *didx, std::vector<int> *win, int *ngroup) {
+// CTAs owning each range's columns.  A group of fewer rows than the grid
+// has row slots (`threads` / lpr per CTA) takes fewer CTAs, so that each has
+// one pass of its threads: a level costs a hand-over between CTAs whatever
+// its size, and matrices of up to two passes stay whole, with none.
+int batch_ranges(const BatchHost &h, int nrhs, long budget, bool windows, int grid, int threads, int lpr,
+                 BatchLayout *out) {
   const int nmat = (int)h.mat_row0.size() - 1;
-  std::vector<long> g0(1, 0);
+  std::vector<int> g0(1, 0);  // first matrix of each group
   long bytes = 0;
+  if (windows) {  // groups of equal size
+    const long total = h.N * (4L * nrhs + 5);
+    budget = std::min(budget, (long)(1.03 * total / ((total + budget - 1) / budget)));
+  }
   for (int m = 0; m < nmat; m++) {
     const long r0 = h.mat_row0[m], r1 = h.mat_row0[m + 1];
-    const long mb = (long)(h.ptr[r1] - h.ptr[r0]) * 8 + (r1 - r0) * (4 + 8L * nrhs);
+    const long mb = windows ? (r1 - r0) * (4L * nrhs + 5)  // a level's rows, their ids and lengths
+                            : (long)(h.ptr[r1] - h.ptr[r0]) * 8 + (r1 - r0) * (4 + 8L * nrhs);
     if (bytes > 0 && bytes + mb > budget) {
-      g0.push_back(r0);
+      g0.push_back(m);
       bytes = 0;
     }
     bytes += mb;
   }
-  g0.push_back(h.N);
-  *ngroup = (int)g0.size() - 1;
-  row_lo->assign((size_t)*ngroup * (grid + 1), 0);
-  dptr->assign((size_t)*ngroup * grid + 1, 0);
-  win->assign((size_t)*ngroup * grid * 2, 0);
-  didx->clear();
-  std::vector<int> seen(grid, -1);
-  for (int g = 0; g < *ngroup; g++) {
-    int *lo = row_lo->data() + (size_t)g * (grid + 1);
-    const long a = g0[g], z = g0[g + 1];
-    const long q0 = h.ptr[a], nz = h.ptr[z] - q0;
-    lo[0] = (int)a;
-    for (int b = 1; b < grid; b++) {
-      const long target = q0 + nz * b / grid;
-      const int r = (int)(std::lower_bound(h.ptr.begin() + a, h.ptr.begin() + z + 1, (int)target) - h.ptr.begin());
-      lo[b] = std::max(std::min(r, (int)z), lo[b - 1]);
+  g0.push_back(nmat);
+  const int ng = out->ngroup = (int)g0.size() - 1;
+  out->row_lo.assign((size_t)ng * (grid + 1), 0);
+  // a row's share of a CTA's time: its entries, and kRowCost entries' time
+  // for its slice header, store and first loads
+  const long kRowCost = windows ? 8 : 0;
+  auto work = [&](long r) { return (long)h.ptr[r] + kRowCost * r; };
+  auto row_at = [&](long target, long a, long z) {  // the first row in [a, z] with at least that work before it
+    long lo = a, hi = z;
+    while (lo < hi) {
+      const long mid = (lo + hi) / 2;
+      if (work(mid) < target) lo = mid + 1;
+      else hi = mid;
     }
-    lo[grid] = (int)z;
-    // the exact set of other CTAs whose rows CTA b reads (its own rows of
-    // the previous level are ordered by its barrier)
+    return lo;
+  };
+  for (int g = 0; g < ng; g++) {
+    int *lo = out->row_lo.data() + (size_t)g * (grid + 1);
+    const long a = h.mat_row0[g0[g]], z = h.mat_row0[g0[g + 1]];
+    const long pass = std::max(1, threads / lpr);  // rows of one pass
+    std::vector<long> cut(1, a);
+    if (z - a <= pass * grid) {
+      for (int m = g0[g]; m < g0[g + 1]; m++) {
+        const long r0 = h.mat_row0[m], r1 = h.mat_row0[m + 1];
+        const long parts = r1 - r0 <= 2 * pass ? 1 : (r1 - r0 + pass - 1) / pass;
+        const long q0 = work(r0), nz = work(r1) - q0;
+        for (long t = 1; t < parts; t++) cut.push_back(std::max(std::min(row_at(q0 + nz * t / parts, r0, r1), r1), cut.back()));
+        cut.push_back(r1);
+      }
+    }
+    if (cut.size() == 1 || (long)cut.size() > grid + 1) {  // equal nonzeros over the whole grid
+      cut.assign(1, a);
+      const long q0 = work(a), nz = work(z) - q0;
+      for (int b = 1; b < grid; b++) cut.push_back(std::max(std::min(row_at(q0 + nz * b / grid, a, z), z), cut.back()));
+      cut.push_back(z);
+    }
+    for (int b = 0; b <= grid; b++) lo[b] = (int)cut[std::min<size_t>(b, cut.size() - 1)];
+  }
+  // the exact set of other CTAs whose rows CTA b reads (its own rows of
+  // the previous level are ordered by its barrier)
+  std::vector<std::vector<int>> dep((size_t)ng * grid);
+  const bool ok = host_parallel(ng, [&](int g) {
+    const int *lo = out->row_lo.data() + (size_t)g * (grid + 1);
+    std::vector<int> seen(grid, -1);
     for (int b = 0; b < grid; b++) {
-      const size_t u = (size_t)g * grid + b;
-      const size_t first = didx->size();
+      std::vector<int> &d = dep[(size_t)g * grid + b];
       for (long q = h.ptr[lo[b]]; q < h.ptr[lo[b + 1]]; q++) {
         const int c = h.col[q];
         if (c >= lo[b] && c < lo[b + 1]) continue;
         const int o = (int)(std::upper_bound(lo, lo + grid, c) - lo) - 1;  // last CTA starting at or before c
-        if (seen[o] != (int)u) { seen[o] = (int)u; didx->push_back(o); }
+        if (seen[o] != b) { seen[o] = b; d.push_back(o); }
       }
-      std::sort(didx->begin() + first, didx->end());
-      (*dptr)[u + 1] = (int)didx->size();
-      if (cap_rows > 0 && lo[b + 1] > lo[b]) {
-        long cmin = lo[b], cmax = lo[b + 1] - 1;
-        for (long q = h.ptr[lo[b]]; q < h.ptr[lo[b + 1]]; q++) {
-          cmin = std::min<long>(cmin, h.col[q]);
-          cmax = std::max<long>(cmax, h.col[q]);
-        }
-        long w0 = cmin, w1 = cmax + 1;
-        if (w1 - w0 > cap_rows) {  // around the own rows, within the column span
-          const long own = lo[b + 1] - lo[b];
-          w0 = own >= cap_rows ? lo[b] : std::max(cmin, lo[b] - (cap_rows - own) / 2);
-          w1 = std::min(cmax + 1, w0 + cap_rows);
-          w0 = std::max(cmin, w1 - cap_rows);
-        }
-        (*win)[2 * u] = (int)w0;
-        (*win)[2 * u + 1] = (int)w1;
-      }
+      std::sort(d.begin(), d.end());
     }
-    std::fill(seen.begin(), seen.end(), -1);
+  });
+  if (!ok) return fail(kENoMem, "batch layout");
+  out->dptr.assign((size_t)ng * grid + 1, 0);
+  out->didx.clear();
+  for (size_t u = 0; u < dep.size(); u++) {
+    out->didx.insert(out->didx.end(), dep[u].begin(), dep[u].end());
+    out->dptr[u + 1] = (int)out->didx.size();
   }
-  if (didx->empty()) didx->push_back(0);
+  if (out->didx.empty()) out->didx.push_back(0);
+  return kOk;
 }
 
-int batch_launch_raw(mpkg_plan *p, float *d_vb, cudaStream_t st, bool capture) {
+// The window of one (group, CTA): the rows its columns reach as at most
+// kBatchIntervals intervals of at most cap_rows rows together.  Columns at
+// most `gap` rows apart share an interval (one copy for several rows); when
+// the rows do not fit, the intervals nearest the CTA's own rows are kept and
+// the entries of the others read global memory.
+struct RowSpan { int lo, hi; };  // rows [lo, hi)
+void batch_window(const BatchHost &h, int r0, int r1, long cap_rows, std::vector<int> *cols, std::vector<RowSpan> *win) {
+  cols->clear();
+  win->clear();
+  for (long q = h.ptr[r0]; q < h.ptr[r1]; q++) cols->push_back(h.col[q]);
+  if (cols->empty()) return;
+  std::sort(cols->begin(), cols->end());
+  cols->erase(std::unique(cols->begin(), cols->end()), cols->end());
+  for (int gap : {32, 0}) {
+    win->clear();
+    long rows = 0;
+    for (int c : *cols) {
+      if (!win->empty() && c - win->back().hi <= gap) {
+        rows += c + 1 - win->back().hi;
+        win->back().hi = c + 1;
+      } else {
+        win->push_back({c, c + 1});
+        rows++;
+      }
+    }
+    while ((int)win->size() > kBatchIntervals) {  // close the narrowest gaps
+      std::vector<int> gaps;
+      for (size_t t = 1; t < win->size(); t++) gaps.push_back((*win)[t].lo - (*win)[t - 1].hi);
+      const size_t over = win->size() - kBatchIntervals;
+      std::nth_element(gaps.begin(), gaps.begin() + (over - 1), gaps.end());
+      const int most = gaps[over - 1];
+      size_t left = over, o = 0;
+      for (size_t t = 1; t < win->size(); t++) {
+        const int gp = (*win)[t].lo - (*win)[o].hi;
+        if (gp <= most && left > 0) {
+          rows += gp;
+          (*win)[o].hi = (*win)[t].hi;
+          left--;
+        } else {
+          (*win)[++o] = (*win)[t];
+        }
+      }
+      win->resize(o + 1);
+    }
+    if (rows <= cap_rows) return;
+  }
+  // too many rows: the nearest intervals, the last one cut towards the own rows
+  auto dist = [&](const RowSpan &w) { return (long)std::max(0, std::max(w.lo - (r1 - 1), r0 - (w.hi - 1))); };
+  std::stable_sort(win->begin(), win->end(), [&](const RowSpan &x, const RowSpan &y) { return dist(x) < dist(y); });
+  long room = cap_rows;
+  std::vector<RowSpan> keep;
+  for (RowSpan w : *win) {
+    if (room <= 0) break;
+    if (w.hi - w.lo > room) {
+      if (w.lo >= r0) w.hi = (int)(w.lo + room);
+      else if (w.hi <= r1) w.lo = (int)(w.hi - room);
+      else {  // around the own rows
+        const long mid = ((long)r0 + r1) / 2;
+        w.lo = (int)std::min<long>(std::max<long>(w.lo, mid - room / 2), w.hi - room);
+        w.hi = (int)(w.lo + room);
+      }
+    }
+    keep.push_back(w);
+    room -= w.hi - w.lo;
+  }
+  std::sort(keep.begin(), keep.end(), [](const RowSpan &x, const RowSpan &y) { return x.lo < y.lo; });
+  *win = keep;
+}
+
+// The packed form of a layout for CTAs of `threads` threads and `smem` bytes
+// of shared memory: windows, slices of rows sorted by length, and the units'
+// blobs (batch_pack_kernel).  `resident`: the resident form; out->resident
+// tells whether it fits (if not, the layout is not complete).
+int batch_pack(const BatchHost &h, int grid, int lpr, int threads, long smem, bool resident, BatchLayout *out) {
+  const int ng = out->ngroup, rps = 32 / lpr, nw = threads / 32;
+  const size_t nu = (size_t)ng * grid;
+  const long row_bytes = (long)lpr * 16;
+  const int cp = bp_chunk_pairs(lpr), cw = bp_chunk_bytes(lpr) / 16;  // pairs and 16-byte words of a chunk
+  const long base = kBatchZero + (resident ? 0 : (long)nw * kBpRing * bp_chunk_bytes(lpr));
+  struct Unit {
+    std::vector<int4> iv;              // window intervals, the own rows first
+    std::vector<unsigned> off;         // per entry of the unit's rows, in CSR order
+    std::vector<int> rows;             // longest first
+    std::vector<int> order;            // slices in stream order
+    std::vector<int> warp_sl, warp_ch; // per warp: first slice of `order`, first chunk
+    long far = 0;
+  };
+  std::vector<Unit> un(nu);
+  out->unit.assign(nu, BatchUnit{});
+  const int chunk = (int)std::min<size_t>(64, 1 + nu / 128);  // (group, CTA) units per task
+  const int ntask = (int)((nu + chunk - 1) / chunk);
+  auto pairs_of_row = [&](int i) { return (h.ptr[i + 1] - h.ptr[i] + 1) / 2; };
+  auto pairs_of = [&](const Unit &x, int sl) { return pairs_of_row(x.rows[(size_t)sl * rps]); };
+  std::atomic<bool> fits{true};
+  bool ok = host_parallel(ntask, [&](int t) {
+    std::vector<int> cols, sorted;
+    std::vector<RowSpan> win;
+    std::vector<int4> ivs;
+    for (size_t u = (size_t)t * chunk; u < std::min(nu, (size_t)(t + 1) * chunk); u++) {
+      const int *lo = out->row_lo.data() + (u / grid) * (grid + 1) + u % grid;
+      const int r0 = lo[0], r1 = lo[1];
+      Unit &x = un[u];
+      BatchUnit &d = out->unit[u];
+      if (r0 >= r1 || !fits) continue;
+      d.nslice = (r1 - r0 + rps - 1) / rps;
+      const long head = (4L * (2 * (nw + 1) + (long)d.nslice * (1 + rps)) + 15) / 16 * 16;
+      if (head > INT32_MAX) throw std::bad_alloc();
+      d.head = (int)head;
+      d.staged = resident || head <= (smem - base) / 4 ? (int)head : 0;
+      long pos = base;
+      batch_window(h, r0, r1, std::max(0L, (smem - base - d.staged) / row_bytes), &cols, &win);
+      auto add = [&](int a, int z) {
+        if (a >= z) return;
+        x.iv.push_back(make_int4(a, z - a, (int)pos, 0));
+        pos += (z - a) * row_bytes;
+        d.win_rows += z - a;
+      };
+      for (const RowSpan &w : win) add(std::max(w.lo, r0), std::min(w.hi, r1));
+      d.ivh = (int)x.iv.size();
+      for (const RowSpan &w : win) {
+        add(w.lo, std::min(w.hi, r0));
+        add(std::max(w.lo, r1), w.hi);
+      }
+      ivs = x.iv;
+      std::sort(ivs.begin(), ivs.end(), [](const int4 &p, const int4 &q) { return p.x < q.x; });
+      const long q0 = h.ptr[r0];
+      x.off.resize(h.ptr[r1] - q0);
+      for (size_t q = 0; q < x.off.size(); q++) {
+        const int c = h.col[q0 + q];
+        auto v = std::upper_bound(ivs.begin(), ivs.end(), c, [](int cc, const int4 &z) { return cc < z.x; });
+        if (v != ivs.begin() && c < v[-1].x + v[-1].y) {
+          x.off[q] = (unsigned)(v[-1].z + (c - v[-1].x) * row_bytes);
+        } else {
+          x.off[q] = 0x80000000u | (unsigned)c;
+          x.far++;
+        }
+      }
+      sorted.resize(r1 - r0);
+      for (int i = r0; i < r1; i++) sorted[i - r0] = i;
+      std::stable_sort(sorted.begin(), sorted.end(),
+                       [&](int i, int j) { return h.ptr[i + 1] - h.ptr[i] > h.ptr[j + 1] - h.ptr[j]; });
+      // a quarter warp reads `quad` rows at once, 128 bytes when they lie in
+      // different banks: of the next rows of the same length, each place
+      // takes the one whose entries meet the fewest of the places before it
+      const int quad = std::max(1, 8 / lpr);
+      auto meets = [&](int i, int j) {
+        const unsigned *p = x.off.data() + (h.ptr[i] - q0), *q = x.off.data() + (h.ptr[j] - q0);
+        const int len = std::min(h.ptr[i + 1] - h.ptr[i], h.ptr[j + 1] - h.ptr[j]);
+        int m = 0;
+        for (int e = 0; e < len; e++) m += p[e] != q[e] && ((p[e] ^ q[e]) & (unsigned)(16 * 8 - 16 * lpr) & 0x70u) == 0;
+        return m;
+      };
+      for (size_t k = 0; quad > 1 && k < sorted.size(); k++) {
+        const size_t first = k - k % quad;
+        if (k == first) continue;
+        size_t best = k;
+        int least = INT32_MAX;
+        for (size_t z = k; z < std::min(sorted.size(), k + 16) && pairs_of_row(sorted[z]) == pairs_of_row(sorted[k]); z++) {
+          int m = 0;
+          for (size_t y = first; y < k; y++) m += meets(sorted[y], sorted[z]);
+          if (m < least) {
+            least = m;
+            best = z;
+          }
+          if (m == 0) break;
+        }
+        std::rotate(sorted.begin() + k, sorted.begin() + best, sorted.begin() + best + 1);
+      }
+      x.rows = sorted;
+      // slices dealt to the warps forth and back, so that every warp has as
+      // many long ones as any other
+      x.warp_sl.push_back(0);
+      x.warp_ch.push_back(0);
+      for (int w = 0; w < nw; w++) {
+        long pairs = 0;
+        for (int r = 0; r * nw < d.nslice; r++) {
+          const int sl = r * nw + (r & 1 ? nw - 1 - w : w);
+          if (sl >= d.nslice) continue;
+          x.order.push_back(sl);
+          pairs += pairs_of(x, sl);
+        }
+        x.warp_sl.push_back((int)x.order.size());
+        x.warp_ch.push_back(x.warp_ch.back() + (int)((pairs + cp - 1) / cp));
+      }
+      d.head_at = (int)pos;
+      if (resident) {
+        const long bytes = head + 16L * cw * x.warp_ch.back();
+        if (pos + bytes > smem || x.far > 0) fits = false;
+        d.staged = (int)std::min<long>(bytes, smem);
+      }
+    }
+  });
+  out->resident = resident && fits;
+  if (ok && resident && !fits) return kOk;
+  if (!ok) return fail(kENoMem, "batch layout");
+  long total = 0;  // 16-byte words of all blobs
+  out->iv.clear();
+  for (size_t u = 0; u < nu; u++) {
+    BatchUnit &d = out->unit[u];
+    if (d.nslice == 0) continue;
+    d.blob16 = (int)total;
+    total += d.head / 16 + (long)un[u].warp_ch.back() * cw;
+    if (total > INT32_MAX) return fail(kERange, "packed batch exceeds 32 GB");
+    d.iv0 = (int)out->iv.size();
+    d.ivh += d.iv0;
+    out->iv.insert(out->iv.end(), un[u].iv.begin(), un[u].iv.end());
+    d.iv1 = (int)out->iv.size();
+  }
+  if (out->iv.empty()) out->iv.push_back(make_int4(0, 0, 0, 0));
+  out->blob_words = (size_t)std::max(1L, total);
+  out->blob.reset(new (std::nothrow) uint4[out->blob_words]);
+  if (!out->blob) return fail(kENoMem, "batch layout");
+  ok = host_parallel(ntask, [&](int t) {
+    for (size_t u = (size_t)t * chunk; u < std::min(nu, (size_t)(t + 1) * chunk); u++) {
+      Unit &x = un[u];
+      const BatchUnit &d = out->unit[u];
+      if (d.nslice == 0) continue;
+      int *head = reinterpret_cast<int *>(out->blob.get() + d.blob16);
+      uint4 *words = out->blob.get() + d.blob16;  // padding: -0, the zero row
+      std::fill(words, words + d.head / 16 + (size_t)x.warp_ch.back() * cw, make_uint4(0x80000000u, 0, 0x80000000u, 0));
+      std::copy(x.warp_sl.begin(), x.warp_sl.end(), head);
+      std::copy(x.warp_ch.begin(), x.warp_ch.end(), head + nw + 1);
+      int *pairs = head + 2 * (nw + 1), *ids = pairs + d.nslice;
+      const int *lo = out->row_lo.data() + (u / grid) * (grid + 1) + u % grid;
+      for (int w = 0; w < nw; w++) {
+        uint4 *ent = out->blob.get() + d.blob16 + d.head / 16 + (size_t)x.warp_ch[w] * cw;
+        for (int k = x.warp_sl[w]; k < x.warp_sl[w + 1]; k++) {
+          const int sl = x.order[k], np = pairs_of(x, sl);
+          bool beyond = false;
+          for (int j = 0; j < rps; j++) {
+            if ((size_t)sl * rps + j >= x.rows.size()) {
+              ids[(size_t)k * rps + j] = -1;
+              continue;
+            }
+            const int i = x.rows[(size_t)sl * rps + j];
+            ids[(size_t)k * rps + j] = i;
+            for (int q = h.ptr[i]; q < h.ptr[i + 1]; q++) {
+              const int e = q - h.ptr[i];
+              const unsigned off = x.off[q - h.ptr[lo[0]]];
+              beyond |= (int)off < 0;
+              unsigned vb;
+              std::memcpy(&vb, &h.val[q], 4);
+              uint4 &o = ent[(size_t)(e / 2) * rps + j];
+              if (e & 1) { o.z = vb; o.w = off; }
+              else { o.x = vb; o.y = off; }
+            }
+          }
+          pairs[k] = beyond ? -np : np;
+          ent += (size_t)np * rps;
+        }
+      }
+    }
+  });
+  if (!ok) return fail(kENoMem, "batch layout");
+  out->far = 0;
+  for (const Unit &x : un) out->far += x.far;
+  return kOk;
+}
+
+int batch_launch_raw(mpkg_plan *p, float *d_vb, cudaStream_t st) {
   BatchArgs a = p->batch;
   a.vb = d_vb;
-  if (capture) {
-    a.base = 1;  // the graph resets the flags before every replay
-  } else {
-    BatchArgs &w = p->batch;
-    const unsigned step = (unsigned)w.ngroup * (unsigned)(w.nlevel + 1);
-    if (w.base == 0 || w.base > (1u << 30)) {
-      CUDA_TRY(cudaMemsetAsync(w.flags, 0, sizeof(unsigned int) * (size_t)w.nblk, st));
-      w.base = 1;
-    } else {
-      w.base += step;
-    }
-    a.base = w.base;
-  }
-  if (capture) CUDA_TRY(cudaMemsetAsync(a.flags, 0, sizeof(unsigned int) * (size_t)a.nblk, st));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(a.nblk);
   cfg.blockDim = dim3(p->batch_threads);
@@ -2492,14 +2927,13 @@ int batch_launch_raw(mpkg_plan *p, float *d_vb, cudaStream_t st, bool capture) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   CUDA_TRY(cudaLaunchKernelEx(&cfg,
-                              p->batch_staged ? batch_stage_kernel_for(p->batch_lpr, p->batch_vw)
+                              p->batch_staged ? batch_pack_kernel_for(p->batch_lpr, p->batch_resident)
                                               : batch_kernel_for(p->batch_lpr, p->batch_vw),
                               a));
   return kOk;
 }
 
-// One replayable graph per output buffer: flag reset + the persistent
-// kernel.  Falls back to a direct launch when capture is not possible.
+// One replayable graph per output buffer: the persistent kernel.  Falls back to a direct launch when capture is not possible.
 int batch_launch(mpkg_plan *p, float *d_vb, cudaStream_t st) {
   if (p->graph_ok && p->graph_key == d_vb) {
     CUDA_TRY(cudaGraphLaunch(p->graph_exec, st));
@@ -2512,7 +2946,7 @@ int batch_launch(mpkg_plan *p, float *d_vb, cudaStream_t st) {
   bool ok = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) == cudaSuccess;
   if (ok) ok = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
   if (ok) {
-    const int rc = batch_launch_raw(p, d_vb, cs, true);
+    const int rc = batch_launch_raw(p, d_vb, cs);
     cudaGraph_t g = nullptr;
     const bool ended = cudaStreamEndCapture(cs, &g) == cudaSuccess;
     ok = rc == kOk && ended && g != nullptr;
@@ -2532,7 +2966,7 @@ int batch_launch(mpkg_plan *p, float *d_vb, cudaStream_t st) {
     CUDA_TRY(cudaGraphLaunch(p->graph_exec, st));
     return kOk;
   }
-  return batch_launch_raw(p, d_vb, st, false);
+  return batch_launch_raw(p, d_vb, st);
 }
 
 int launch_spmv(int n, const int *ptr, const int *col, const double *coef, bool valued, int nlevel,
@@ -2763,6 +3197,7 @@ void mpkg_plan_destroy(mpkg_plan *p) {
   if (p && p->graph) cudaGraphDestroy(p->graph);
   if (!p) return;
   for (void *q : p->owned) cudaFree(q);
+  for (void *q : p->batch_owned) cudaFree(q);
   if (p->d_vv) cudaFree(p->d_vv);
   if (p->d_fb) cudaFree(p->d_fb);
   if (p->stream) cudaStreamDestroy(p->stream);
@@ -3344,36 +3779,76 @@ extern "C" {
 
 namespace {
 
-// Device state of one (lpr, vw, budget, grid) configuration of a batch plan.
-int batch_configure(mpkg_plan *p, const BatchHost &h, int lpr, int vw, long budget, int grid, bool staged,
-                    int threads, size_t smem) {
-  std::vector<int> lo, dlo, dhi, win;
-  int ngroup = 0;
-  const long cap_rows = staged ? (long)(smem / (4 * (size_t)p->batch.nrhs)) : 0;
-  batch_layout(h, p->batch.nrhs, budget, grid, cap_rows, &lo, &dlo, &dhi, &win, &ngroup);
+// One configuration of a batch plan.
+struct BatchCand {
+  int lpr, vw;
+  long budget;  // L2 group
+  int grid;
+  bool staged;
+  int threads;
+  size_t smem;  // shared memory per CTA
+};
+
+int batch_build_layout(const BatchHost &h, int nrhs, const BatchCand &c, BatchLayout *lay) {
+  int rc = batch_ranges(h, nrhs, c.budget, c.staged, c.grid, c.threads, c.lpr, lay);
+  if (rc || !c.staged) return rc;
+  // the resident form where the matrix, the windows (a tenth of them halo)
+  // and half a chunk per warp fit all the CTAs together; each is checked
+  const long need = 9L * (long)h.col.size() + h.N * (4L * nrhs * 11 / 10 + 10) +
+                    (long)c.grid * (c.threads / 32) * bp_chunk_bytes(c.lpr) / 2;
+  if (lay->ngroup == 1 && need < (long)(0.93 * c.grid * (double)c.smem)) {
+    rc = batch_pack(h, c.grid, c.lpr, c.threads, (long)c.smem, true, lay);
+    if (rc || lay->resident) return rc;
+  }
+  return batch_pack(h, c.grid, c.lpr, c.threads, (long)c.smem, false, lay);
+}
+
+// The device state of a configuration, in place of the one before it.
+int batch_configure(mpkg_plan *p, const BatchHost &h, const BatchCand &c, const BatchLayout &lay) {
   BatchArgs &a = p->batch;
-  // previous layout arrays are freed with the plan (owned list); small
-  int *d_lo = nullptr, *d_dlo = nullptr, *d_dhi = nullptr, *d_win = nullptr;
-  unsigned int *d_flags = nullptr;
-  int rc = dev_copy(p, &d_lo, lo.data(), lo.size());
-  if (!rc) rc = dev_copy(p, &d_dlo, dlo.data(), dlo.size());
-  if (!rc) rc = dev_copy(p, &d_dhi, dhi.data(), dhi.size());
-  if (!rc && staged) rc = dev_copy(p, &d_win, win.data(), win.size());
-  if (!rc) rc = dev_alloc(p, &d_flags, (size_t)grid);
-  if (!rc && staged &&
-      cudaFuncSetAttribute((const void *)batch_stage_kernel_for(lpr, vw),
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    rc = fail(kECuda, "shared memory attribute");
-  if (rc) return rc;
-  a.row_lo = d_lo; a.dep_ptr = d_dlo; a.dep_idx = d_dhi; a.flags = d_flags; a.win = d_win;
-  a.nblk = grid; a.ngroup = ngroup; a.base = 0;
-  p->batch_lpr = lpr; p->batch_vw = vw; p->batch_group_bytes = budget;
-  p->batch_staged = staged; p->batch_threads = threads; p->batch_smem = staged ? smem : 0;
-  p->pipe_grid = grid;
   if (p->graph_exec) { cudaGraphExecDestroy(p->graph_exec); p->graph_exec = nullptr; }
   if (p->graph) { cudaGraphDestroy(p->graph); p->graph = nullptr; }
   p->graph_ok = false;
   p->graph_key = nullptr;
+  for (void *q : p->batch_owned) cudaFree(q);
+  p->batch_owned.clear();
+  p->device_bytes -= p->batch_bytes;
+  const size_t owned0 = p->owned.size();
+  const long bytes0 = p->device_bytes;
+  int *d_lo = nullptr, *d_dlo = nullptr, *d_dhi = nullptr;
+  unsigned int *d_flags = nullptr;
+  int rc = dev_copy(p, &d_lo, lay.row_lo.data(), lay.row_lo.size());
+  if (!rc) rc = dev_copy(p, &d_dlo, lay.dptr.data(), lay.dptr.size());
+  if (!rc) rc = dev_copy(p, &d_dhi, lay.didx.data(), lay.didx.size());
+  if (!rc) rc = dev_alloc(p, &d_flags, (size_t)c.grid);
+  if (!rc && cudaMemset(d_flags, 0, sizeof(unsigned int) * (size_t)c.grid) != cudaSuccess) rc = fail(kECuda, "memset failed");
+  if (!rc && c.staged) {
+    BatchUnit *unit = nullptr;
+    int4 *iv = nullptr;
+    uint4 *blob = nullptr;
+    rc = dev_copy(p, &unit, lay.unit.data(), lay.unit.size());
+    if (!rc) rc = dev_copy(p, &iv, lay.iv.data(), lay.iv.size());
+    if (!rc) rc = dev_copy(p, &blob, lay.blob.get(), lay.blob_words);
+    a.unit = unit; a.iv = iv; a.blob = reinterpret_cast<const unsigned char *>(blob);
+  }
+  p->batch_owned.assign(p->owned.begin() + owned0, p->owned.end());
+  p->owned.resize(owned0);
+  p->batch_bytes = p->device_bytes - bytes0;
+  if (!rc && !c.staged && !a.ptr) {  // batch_kernel reads the CSR
+    int *d_ptr = nullptr, *d_col = nullptr;
+    float *d_val = nullptr;
+    rc = dev_copy(p, &d_ptr, h.ptr.data(), h.ptr.size());
+    if (!rc) rc = dev_copy(p, &d_col, h.col.data(), h.col.size());
+    if (!rc) rc = dev_copy(p, &d_val, h.val.data(), h.val.size());
+    a.ptr = d_ptr; a.col = d_col; a.val = d_val;
+  }
+  if (rc) return rc;
+  a.row_lo = d_lo; a.dep_ptr = d_dlo; a.dep_idx = d_dhi; a.flags = d_flags;
+  a.nblk = c.grid; a.ngroup = lay.ngroup;
+  p->batch_lpr = c.lpr; p->batch_vw = c.vw; p->batch_group_bytes = c.budget;
+  p->batch_resident = c.staged && lay.resident;
+  p->batch_staged = c.staged; p->batch_threads = c.threads; p->batch_smem = c.staged ? c.smem : 0;
+  p->pipe_grid = c.grid;
   return kOk;
 }
 
@@ -3429,73 +3904,85 @@ int mpkg_plan_batch(int nmat, const int *n, const int *const *ptr, const int *co
     rc = fail(kECuda, "stream creation failed");
   BatchArgs &a = p->batch;
   a.N = h.N; a.nrhs = nrhs; a.nlevel = nlevel;
-  int *d_ptr = nullptr, *d_col = nullptr;
-  float *d_val = nullptr;
-  if (!rc) rc = dev_copy(p, &d_ptr, h.ptr.data(), h.ptr.size());
-  if (!rc) rc = dev_copy(p, &d_col, h.col.data(), h.col.size());
-  if (!rc) rc = dev_copy(p, &d_val, h.val.data(), h.val.size());
   if (!rc) rc = dev_alloc(p, &p->d_err, 1);
   if (!rc && cudaMemset(p->d_err, 0, sizeof(int)) != cudaSuccess) rc = fail(kECuda, "memset failed");
-  a.ptr = d_ptr; a.col = d_col; a.val = d_val; a.err = p->d_err;
-  int nsm = 0;
-  if (!rc && cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device) != cudaSuccess)
+  a.err = p->d_err;
+  int nsm = 0, sm_per_sm = 0, sm_optin = 0;
+  if (!rc &&
+      (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device) != cudaSuccess ||
+       cudaDeviceGetAttribute(&sm_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, p->device) != cudaSuccess ||
+       cudaDeviceGetAttribute(&sm_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, p->device) != cudaSuccess))
     rc = fail(kECuda, "device query failed");
-  // candidates: lanes x vector width covering nrhs, group budget, CTAs per
-  // SM; and the staged kernel at one or two CTAs per SM
-  struct Cand { int lpr, vw; long budget; int grid; bool staged; int threads; size_t smem; };
-  std::vector<Cand> cands;
+  // candidates: the packed kernel at four, two or one CTAs per SM (nrhs a
+  // multiple of 4), and the CSR kernel; each with groups of three sizes
+  std::vector<BatchCand> cands;
+  const bool packable = nrhs % 4 == 0;
+  for (int ctas : {1, 2, 4}) {
+    if (rc || !packable) break;
+    const int threads = 1024 / ctas, lpr = nrhs / 4;
+    // the SM's share, less the static part and the per-CTA reserve
+    size_t smem = std::min<size_t>((size_t)sm_optin, (size_t)sm_per_sm / ctas) - 2048;
+    // the limit of a function is the largest that any plan uses: plans of
+    // other windows share it
+    int per_sm = INT32_MAX;
+    for (bool resident : {false, true}) {
+      BatchKernel k = batch_pack_kernel_for(lpr, resident);
+      int fit = 0;
+      if (cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_optin - 1024) !=
+              cudaSuccess ||
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, threads, smem) != cudaSuccess) {
+        cudaGetLastError();
+        fit = 0;
+      }
+      per_sm = std::min(per_sm, fit);
+    }
+    if (per_sm <= 0) continue;
+    const long window = (long)smem - kBatchZero - (long)(threads / 32) * kBpRing * bp_chunk_bytes(lpr);
+    for (double share : {0.95, 0.6, 0.4})
+      cands.push_back({lpr, 4, (long)(share * per_sm * nsm * window), (int)std::min<long>((long)per_sm * nsm, h.N), true, threads, smem});
+  }
   for (int vw : {4, 2, 1}) {
-    if (nrhs % vw) continue;
+    if (rc || nrhs % vw || (packable && vw < 4)) continue;
     const int lpr = nrhs / vw;
-    if (lpr > 32) continue;
     int per_sm = 0;
-    if (!rc && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel_for(lpr, vw), 256, 0) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel_for(lpr, vw), 256, 0) != cudaSuccess)
       rc = fail(kECuda, "occupancy query failed");
     if (rc || per_sm <= 0) continue;
-    for (long budget : {32L << 20, 64L << 20, 1L << 40})
+    for (long budget : {64L << 20, 32L << 20, 1L << 40})
       for (int occ : {per_sm, std::max(1, per_sm / 2)}) {
-        cands.push_back({lpr, vw, budget, std::max(1, std::min<int>(occ * nsm, (int)std::min<long>(h.N, INT32_MAX))),
-                         false, 256, 0});
+        cands.push_back({lpr, vw, budget, (int)std::min<long>((long)occ * nsm, h.N), false, 256, 0});
         if (occ == std::max(1, per_sm / 2)) break;
       }
   }
-  if (!rc && nrhs % 4 == 0 && nrhs / 4 <= 32) {
-    int sm_per_sm = 0, sm_optin = 0;
-    if (cudaDeviceGetAttribute(&sm_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, p->device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sm_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, p->device) != cudaSuccess)
-      rc = fail(kECuda, "device query failed");
-    for (int ctas : {1, 2, 4}) {
-      if (rc) break;
-      const int threads = 1024 / ctas;
-      // a window of whole rows within the SM's share, less the static part and the per-CTA reserve
-      size_t smem = std::min<size_t>((size_t)sm_optin, (size_t)sm_per_sm / ctas) - 2048;
-      smem -= smem % (4 * (size_t)nrhs);
-      BatchKernel k = batch_stage_kernel_for(nrhs / 4, 4);
-      int per_sm = 0;
-      if (cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-              cudaSuccess ||
-          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem) != cudaSuccess) {
-        cudaGetLastError();
-        continue;
-      }
-      if (per_sm <= 0) continue;
-      for (long budget : {32L << 20, 64L << 20, 1L << 40})
-        cands.push_back({nrhs / 4, 4, budget, std::max(1, std::min<int>(per_sm * nsm, (int)std::min<long>(h.N, INT32_MAX))),
-                         true, threads, smem});
-    }
-  }
   if (!rc && cands.empty()) rc = fail(kEInval, "no kernel configuration for this nrhs");
-  Cand best = cands.empty() ? Cand{1, 1, 0, 1, false, 256, 0} : cands[0];
+  BatchCand best = cands.empty() ? BatchCand{1, 1, 0, 1, false, 256, 0} : cands[0];
+  BatchLayout lay;
+  bool laid = false;  // lay is best's
   if (!rc && tune >= MPKG_BATCH_STAGED) {  // untimed staged configuration
     const int want_threads = tune == MPKG_BATCH_STAGED ? 1024 : tune == MPKG_BATCH_STAGED2 ? 512 : 256;
     bool found = false;
-    for (const Cand &c : cands)
-      if (c.staged && c.threads == want_threads && c.budget == (64L << 20)) {
+    for (const BatchCand &c : cands)
+      if (c.staged && c.threads == want_threads) {
         best = c;
         found = true;
         break;
       }
     if (!found) rc = fail(kEInval, "no staged configuration for this nrhs and device");
+  } else if (!rc && tune == MPKG_BATCH_DEFAULT && packable) {
+    // one CTA per SM (the least halo; two and four measure the same on large
+    // batches and more on small ones); where its windows miss a fourth of the
+    // columns, the CSR kernel
+    if (best.staged) {
+      rc = batch_build_layout(h, nrhs, best, &lay);
+      laid = !rc;
+    }
+    if (!rc && (!best.staged || 4 * lay.far > nnz))
+      for (const BatchCand &c : cands)
+        if (!c.staged) {
+          best = c;
+          laid = false;
+          break;
+        }
   } else if (!rc && tune == MPKG_BATCH_TUNE && cands.size() > 1) {
     // time every candidate on the plan's own matrices (zero input; the
     // arithmetic does not depend on the values)
@@ -3509,17 +3996,23 @@ int mpkg_plan_batch(int nmat, const int *n, const int *const *ptr, const int *co
       rc = fail(kECuda, "event creation failed");
     float best_ms = 1e30f;
     auto t_start = std::chrono::steady_clock::now();
-    for (const Cand &c : cands) {
+    for (const BatchCand &c : cands) {
       if (rc) break;
-      if ((rc = batch_configure(p, h, c.lpr, c.vw, c.budget, c.grid, c.staged, c.threads, c.smem))) break;
-      for (int w = 0; w < 2 && !rc; w++) rc = batch_launch_raw(p, scratch, p->stream, false);
+      BatchLayout l;
+      if ((rc = batch_build_layout(h, nrhs, c, &l)) || (rc = batch_configure(p, h, c, l))) break;
+      for (int w = 0; w < 2 && !rc; w++) rc = batch_launch_raw(p, scratch, p->stream);
       if (!rc && cudaEventRecord(e0, p->stream) != cudaSuccess) rc = fail(kECuda, "event record");
-      for (int w = 0; w < 3 && !rc; w++) rc = batch_launch_raw(p, scratch, p->stream, false);
+      for (int w = 0; w < 3 && !rc; w++) rc = batch_launch_raw(p, scratch, p->stream);
       if (!rc && cudaEventRecord(e1, p->stream) != cudaSuccess) rc = fail(kECuda, "event record");
       if (!rc) rc = mpkg_sync(p, p->stream);
       float ms = 0.f;
       if (!rc && cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) rc = fail(kECuda, "event time");
-      if (!rc && ms < best_ms) { best_ms = ms; best = c; }
+      if (!rc && ms < best_ms) {
+        best_ms = ms;
+        best = c;
+        lay = std::move(l);
+        laid = true;
+      }
     }
     p->batch_tune_ms =
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
@@ -3527,9 +4020,9 @@ int mpkg_plan_batch(int nmat, const int *n, const int *const *ptr, const int *co
     if (e1) cudaEventDestroy(e1);
     if (scratch) cudaFree(scratch);
   }
+  if (!rc && !laid) rc = batch_build_layout(h, nrhs, best, &lay);
   p->batch_candidates = (int)cands.size();
-  if (!rc)
-    rc = batch_configure(p, h, best.lpr, best.vw, best.budget, best.grid, best.staged, best.threads, best.smem);
+  if (!rc) rc = batch_configure(p, h, best, lay);
   if (rc) { mpkg_plan_destroy(p); return rc; }
   *out = p;
   return kOk;
@@ -4381,7 +4874,8 @@ int mpkg_sync(mpkg_plan *p, void *stream) {
     }
     if (p->exec == MPKG_EXEC_WAVE) p->wave.base = 0;  // flags restart from zero on the next call
     if (p->inner) p->inner->wave.base = 0;
-    if (p->exec == MPKG_EXEC_BATCH) p->batch.base = 0;
+    if (p->exec == MPKG_EXEC_BATCH && p->batch.flags)  // left behind by an abort
+      cudaMemset(p->batch.flags, 0, sizeof(unsigned int) * (size_t)p->batch.nblk);
     if (err == kErrTimeout) return fail(kETimeout, "a device-side wait exceeded its spin limit");
     return fail(kERange, "device-side bounds check failed");
   }
