@@ -51,6 +51,52 @@ __device__ __forceinline__ double row_term(double s, double a, double x) {
   return __fma_rn(a, x, s);
 }
 
+// a * x rounded to nearest even on the integer pipes: the 53 x 53 bit product
+// as four 32-bit multiplies, the top 53 bits rounded on what lies below.
+// False (and no result) unless both exponents are within 2^-503 .. 2^496,
+// where neither operand nor product is subnormal, zero, infinite or NaN.
+// GB300 has two FP64 lanes per SM and clock, so an FP64 product holds its
+// scheduler's pipe for 64 cycles; this one takes about 40 issue slots of the
+// idle integer pipes beside it.  Products per second, 1024 threads per SM:
+// 0.50 T all FP64, 0.53 T all integer, 0.98 T half and half.
+__device__ __forceinline__ bool mul_int(double a, double x, double *p) {
+  const unsigned long long A = (unsigned long long)__double_as_longlong(a);
+  const unsigned long long X = (unsigned long long)__double_as_longlong(x);
+  const uint32_t ea = (uint32_t)(A >> 52) & 0x7FFu, ex = (uint32_t)(X >> 52) & 0x7FFu;
+  if (ea - 520u >= 1000u || ex - 520u >= 1000u) return false;
+  const unsigned long long ma = (A << 11) | 0x8000000000000000ull;                     // top bit 63
+  const unsigned long long mx = (X & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;        // top bit 52
+  const uint32_t al = (uint32_t)ma, ah = (uint32_t)(ma >> 32), xl = (uint32_t)mx, xh = (uint32_t)(mx >> 32);
+  const unsigned long long t0 = (unsigned long long)al * xl;
+  const unsigned long long t1 = (unsigned long long)ah * xl + (t0 >> 32);
+  const unsigned long long t2 = (unsigned long long)al * xh + (uint32_t)t1;
+  const unsigned long long t3 = (unsigned long long)ah * xh + (t1 >> 32);
+  unsigned long long hi = t3 + (t2 >> 32), lo = (t2 << 32) | (uint32_t)t0;             // hi: 52 or 53 bits
+  const uint32_t n = ((uint32_t)(hi >> 52) & 1u) ^ 1u;
+  hi = (hi << n) | ((lo >> 63) & n);
+  lo <<= n;  // its low 11 bits are zero: no overflow below
+  hi += lo + 0x7FFFFFFFFFFFFFFFull + (hi & 1ull) < lo ? 1ull : 0ull;
+  // hi's bit 52 (53 after a carry) adds to the exponent field
+  *p = __longlong_as_double((long long)(((A ^ X) & 0x8000000000000000ull) |
+                                        (((unsigned long long)(ea + ex - 1023u - n) << 52) + hi)));
+  return true;
+}
+
+// row_term(+0, a, x): the first term of a row is a product alone.
+template <int ARITH>
+__device__ __forceinline__ double row_first(double a, double x) {
+  double p;
+  return mul_int(a, x, &p) ? p : row_term<ARITH>(0.0, a, x);
+}
+
+// row_term with the separately rounded product on the integer pipes.
+template <int ARITH>
+__device__ __forceinline__ double row_next(double s, double a, double x) {
+  double p;
+  if (ARITH == MPKG_ARITH_SEPARATE) return __dadd_rn(s, mul_int(a, x, &p) ? p : __dmul_rn(a, x));
+  return row_term<ARITH>(s, a, x);
+}
+
 __device__ __forceinline__ double ld_cg(const double *p) { return __ldcg(p); }
 
 // ------------------------------------------------------------------------
@@ -64,14 +110,28 @@ __global__ void __launch_bounds__(256) spmv_level_kernel(int n, const int *__res
                                                          double *__restrict__ y) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  int j0 = ptr[i], j1 = ptr[i + 1];
+  const int j0 = ptr[i], j1 = ptr[i + 1];
+  const double a = VALUED ? 0.0 : coef[i];  // 1/deg, rounded on the host exactly as 1.0/deg
   double s = 0.0;
-  if (VALUED) {
-    for (int j = j0; j < j1; j++) s = row_term<ARITH>(s, coef[j], x[col[j]]);
-  } else {
-    double a = coef[i];  // 1/deg, rounded on the host exactly as 1.0/deg
-    for (int j = j0; j < j1; j++) s = row_term<ARITH>(s, a, x[col[j]]);
+  if (j0 < j1) s = row_first<ARITH>(VALUED ? coef[j0] : a, x[col[j0]]);
+  int j = j0 + 1;
+  if (ARITH == MPKG_ARITH_SEPARATE) {
+    // three products of four on the integer pipes, the fourth beside them on
+    // the FP64 pipe (97 x 96 x 95 diffusion, 6 levels: 175 us with all on the
+    // FP64 pipe, 136 with none, 125 so; of 2, 3, 5, 6: 164, 130, 129, 152)
+    constexpr int G = 4;
+    for (; j + G <= j1; j += G) {
+      double xv[G], v[G];
+#pragma unroll
+      for (int u = 0; u < G; u++) {
+        xv[u] = x[col[j + u]];
+        v[u] = VALUED ? coef[j + u] : a;
+      }
+#pragma unroll
+      for (int u = 0; u < G; u++) s = u < G - 1 ? row_next<ARITH>(s, v[u], xv[u]) : row_term<ARITH>(s, v[u], xv[u]);
+    }
   }
+  for (; j < j1; j++) s = row_next<ARITH>(s, VALUED ? coef[j] : a, x[col[j]]);
   y[i] = s;
 }
 
@@ -850,30 +910,35 @@ __device__ __forceinline__ int ld_off(const short *p) {
   return (int)__ldg(p);
 }
 
+// Separate arithmetic: the first kIntTerms terms of a row have integer
+// products, the others FP64 ones (110 x 111 x 112, 1/deg, 8 levels, all on the
+// FP64 pipe 392 us; 4, 5, 6, 7 of 7: 273, 255, 252, 258).
+constexpr int kIntTerms = 6;
+
 // One row's sum over its entries (CSR order): the row's int16 offsets are
 // RS apart (32: per-lane layout, a constant after inlining; 1: a slice's
-// shared list), values and int32 columns 32 apart.  Up to 8 (12 for FP32) entries have all their
-// loads in flight together.
+// shared list), values and int32 columns 32 apart.  The first 8 (12 for FP32)
+// entries have all their loads in flight together, whatever the row's
+// length; the first product runs on the integer pipes (128^3 1/deg, 8 levels:
+// 270 -> 249 us; 9-point diffusion 1400 x 1300 in FP64, whose rows of 9 used
+// to load entry by entry: 360 -> 293 us).
 template <int ARITH, bool VALUED, bool REL, bool STAGE>
 __device__ __forceinline__ double fp_row(int len, int RS, double cf, const short *cr, const int *cc,
                                          const double *cv, const double *xb, const double *src) {
-  double s = 0.0;
-  int t = 0;
-  if (len <= 8) {
-    double x[8], v[8];
+  double x[8], v[8];
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-      if (u < len) {
-        x[u] = REL ? xb[ld_off<STAGE>(cr + RS * u)] : src[__ldg(cc + 32 * u)];
-        v[u] = VALUED ? __ldg(cv + 32 * u) : cf;
-      }
+  for (int u = 0; u < 8; u++) {
+    if (u < len) {
+      x[u] = REL ? xb[ld_off<STAGE>(cr + RS * u)] : src[__ldg(cc + 32 * u)];
+      v[u] = VALUED ? __ldg(cv + 32 * u) : cf;
     }
-#pragma unroll
-    for (int u = 0; u < 8; u++)
-      if (u < len) s = row_term<ARITH>(s, v[u], x[u]);
-    t = len;
   }
-  for (; t < len; t++)
+  double s = 0.0;
+  if (len > 0) s = row_first<ARITH>(v[0], x[0]);
+#pragma unroll
+  for (int u = 1; u < 8; u++)
+    if (u < len) s = u < kIntTerms ? row_next<ARITH>(s, v[u], x[u]) : row_term<ARITH>(s, v[u], x[u]);
+  for (int t = 8; t < len; t++)
     s = row_term<ARITH>(s, VALUED ? __ldg(cv + 32L * t) : cf,
                         REL ? xb[ld_off<STAGE>(cr + RS * t)] : src[__ldg(cc + 32L * t)]);
   return s;
