@@ -14,7 +14,7 @@ BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libmpk_gb300.so")
 
 HOST_SOURCES = ["graph.cc", "partition.cc", "prep.cc", "bufs.cc", "pdmpk.cc", "api.cc"]
-CUDA_SOURCES = ["device.cu", "sstep.cu", "mlp.cu", "prep_gpu.cu"]
+CUDA_SOURCES = ["device.cu", "diag.cu", "sstep.cu", "mlp.cu", "prep_gpu.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
@@ -67,9 +67,9 @@ def _build(nvcc, metis, verbose, force):
         force = True
         with open(stamp, "w") as f:
             f.write(want)
-    headers = [os.path.join(CSRC, h) for h in os.listdir(CSRC) if h.endswith(".h")]
+    headers = [os.path.join(CSRC, h) for h in os.listdir(CSRC) if h.endswith((".h", ".cuh"))]
     inc = os.path.join(os.path.dirname(HERE), "include")
-    headers += [os.path.join(inc, h) for h in os.listdir(inc) if h.endswith(".h")]
+    headers += [os.path.join(inc, h) for h in os.listdir(inc) if h.endswith((".h", ".cuh"))]
     jobs, objs = [], []
     for src in HOST_SOURCES:
         s = os.path.join(CSRC, src)

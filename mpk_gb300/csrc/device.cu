@@ -28,74 +28,13 @@
 #include <vector>
 
 #include "../../include/mpk_gb300.h"
+#include "diag.cuh"
 #include "host.h"
+#include "rows.cuh"
 
 using namespace mpkg;
 
 namespace {
-
-constexpr int kErrTimeout = 2;
-constexpr int kErrBounds = 3;
-constexpr long kSpinLimit = 4000000;  // polls of one flag (~1 s with backoff)
-
-#define CUDA_TRY(expr)                                                             \
-  do {                                                                             \
-    cudaError_t e_ = (expr);                                                       \
-    if (e_ != cudaSuccess)                                                         \
-      return fail(kECuda, std::string(#expr) + ": " + cudaGetErrorString(e_));     \
-  } while (0)
-
-template <int ARITH>
-__device__ __forceinline__ double row_term(double s, double a, double x) {
-  if (ARITH == MPKG_ARITH_SEPARATE) return __dadd_rn(s, __dmul_rn(a, x));
-  return __fma_rn(a, x, s);
-}
-
-// a * x rounded to nearest even on the integer pipes: the 53 x 53 bit product
-// as four 32-bit multiplies, the top 53 bits rounded on what lies below.
-// False (and no result) unless both exponents are within 2^-503 .. 2^496,
-// where neither operand nor product is subnormal, zero, infinite or NaN.
-// GB300 has two FP64 lanes per SM and clock, so an FP64 product holds its
-// scheduler's pipe for 64 cycles; this one takes about 40 issue slots of the
-// idle integer pipes beside it.  Products per second, 1024 threads per SM:
-// 0.50 T all FP64, 0.53 T all integer, 0.98 T half and half.
-__device__ __forceinline__ bool mul_int(double a, double x, double *p) {
-  const unsigned long long A = (unsigned long long)__double_as_longlong(a);
-  const unsigned long long X = (unsigned long long)__double_as_longlong(x);
-  const uint32_t ea = (uint32_t)(A >> 52) & 0x7FFu, ex = (uint32_t)(X >> 52) & 0x7FFu;
-  if (ea - 520u >= 1000u || ex - 520u >= 1000u) return false;
-  const unsigned long long ma = (A << 11) | 0x8000000000000000ull;                     // top bit 63
-  const unsigned long long mx = (X & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;        // top bit 52
-  const uint32_t al = (uint32_t)ma, ah = (uint32_t)(ma >> 32), xl = (uint32_t)mx, xh = (uint32_t)(mx >> 32);
-  const unsigned long long t0 = (unsigned long long)al * xl;
-  const unsigned long long t1 = (unsigned long long)ah * xl + (t0 >> 32);
-  const unsigned long long t2 = (unsigned long long)al * xh + (uint32_t)t1;
-  const unsigned long long t3 = (unsigned long long)ah * xh + (t1 >> 32);
-  unsigned long long hi = t3 + (t2 >> 32), lo = (t2 << 32) | (uint32_t)t0;             // hi: 52 or 53 bits
-  const uint32_t n = ((uint32_t)(hi >> 52) & 1u) ^ 1u;
-  hi = (hi << n) | ((lo >> 63) & n);
-  lo <<= n;  // its low 11 bits are zero: no overflow below
-  hi += lo + 0x7FFFFFFFFFFFFFFFull + (hi & 1ull) < lo ? 1ull : 0ull;
-  // hi's bit 52 (53 after a carry) adds to the exponent field
-  *p = __longlong_as_double((long long)(((A ^ X) & 0x8000000000000000ull) |
-                                        (((unsigned long long)(ea + ex - 1023u - n) << 52) + hi)));
-  return true;
-}
-
-// row_term(+0, a, x): the first term of a row is a product alone.
-template <int ARITH>
-__device__ __forceinline__ double row_first(double a, double x) {
-  double p;
-  return mul_int(a, x, &p) ? p : row_term<ARITH>(0.0, a, x);
-}
-
-// row_term with the separately rounded product on the integer pipes.
-template <int ARITH>
-__device__ __forceinline__ double row_next(double s, double a, double x) {
-  double p;
-  if (ARITH == MPKG_ARITH_SEPARATE) return __dadd_rn(s, mul_int(a, x, &p) ? p : __dmul_rn(a, x));
-  return row_term<ARITH>(s, a, x);
-}
 
 __device__ __forceinline__ double ld_cg(const double *p) { return __ldcg(p); }
 
@@ -299,12 +238,6 @@ constexpr int kPipeThreads = 256;
 constexpr int kPipeChunk = kPipeThreads;  // rows per chunk, one per thread
 constexpr int kPipeGroup = 1;             // chunks per completion counter
 
-__device__ __forceinline__ unsigned int ld_acquire(const unsigned int *p) {
-  unsigned int v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
 __device__ __forceinline__ unsigned int group_size(const PipeArgs &a, int g) {
   return (unsigned)min(kPipeGroup, a.nchunk - g * kPipeGroup);
 }
@@ -341,31 +274,6 @@ __device__ __forceinline__ void pipe_publish(const PipeArgs &a, int c, int level
     __threadfence();
     atomicAdd(a.counts + (long)level * a.ngroups + c / kPipeGroup, 1u);
   }
-}
-
-// ---- 1-D bulk copies (TMA) of a chunk's CSR slice into shared memory ----
-__device__ __forceinline__ unsigned smem_u32(const void *p) {
-  return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(unsigned long long *bar) {
-  asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect(unsigned long long *bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(unsigned long long *bar, unsigned phase) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok) : "r"(smem_u32(bar)), "r"(phase) : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes, unsigned long long *bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
 }
 
 // Element range [g0, g1) of a global array (16-byte aligned base, element
@@ -506,85 +414,6 @@ __global__ void __launch_bounds__(kPipeThreads) pipe_kernel(PipeArgs a) {
       pipe_publish(a, c, l);
     }
   }
-}
-
-// ------------------------------------------------------------------------
-// Double-float ("df64") arithmetic on the FP32 pipes.  A value is an
-// unevaluated sum h + l of two floats with |l| <= ulp(h)/2 after
-// normalisation (48 significand bits).  Products use the exact FMA
-// residual; sums use Knuth's TwoSum.  Intrinsics (__fmul_rn, __fadd_rn)
-// keep the compiler from contracting the error-free transformations.
-// FP64 <-> df64 conversions use integer bit manipulation so that they do
-// not occupy the narrow FP64 pipe.
-// ------------------------------------------------------------------------
-__device__ __forceinline__ float2 df_split(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const int e = (int)((b >> 52) & 0x7FF);
-  const int E = e - 1023;
-  const unsigned int sgn = (unsigned int)(b >> 63) << 31;
-  if (e == 0x7FF || E > 127) {  // inf/nan or beyond the float range
-    const float h = __double2float_rn(x);
-    return make_float2(h, 0.0f);
-  }
-  if (E < -126) return make_float2(0.0f, 0.0f);  // below the df64 range
-  const unsigned long long m = b & 0xFFFFFFFFFFFFFull;
-  const float h = __uint_as_float(sgn | ((unsigned)(E + 127) << 23) | (unsigned)(m >> 29));
-  const unsigned int rem = (unsigned int)(m & 0x1FFFFFFFull);  // low 29 bits, weight 2^(E-52)
-  float lo = 0.0f;
-  if (rem != 0 && E - 52 >= -126) {
-    lo = __fmul_rn(__uint2float_rn(rem), __uint_as_float((unsigned)(E - 52 + 127) << 23));
-    lo = __uint_as_float(__float_as_uint(lo) | sgn);
-  }
-  return make_float2(h, lo);
-}
-
-__device__ __forceinline__ double df_widen(float f) {
-  const unsigned int u = __float_as_uint(f);
-  const unsigned int e = (u >> 23) & 0xFF;
-  if (e == 0) return __longlong_as_double((long long)((unsigned long long)(u >> 31) << 63));  // +-0
-  if (e == 0xFF) return (double)f;
-  return __longlong_as_double((long long)(((unsigned long long)(u >> 31) << 63) |
-                                          ((unsigned long long)(e + 896) << 52) |
-                                          ((unsigned long long)(u & 0x7FFFFF) << 29)));
-}
-
-__device__ __forceinline__ double df_to_double(float2 v) { return __dadd_rn(df_widen(v.x), df_widen(v.y)); }
-
-// s += a * x in double-float
-__device__ __forceinline__ void df_mac(float2 a, float2 x, float &sh, float &sl) {
-  const float p = __fmul_rn(a.x, x.x);
-  float e = __fmaf_rn(a.x, x.x, -p);
-  e = __fmaf_rn(a.x, x.y, e);
-  e = __fmaf_rn(a.y, x.x, e);
-  const float s = __fadd_rn(sh, p);
-  const float bp = __fadd_rn(s, -sh);
-  const float t = __fadd_rn(__fadd_rn(sh, -__fadd_rn(s, -bp)), __fadd_rn(p, -bp));
-  sh = s;
-  sl = __fadd_rn(sl, __fadd_rn(t, e));
-}
-
-__device__ __forceinline__ float2 df_norm(float sh, float sl) {
-  const float h = __fadd_rn(sh, sl);
-  const float l = __fadd_rn(sl, -__fadd_rn(h, -sh));
-  return make_float2(h, l);
-}
-
-// s += x in double-float (two-sum of the high parts, low parts added)
-__device__ __forceinline__ void df_acc(float2 x, float &sh, float &sl) {
-  const float s = __fadd_rn(sh, x.x);
-  const float bp = __fadd_rn(s, -sh);
-  const float t = __fadd_rn(__fadd_rn(sh, -__fadd_rn(s, -bp)), __fadd_rn(x.x, -bp));
-  sh = s;
-  sl = __fadd_rn(sl, __fadd_rn(t, x.y));
-}
-
-// a * v in double-float (v normalised)
-__device__ __forceinline__ float2 df_scale(float2 a, float2 v) {
-  const float p = __fmul_rn(a.x, v.x);
-  float e = __fmaf_rn(a.x, v.x, -p);
-  e = __fmaf_rn(a.x, v.y, e);
-  e = __fmaf_rn(a.y, v.x, e);
-  return df_norm(p, e);
 }
 
 // Pipeline in double-float: levels travel between chunks through a
@@ -801,9 +630,6 @@ __global__ void __launch_bounds__(256) bufs_phase_kernel(int list_base, const lo
 // moved on (their flags are in the list too), and read after an acquire
 // of the writers' flags, so L1 never serves a stale line.
 // ------------------------------------------------------------------------
-__device__ __forceinline__ float to_f32(float v) { return v; }
-__device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
-
 struct WaveArgs {
   int n, nlevel, nblk;
   uint32_t base;               // flags of this call start at base (level l publishes base + l)
@@ -909,11 +735,6 @@ __device__ __forceinline__ int ld_off(const short *p) {
   if (STAGE) return (int)*p;
   return (int)__ldg(p);
 }
-
-// Separate arithmetic: the first kIntTerms terms of a row have integer
-// products, the others FP64 ones (110 x 111 x 112, 1/deg, 8 levels, all on the
-// FP64 pipe 392 us; 4, 5, 6, 7 of 7: 273, 255, 252, 258).
-constexpr int kIntTerms = 6;
 
 // One row's sum over its entries (CSR order): the row's int16 offsets are
 // RS apart (32: per-lane layout, a constant after inlining; 1: a slice's
@@ -1561,19 +1382,6 @@ struct TileRegArgs {
   float scale;
   int *err;
 };
-
-__device__ __forceinline__ bool tr_wait(unsigned long long *bar, unsigned phase, int *err) {
-  long spins = 0;
-  while (!mbar_try(bar, phase)) {
-    if (spins > 16) __nanosleep(64);
-    if (++spins > kSpinLimit) {  // a copy of this CTA never completed: report, drain with a second bound
-      if (threadIdx.x == 0) atomicCAS(err, 0, kErrTimeout);
-      for (long s2 = 0; s2 < kSpinLimit && !mbar_try(bar, phase); s2++) __nanosleep(256);
-      return false;
-    }
-  }
-  return true;
-}
 
 __device__ __forceinline__ void cp_async4(float *dst, const float *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
@@ -2265,6 +2073,9 @@ struct mpkg_plan {
   int wave_grid = 0;
   bool wave_rel = false;
   bool wave_uni = false;  // pattern-compressed offsets (plans with matrix values)
+  DiagArgs dg{};          // rows on a few diagonals: the diagonal wavefront
+  bool dg_on = false;
+  int dg_form = 0, dg_w = 0, dg_gl = 0, dg_threads = 0;
   // batched block-vector form
   BatchArgs batch{};
   int batch_lpr = 0, batch_vw = 0, batch_nmat = 0;
@@ -2547,16 +2358,40 @@ size_t wave_dyn_smem(const mpkg_plan *p) {
   return w.stage_rel_bytes > 0 ? (size_t)w.stage_rel_bytes + w.stage_len_bytes + 5L * w.stage_slices : 0;
 }
 
-int launch_wave(mpkg_plan *p, double *d_vv, cudaStream_t st, double *hv = nullptr) {
+// The tags of a wavefront plan's next call.
+int wave_next(mpkg_plan *p, cudaStream_t st) {
   WaveArgs &w = p->wave;
   const unsigned step = (unsigned)p->nlevel + (p->arith == MPKG_ARITH_FIXED ? 2 : 1);
   if (w.base == 0 || w.base > (1u << 30)) {  // first call, or the flags would wrap: start over
-    CUDA_TRY(cudaMemsetAsync(w.flags, 0, sizeof(unsigned int) * (size_t)w.nblk, st));
+    CUDA_TRY(cudaMemsetAsync(w.flags, 0, sizeof(unsigned int) * (size_t)w.nblk * (p->dg_on ? kFlagStride : 1), st));
     if (w.fix_word) CUDA_TRY(cudaMemsetAsync(w.fix_word, 0, sizeof(unsigned long long), st));
     w.base = 1;
   } else {
     w.base += step;
   }
+  return kOk;
+}
+
+// The diagonal wavefront: FP64 and double-float levels in vv (x and the
+// results also or, double-float, only through hv when it is given), mixed
+// ones in vf.
+int launch_diag(mpkg_plan *p, double *vv, double *hv, float *vf, float scale, int *err, cudaStream_t st) {
+  int rc = wave_next(p, st);
+  if (rc) return rc;
+  DiagArgs a = p->dg;
+  a.base = p->wave.base; a.stall = p->wave.stall; a.flags = p->wave.flags; a.err = err;
+  a.vv = vv; a.hv = hv; a.vf = vf; a.scale = scale;
+  void *args[] = {&a};
+  CUDA_TRY(cudaLaunchCooperativeKernel(diag_kernel_ptr(p->dg_form, p->dg_w, p->dg_gl), dim3(a.nblk),
+                                       dim3(p->dg_threads), args, (size_t)a.smem, st));
+  return kOk;
+}
+
+int launch_wave(mpkg_plan *p, double *d_vv, cudaStream_t st, double *hv = nullptr) {
+  if (p->dg_on) return launch_diag(p, d_vv, hv, nullptr, 0.f, p->d_err, st);
+  WaveArgs &w = p->wave;
+  int rc = wave_next(p, st);
+  if (rc) return rc;
   WaveArgs a = w;
   a.vv = d_vv;
   a.hv = hv;
@@ -3616,6 +3451,112 @@ int mpkg_plan_wave_ctas(int n, const int *ptr, const int *col, const double *val
 
 namespace {
 
+// Device state of the diagonal wavefront on plan p (arrays of n rows; val:
+// FP64 values or null); *done says whether the matrix suits it.  p's wave
+// member carries the flags and tags.
+int diag_setup(mpkg_plan *p, int form, const int *ptr, const int *col, const double *val, bool *done) {
+  *done = false;
+  const int n = p->n;
+  int nsm = 0, optin = 0, coop = 0, per_sm = 0;
+  CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
+  CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, p->device));
+  CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, p->device));
+  if (!coop) return kOk;
+  const int smem = optin - 1024;  // less the kernel's static part
+  DiagLayout l;
+  int rc = diag_layout(n, ptr, col, form, nsm, smem, &l);
+  if (rc || !l.fits) return rc;
+  const void *fn = diag_kernel_ptr(form, l.w, l.gl);
+  CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kDiagThreads, smem));
+  if ((long)per_sm * nsm < l.grid) return kOk;
+  DiagArgs &a = p->dg;
+  a.n = n; a.nlevel = p->nlevel; a.nblk = l.grid; a.halo = l.halo; a.smem = smem; a.win_bytes = l.win_bytes;
+  a.halo_bytes = l.halo_bytes;
+  a.ring_all = l.irregular > 0;
+  for (int u = 0; u < l.w; u++) {
+    a.d[u] = l.d[u];
+    a.db[u] = l.d[u] * diag_elem_bytes(form);
+  }
+  int *lo = nullptr, *dp = nullptr, *di = nullptr, *nres = nullptr;
+  int2 *own = nullptr;
+  unsigned short *pat = nullptr, *mask = nullptr;
+  rc = dev_copy(p, &lo, l.lo.data(), l.lo.size());
+  if (!rc) rc = dev_copy(p, &dp, l.dptr.data(), l.dptr.size());
+  if (!rc) rc = dev_copy(p, &di, l.didx.data(), l.didx.size());
+  if (!rc) rc = dev_copy(p, &own, l.own.data(), l.own.size());
+  if (!rc) rc = dev_copy(p, &nres, l.nres.data(), l.nres.size());
+  if (!rc) rc = dev_copy(p, &pat, l.pat.data(), l.pat.size());
+  if (!rc) rc = dev_copy(p, &mask, l.mask.data(), l.mask.size());
+  if (!rc) rc = dev_alloc(p, &p->wave.flags, (size_t)l.grid * kFlagStride);
+  a.row_lo = lo; a.dep_ptr = dp; a.dep_idx = di; a.own = own; a.nres = nres; a.pat = pat; a.mask = mask;
+  const size_t nv = (size_t)l.pat.size() * l.w * 32;
+  const bool df = form == kDiagDf || form == kDiagDfVal;
+  auto upload = [&](auto zero, auto conv, auto **dst) -> int {
+    using T = decltype(zero);
+    std::unique_ptr<T[]> v(new (std::nothrow) T[nv]);
+    if (!v) return fail(kENoMem, "diagonal values");
+    std::fill(v.get(), v.get() + nv, zero);
+    diag_values(n, ptr, col, l, conv, v.get());
+    return dev_copy(p, dst, v.get(), nv);
+  };
+  if (!rc && val && diag_value_bytes(form) == 8) {
+    double *v = nullptr;
+    rc = upload(0.0, [&](int q) { return val[q]; }, &v);
+    a.vals = v;
+    if (!rc && df) {
+      float2 *v2 = nullptr;
+      rc = dev_alloc(p, &v2, nv);
+      if (!rc) split_kernel<<<592, 256, 0, p->stream>>>(v, v2, (long)nv);
+      a.vals = v2;
+    }
+  } else if (!rc && form == kDiagF32) {
+    float *v = nullptr;
+    rc = upload(0.f, [&](int q) { return (float)val[q]; }, &v);
+    a.vals = v;
+  } else if (!rc && form == kDiagBf16) {
+    __nv_bfloat16 *v = nullptr;
+    rc = upload(__nv_bfloat16{}, [&](int q) { return __double2bfloat16(val[q]); }, &v);
+    a.vals = v;
+  }
+  a.ptr = p->d_ptr; a.col = p->d_col;
+  a.coef = df ? (const void *)p->d_coef2 : (const void *)p->d_coef;
+  if (form == kDiagF32 || form == kDiagBf16) a.coef = p->mix.val;
+  if (!rc && !val) {
+    std::vector<double> lut(256, 0.0);
+    for (int d = 1; d < 256; d++) lut[d] = 1.0 / d;  // as the plan's 1/deg (mpk2/mpkexec.c:28)
+    double *dl = nullptr;
+    rc = dev_copy(p, &dl, lut.data(), lut.size());
+    a.lut = dl;
+    if (!rc && df) {
+      float2 *l2 = nullptr;
+      rc = dev_alloc(p, &l2, 256);
+      if (!rc) split_kernel<<<1, 256, 0, p->stream>>>(dl, l2, 256);
+      a.lut2 = l2;
+    }
+  }
+  if (!rc && df) {
+    float2 *ring = nullptr;
+    rc = dev_alloc(p, &ring, (size_t)3 * n);
+    a.ring = ring;
+  }
+  if (!rc && (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(p->stream) != cudaSuccess))
+    rc = fail(kECuda, "diagonal layout failed");
+  if (rc) return rc;
+  p->wave.n = n; p->wave.nlevel = p->nlevel; p->wave.nblk = l.grid; p->wave.base = 0; p->wave.err = p->d_err;
+  p->wave_grid = l.grid;
+  p->pipe_grid = l.grid;
+  p->pipe_reach = (int)l.reach;
+  p->rows_computed = (long)n * p->nlevel;
+  p->dg_form = form; p->dg_w = l.w; p->dg_gl = l.gl;
+  int slices = 0;  // a warp per slice, as far as they go
+  for (int b = 0; b < l.grid; b++) slices = std::max(slices, (l.lo[b + 1] - l.lo[b] + 31) / 32);
+  p->dg_threads = std::min(kDiagThreads, std::max(128, 32 * slices));
+  p->dg_on = true;
+  *done = true;
+  return kOk;
+}
+
 // occ_value_type >= 0: size the grid for the mixed-precision kernel of that
 // value type instead of the plan's own kernel
 int plan_wave_impl(int n, const int *ptr, const int *col, const double *val, int nlevel, int arith,
@@ -3627,6 +3568,16 @@ int plan_wave_impl(int n, const int *ptr, const int *col, const double *val, int
   if (!p) return fail(kENoMem, "plan allocation failed");
   p->exec = MPKG_EXEC_WAVE;
   int rc = plan_common(p, n, ptr, col, val, nlevel, arith, true);
+  if (!rc && occ_value_type < 0 && g_wave_ctas_per_sm == 0 && arith != MPKG_ARITH_FIXED) {
+    const int form = arith == MPKG_ARITH_DF64 ? (val ? kDiagDfVal : kDiagDf)
+                     : arith == MPKG_ARITH_SEPARATE ? (val ? kDiagSepVal : kDiagSep) : (val ? kDiagFmaVal : kDiagFma);
+    bool done = false;
+    rc = diag_setup(p, form, ptr, col, val, &done);
+    if (!rc && done) {
+      *out = p;
+      return kOk;
+    }
+  }
   if (!rc && arith == MPKG_ARITH_FIXED) {
     int maxlen = 0;
     for (int i = 0; i < n; i++) maxlen = std::max(maxlen, ptr[i + 1] - ptr[i]);
@@ -4413,7 +4364,26 @@ int mpkg_plan_mixed(int n, const int *ptr, const int *col, const double *val, in
   }
   // the wavefront schedule (preferred): its layout from an FP64 wave plan,
   // plus the values in the sliced order and the storage type
-  if (!rc && mixed_wave_setup(p, n, ptr, col, val, nlevel, value_type) != kOk) {
+  bool diag = false;
+  if (!rc) {
+    mpkg_plan *w = new_plan();
+    if (!w) {
+      rc = fail(kENoMem, "plan allocation failed");
+    } else {
+      p->inner = w;
+      w->exec = MPKG_EXEC_WAVE;
+      w->n = n; w->nlevel = nlevel; w->device = p->device; w->d_ptr = p->d_ptr; w->d_col = p->d_col; w->d_err = p->d_err;
+      w->mix.val = p->mix.val;
+      if (cudaStreamCreateWithFlags(&w->stream, cudaStreamNonBlocking) != cudaSuccess) rc = fail(kECuda, "stream creation failed");
+      if (!rc && diag_setup(w, value_type == MPKG_VALUE_F32 ? kDiagF32 : kDiagBf16, ptr, col, val, &diag) != kOk)
+        clear_error();  // the general wavefront, or the chunk pipeline
+      if (!diag) {
+        mpkg_plan_destroy(w);
+        p->inner = nullptr;
+      }
+    }
+  }
+  if (!rc && !diag && mixed_wave_setup(p, n, ptr, col, val, nlevel, value_type) != kOk) {
     if (p->inner) { mpkg_plan_destroy(p->inner); p->inner = nullptr; }
     clear_error();  // keep the chunk pipeline
   }
@@ -4830,6 +4800,10 @@ int mpkg_exec_mixed_device(mpkg_plan *p, float *d_vv, void *stream) {
     p->launches = 1;
     return kOk;
   }
+  if (p->inner && p->inner->dg_on) {  // diagonal wavefront
+    p->launches = 1;
+    return launch_diag(p->inner, nullptr, nullptr, d_vv, p->mix.scale, p->d_err, st);
+  }
   if (p->inner) {  // wavefront schedule
     WaveArgs &w = p->inner->wave;
     const unsigned step = (unsigned)p->nlevel + 1;
@@ -4959,8 +4933,10 @@ int mpkg_exec_host(mpkg_plan *p, double *vv) {
   if (p->exec == MPKG_EXEC_WAVE && (p->arith == MPKG_ARITH_DF64 || p->arith == MPKG_ARITH_FIXED)) {
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, vv) == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer) {
-      int rc = plan_launch(p, static_cast<double *>(at.devicePointer), p->stream);
+      double *h = static_cast<double *>(at.devicePointer);
+      int rc = p->dg_on ? launch_wave(p, nullptr, p->stream, h) : plan_launch(p, h, p->stream);
       if (rc) return rc;
+      p->launches = 1;
       return mpkg_sync(p, p->stream);
     }
     cudaGetLastError();  // pageable memory: the copies below

@@ -1,0 +1,490 @@
+// Diagonal wavefront (sm_103a): the wavefront executor for matrices whose
+// rows keep to a few diagonals (meshes in their natural order).
+//
+// One CTA of 1024 threads per SM owns a contiguous, slice-aligned row range
+// at every level and computes level l once the CTAs owning its columns have
+// published level l-1, as the general wavefront does.  Two windows in shared
+// memory hold its rows of the previous level and of the one being computed,
+// so that a row reads its columns at constant distances from its own place: no
+// index is loaded, and an entry is a shared-memory load and its arithmetic.
+// Beside the window that is read lie `halo` rows of the CTAs before and after,
+// fetched once those have published them; slices that read own rows only are
+// computed before that wait.  Where the outermost diagonal on either side
+// reaches further than the own rows (the planes of a 3-D mesh), that one entry
+// is read from global memory instead, a slice ahead.  A slice of 32 rows that
+// lacks some of the diagonals (mesh boundaries) has a pattern, a mask of
+// diagonals per lane; slices with other columns run from the CSR.  Values lie
+// [slice][diagonal][lane]; shared memory keeps as many slices of them as fit
+// beside the windows for the whole call.
+//
+// Row sums run over the entries in CSR order with the arithmetic of
+// wave_kernel, wave_df_kernel and wave_mix_kernel: the same bits.
+//
+// What bounds it: in FP64 the FP64 pipe, 6 fused multiply-adds a 7-point row
+// (47 K cycles a level on 128^3, 41 K of them that pipe's), else the
+// instructions, about 100 a slice; and at every level some 5 K cycles of
+// hand-over (release after the barrier 1.5-3 K, the neighbours' flags 1-2 K,
+// the halo 1 K).  Against the general wavefront, which reads every index and
+// its columns through L1 (us): 128^3 1/deg k = 8 228 / 249; 100^2 1/deg k = 4
+// 12.3 / 14.6; 9-point FP64 1400 x 1300 k = 8 264 / 293; double-float 1/deg
+// 101 x 97 x 89 k = 8 79 / 105; mixed FP32 120 x 110 x 100 k = 8 69 / 141, BF16
+// 9-point 701 x 699 k = 4 18.4 / 40.8.
+#include <algorithm>
+#include <atomic>
+#include <cstring>
+#include <map>
+#include <thread>
+#include <type_traits>
+#include <vector>
+
+#include "diag.cuh"
+#include "rows.cuh"
+
+using namespace mpkg;
+
+namespace {
+
+template <int F>
+struct Form;
+template <int A, bool V>
+struct Fp64Form {
+  static constexpr int kArith = A;
+  static constexpr bool kVal = V;
+  using Elem = double;
+  using Val = double;
+};
+template <>
+struct Form<kDiagFma> : Fp64Form<MPKG_ARITH_FMA, false> {};
+template <>
+struct Form<kDiagFmaVal> : Fp64Form<MPKG_ARITH_FMA, true> {};
+template <>
+struct Form<kDiagSep> : Fp64Form<MPKG_ARITH_SEPARATE, false> {};
+template <>
+struct Form<kDiagSepVal> : Fp64Form<MPKG_ARITH_SEPARATE, true> {};
+template <bool V>
+struct DfForm {
+  static constexpr int kArith = MPKG_ARITH_DF64;
+  static constexpr bool kVal = V;
+  using Elem = float2;
+  using Val = float2;
+};
+template <>
+struct Form<kDiagDf> : DfForm<false> {};
+template <>
+struct Form<kDiagDfVal> : DfForm<true> {};
+template <typename VT>
+struct MixForm {
+  static constexpr int kArith = -1;
+  static constexpr bool kVal = true;
+  using Elem = float;
+  using Val = VT;
+};
+template <>
+struct Form<kDiagF32> : MixForm<float> {};
+template <>
+struct Form<kDiagBf16> : MixForm<__nv_bfloat16> {};
+
+// A row's running sum.
+template <int F>
+struct Sum {  // FP64 and mixed
+  using E = typename Form<F>::Elem;
+  E s = 0;
+  template <typename V>
+  __device__ __forceinline__ void add(int u, V v, E x) {
+    if constexpr (Form<F>::kArith < 0) s = __fmaf_rn(to_f32(v), x, s);
+    else if (u == 0) s = row_first<Form<F>::kArith>(v, x);
+    else if (u < kIntTerms) s = row_next<Form<F>::kArith>(s, v, x);
+    else s = row_term<Form<F>::kArith>(s, v, x);
+  }
+};
+template <>
+struct Sum<kDiagDf> {
+  float h = 0.f, l = 0.f;
+  __device__ __forceinline__ void add(int, float2, float2 x) { df_acc(x, h, l); }
+};
+template <>
+struct Sum<kDiagDfVal> {
+  float h = 0.f, l = 0.f;
+  __device__ __forceinline__ void add(int, float2 v, float2 x) { df_mac(v, x, h, l); }
+};
+
+// Waits (bounded) for the CTAs list[c0 .. c1) (or c0 .. c1 themselves) to
+// publish `want`; every thread calls it.  One thread per flag polls: with every
+// warp polling, the flags' lines are so busy that a wait of 1-2 thousand cycles
+// takes 6-11 thousand.
+__device__ __forceinline__ bool diag_wait(const DiagArgs &a, const int *list, int c0, int c1, unsigned want,
+                                          int *s_abort) {
+  for (int k = c0 + (int)threadIdx.x; k < c1; k += blockDim.x) {
+    const int c = list ? list[k] : k;
+    long spins = 0;
+    while (ld_acquire(a.flags + kFlagStride * c) < want + a.stall) {
+      if (++spins > kSpinLimit || *((volatile int *)a.err)) {
+        atomicCAS(a.err, 0, kErrTimeout);
+        *s_abort = 1;
+        break;
+      }
+      __nanosleep(spins < 16 ? 32 : 256);
+    }
+  }
+  __syncthreads();
+  return *s_abort == 0;
+}
+
+__device__ __forceinline__ void diag_publish(const DiagArgs &a, int b, unsigned v) {
+  __syncthreads();
+  if (threadIdx.x == 0)
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.flags + kFlagStride * b), "r"(v) : "memory");
+}
+
+constexpr int kXGroups = 8;  // host execution: CTA groups that copy x in turn (as wave_kernel)
+
+template <int F, int W, int GL>
+__global__ void __launch_bounds__(kDiagThreads, 1) diag_kernel(const __grid_constant__ DiagArgs a) {
+  using FM = Form<F>;
+  using E = typename FM::Elem;
+  using V = typename FM::Val;
+  constexpr bool kDf = FM::kArith == MPKG_ARITH_DF64, kMix = FM::kArith < 0;
+  extern __shared__ __align__(128) unsigned char dg_smem[];
+  __shared__ int s_abort;
+  __shared__ __align__(8) unsigned long long s_bar;
+  const int b = blockIdx.x, r0 = a.row_lo[b], r1 = a.row_lo[b + 1];
+  const int s0 = r0 >> 5, ns = (r1 + 31 - r0) >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nt = blockDim.x, nw = nt >> 5;
+  // shared memory: patterns, values, then the two windows at the end
+  unsigned short *s_pat = reinterpret_cast<unsigned short *>(dg_smem);
+  V *s_val = reinterpret_cast<V *>(dg_smem + ((2 * ns + 15) & ~15));
+  const V *vals = reinterpret_cast<const V *>(a.vals) + (size_t)s0 * W * 32;
+  const int nres = FM::kVal ? a.nres[b] : 0;
+  // halo, window A, halo, window B, halo: the middle one serves both
+  unsigned char *wins = dg_smem + a.smem - 2 * a.win_bytes - 2 * a.halo_bytes;
+  const int w0 = max(0, r0 - a.halo), w1 = min(a.n, r1 + a.halo);
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    if (FM::kVal) {  // the values stream in while the window is filled
+      mbar_init(&s_bar);
+      const unsigned bytes = (unsigned)(nres * W * 32 * (int)sizeof(V));
+      mbar_expect(&s_bar, bytes);
+      for (unsigned o = 0; o < bytes; o += 32768)
+        bulk_g2s(reinterpret_cast<unsigned char *>(s_val) + o, reinterpret_cast<const unsigned char *>(vals) + o,
+                 min(32768u, bytes - o), &s_bar);
+    }
+  }
+  for (int k = threadIdx.x; k < ns; k += nt) s_pat[k] = a.pat[s0 + k];
+  auto level = [&](int l) -> const E * {  // where other CTAs' rows of level l are read
+    if constexpr (kDf) return a.ring + (size_t)(l % 3) * a.n;
+    else if constexpr (kMix) return a.vf + (size_t)l * a.n;
+    else return a.vv + (size_t)l * a.n;
+  };
+  // host execution: each CTA copies its rows of x to the device and publishes
+  // level 0, in kXGroups groups of CTAs taken in order
+  const bool host = !kMix && a.hv != nullptr;
+  if constexpr (!kMix) {
+    if (host) {
+      const int grp = (int)((long)b * kXGroups / a.nblk);
+      if (grp > 0) {
+        const int c0 = (int)(((long)(grp - 1) * a.nblk + kXGroups - 1) / kXGroups);
+        const int c1 = (int)(((long)grp * a.nblk + kXGroups - 1) / kXGroups);
+        __syncthreads();
+        if (!diag_wait(a, nullptr, c0, c1, a.base, &s_abort)) return;
+      }
+      for (int i = r0 + (int)threadIdx.x; i < r1; i += nt) {
+        if constexpr (kDf) a.ring[i] = df_split(a.hv[i]);
+        else a.vv[i] = a.hv[i];
+      }
+      diag_publish(a, b, a.base);
+      if (!diag_wait(a, a.dep_idx, a.dep_ptr[b], a.dep_ptr[b + 1], a.base, &s_abort)) return;
+    }
+  }
+  auto first = [&](int i) -> E {  // row i of level 0
+    if constexpr (kDf) return host ? __ldcg(a.ring + i) : df_split(__ldg(a.vv + i));
+    else if constexpr (kMix) return a.vf[i];
+    else return __ldcg(a.vv + i);
+  };
+  {
+    E *in = reinterpret_cast<E *>(wins) - r0;
+    for (int i = w0 + (int)threadIdx.x; i < w1; i += nt) in[i] = first(i);
+  }
+  const int own0 = a.own[b].x, own1 = a.own[b].y;
+  V coef{};  // of a row with all the diagonals
+  if constexpr (!kDf && !kMix && !FM::kVal) coef = __ldg(a.lut + W);
+  float2 coef2 = make_float2(0.f, 0.f);
+  if constexpr (kDf && !FM::kVal) coef2 = __ldg(a.lut2 + W);
+  __syncthreads();
+  if (FM::kVal && !tr_wait(&s_bar, 0, a.err)) return;
+  for (int l = 1; l <= a.nlevel; l++) {
+    const int second = a.win_bytes + a.halo_bytes;
+    E *in = reinterpret_cast<E *>(wins + (l & 1 ? 0 : second)) - r0;
+    E *out = reinterpret_cast<E *>(wins + (l & 1 ? second : 0)) - r0;
+    const E *prev = level(l - 1);
+    auto far = [&](int i) -> E { return kDf && l == 1 ? first(i) : __ldcg(prev + i); };
+    for (int part = 0; part < 2; part++) {
+      // part 0: slices [own0, own1), which read own rows only; part 1: the
+      // others, once the CTAs that own their columns have published them
+      const int cnt = part == 0 ? own1 - own0 : ns - (own1 - own0);
+      auto at = [&](int j) { return part == 0 ? own0 + j : j < own0 ? j : j + (own1 - own0); };
+      E g0{}, g1{};
+      auto fetch = [&](int j) {  // the far entries of slice j
+        if (GL > 0 && j < cnt) {
+          const int i = r0 + 32 * at(j) + lane, lo = i + a.d[0], hi = i + a.d[W - 1];
+          if (lo >= 0 && i < r1) g0 = far(lo);
+          if (hi < a.n) g1 = far(hi);  // hi > i
+        }
+      };
+      if (part == 1 && l > 1) {
+        if (!diag_wait(a, a.dep_idx, a.dep_ptr[b], a.dep_ptr[b + 1], a.base + (unsigned)(l - 1), &s_abort)) return;
+        fetch(warp);
+        for (int i = w0 + (int)threadIdx.x; i < r0; i += nt) in[i] = __ldcg(prev + i);
+        for (int i = r1 + (int)threadIdx.x; i < w1; i += nt) in[i] = __ldcg(prev + i);
+        __syncthreads();
+      } else {
+        fetch(warp);
+      }
+      for (int j = warp; j < cnt; j += nw) {
+        const int k = at(j), i = r0 + 32 * k + lane;
+        const E x0 = g0, x1 = g1;
+        fetch(j + nw);
+        if (i >= r1) continue;
+        const int pat = s_pat[k];
+        Sum<F> s;
+        int len = W;
+        if (pat != kDiagIrregular) {
+          const int m = pat == 0 ? (1 << W) - 1 : __ldg(a.mask + 32 * pat + lane);
+          const unsigned char *own = reinterpret_cast<const unsigned char *>(in + i);
+          auto entry = [&](int u) -> E {
+            return GL > 0 && u == 0 ? x0 : GL > 0 && u == W - 1 ? x1 : *reinterpret_cast<const E *>(own + a.db[u]);
+          };
+          auto row = [&](auto value) {  // value(u): from shared memory, or from global memory
+            if (pat == 0) {
+              E x[W];
+#pragma unroll
+              for (int u = 0; u < W; u++) x[u] = entry(u);
+#pragma unroll
+              for (int u = 0; u < W; u++) s.add(u, FM::kVal ? value(u) : coef, x[u]);
+            } else {
+              len = __popc(m);
+              V c{};
+              if constexpr (!kDf && !kMix && !FM::kVal) c = __ldg(a.lut + len);
+#pragma unroll
+              for (int u = 0; u < W; u++)
+                if (m & (1 << u)) s.add(u, FM::kVal ? value(u) : c, entry(u));
+            }
+          };
+          const V *v = s_val + k * W * 32 + lane;
+          if (!FM::kVal || k < nres) {
+            row([&](int u) { return v[32 * u]; });
+          } else {
+            const V *vg = vals + (size_t)k * W * 32 + lane;
+            V w[W];
+#pragma unroll
+            for (int u = 0; u < W; u++) w[u] = __ldg(vg + 32 * u);
+            row([&](int u) { return w[u]; });
+          }
+        } else {  // any columns: the CSR row
+          const int q0 = __ldg(a.ptr + i);
+          len = __ldg(a.ptr + i + 1) - q0;
+          const V *cf = static_cast<const V *>(a.coef);
+          for (int q = 0; q < len; q++) {
+            const int col = __ldg(a.col + q0 + q);
+            const E x = col >= w0 && col < w1 ? in[col] : far(col);
+            s.add(kIntTerms, kDf && !FM::kVal ? V{} : cf[FM::kVal ? q0 + q : i], x);
+          }
+        }
+        if constexpr (kDf) {
+          float2 r = df_norm(s.h, s.l);
+          if (!FM::kVal)
+            r = df_scale(pat == 0 ? coef2 : len < 256 ? __ldg(a.lut2 + len) : static_cast<const float2 *>(a.coef)[i], r);
+          out[i] = r;
+          // others read the rows near the ends, with far diagonals any
+          if (GL > 0 || i - r0 < a.halo || r1 - i <= a.halo || a.ring_all) a.ring[(size_t)(l % 3) * a.n + i] = r;
+          __stcs((host ? a.hv : a.vv) + (size_t)l * a.n + i, df_to_double(r));
+        } else if constexpr (kMix) {
+          const float y = s.s * a.scale;
+          out[i] = y;
+          __stcs(a.vf + (size_t)l * a.n + i, y);
+        } else {
+          out[i] = s.s;
+          __stcs(a.vv + (size_t)l * a.n + i, s.s);
+          if (host) a.hv[(size_t)l * a.n + i] = s.s;
+        }
+      }
+    }
+    if (l < a.nlevel) diag_publish(a, b, a.base + (unsigned)l);
+  }
+}
+
+template <int F>
+const void *kernel_of(int w, int gl) {
+  if (w == 5) return gl ? (const void *)diag_kernel<F, 5, 1> : (const void *)diag_kernel<F, 5, 0>;
+  if (w == 7) return gl ? (const void *)diag_kernel<F, 7, 1> : (const void *)diag_kernel<F, 7, 0>;
+  return w == 9 && !gl ? (const void *)diag_kernel<F, 9, 0> : nullptr;
+}
+
+}  // namespace
+
+namespace mpkg {
+
+const void *diag_kernel_ptr(int form, int w, int gl) {
+  switch (form) {
+    case kDiagFma: return kernel_of<kDiagFma>(w, gl);
+    case kDiagFmaVal: return kernel_of<kDiagFmaVal>(w, gl);
+    case kDiagSep: return kernel_of<kDiagSep>(w, gl);
+    case kDiagSepVal: return kernel_of<kDiagSepVal>(w, gl);
+    case kDiagDf: return kernel_of<kDiagDf>(w, gl);
+    case kDiagDfVal: return kernel_of<kDiagDfVal>(w, gl);
+    case kDiagF32: return kernel_of<kDiagF32>(w, gl);
+    case kDiagBf16: return kernel_of<kDiagBf16>(w, gl);
+  }
+  return nullptr;
+}
+
+int diag_elem_bytes(int form) { return form >= kDiagF32 ? 4 : 8; }
+int diag_value_bytes(int form) {
+  switch (form) {
+    case kDiagFmaVal: case kDiagSepVal: case kDiagDfVal: return 8;
+    case kDiagF32: return 4;
+    case kDiagBf16: return 2;
+  }
+  return 0;
+}
+
+int diag_layout(int n, const int *ptr, const int *col, int form, int nsm, int smem, DiagLayout *out) {
+  DiagLayout &l = *out;
+  l.fits = false;
+  const int nslice = (n + 31) / 32;
+  const bool ring = form == kDiagDf || form == kDiagDfVal;
+  const long eb = diag_elem_bytes(form), vb = diag_value_bytes(form);
+  // the diagonals that more than half of 64 rows all over the matrix have
+  std::map<int, int> seen;
+  const int probes = std::min(n, 64);
+  for (int t = 0; t < probes; t++) {
+    const int i = (int)((0x9E3779B9ull * (unsigned long long)(t + 1)) % (unsigned long long)n);  // spread over all residues
+    if (ptr[i + 1] - ptr[i] > 2 * kDiagMax) return kOk;
+    for (int q = ptr[i]; q < ptr[i + 1]; q++) seen[col[q] - i]++;
+  }
+  l.w = 0;
+  for (const auto &s : seen)
+    if (2 * s.second > probes) {
+      if (l.w == kDiagMax) return kOk;
+      l.d[l.w++] = s.first;
+    }
+  if (l.w != 5 && l.w != 7 && l.w != 9) return kOk;  // the kernels there are: 2-D and 3-D stencils
+  const int W = l.w;
+  // slice-aligned row ranges of equal length: a slice costs the same with
+  // and without its holes
+  for (int i = 0; i < n; i++)
+    if (ptr[i + 1] - ptr[i] > 65535) return kOk;  // refused by the general wavefront
+  const int grid = l.grid = std::min(nsm, nslice);
+  l.lo.assign(grid + 1, 0);
+  for (int b = 1; b <= grid; b++) l.lo[b] = (int)std::min<long>(n, 32L * ((long)nslice * b / grid));
+  const int own = 32 * ((nslice + grid - 1) / grid);
+  // the halo holds all the diagonals or all but the outermost pair: the first
+  // fetches 2 halo rows per CTA and level, the second two per own row, so a
+  // halo beyond the own rows is taken only where the second does not do
+  const bool pair = W < 9 && l.d[0] < 0 && l.d[W - 1] > 0;
+  l.win_bytes = (int)((own * eb + 15) / 16 * 16);
+  int gl = -1;
+  for (const int t : {0, 1, 2}) {
+    const int g = t & 1;
+    if (g && !pair) continue;
+    const long halo = std::max({0, -l.d[g], l.d[W - 1 - g]});
+    if (t == 0 && pair && halo > own) continue;
+    const long hb = (halo * eb + 15) / 16 * 16;
+    if (2L * l.win_bytes + 3 * hb + (2L * own / 32 + 16) > smem) continue;
+    gl = g;
+    l.halo = (int)halo;
+    l.halo_bytes = (int)hb;
+    break;
+  }
+  if (gl < 0) return kOk;
+  l.gl = gl;
+  // patterns
+  l.pat.assign(nslice, 0);
+  std::map<std::vector<unsigned short>, int> known;
+  const unsigned short all = (unsigned short)((1 << W) - 1);
+  std::vector<unsigned short> m(32);
+  known[std::vector<unsigned short>(32, all)] = 0;
+  l.mask.assign(32, all);
+  long &irregular = l.irregular = 0;
+  for (int sl = 0; sl < nslice; sl++) {
+    bool ok = true;
+    std::fill(m.begin(), m.end(), 0);
+    bool full = sl * 32 + 32 <= n;
+    for (int i = sl * 32; i < std::min(n, sl * 32 + 32) && ok; i++) {
+      int u = 0;
+      unsigned bits = 0;
+      for (int q = ptr[i]; q < ptr[i + 1]; q++) {
+        while (u < W && l.d[u] != col[q] - i) u++;
+        if (u == W) { ok = false; break; }
+        bits |= 1u << u++;
+      }
+      m[i & 31] = (unsigned short)bits;
+      full &= bits == all;
+    }
+    if (!ok) {  // its rows run one entry after another: at most one slice in twenty
+      l.pat[sl] = kDiagIrregular;
+      if (++irregular * 20 > nslice) return kOk;
+      continue;
+    }
+    if (full) continue;
+    const auto f = known.find(m);
+    if (f != known.end()) {
+      l.pat[sl] = (unsigned short)f->second;
+      continue;
+    }
+    if (known.size() == kDiagIrregular) return kOk;
+    l.pat[sl] = (unsigned short)known.size();
+    known[m] = l.pat[sl];
+    l.mask.insert(l.mask.end(), m.begin(), m.end());
+  }
+  // per CTA: slice ranges, resident values, dependencies
+  l.own.assign(grid, make_int2(0, 0));
+  l.nres.assign(grid, 0);
+  std::vector<std::vector<int>> waits(grid);
+  auto owner = [&](int c) { return (int)(std::upper_bound(l.lo.begin(), l.lo.end() - 1, c) - l.lo.begin()) - 1; };
+  for (int b = 0; b < grid; b++) {
+    const int r0 = l.lo[b], r1 = l.lo[b + 1], ns = (r1 - r0 + 31) / 32;
+    const int reach_lo = std::max(0, -l.d[0]), reach_hi = std::max(0, l.d[W - 1]);
+    int ka = (reach_lo + 31) / 32, kb = std::max(ka, (r1 - reach_hi - r0) / 32);
+    if (ka > ns || kb > ns || ka >= kb) ka = kb = 0;
+    for (int k = ka; k < kb; k++)
+      if (l.pat[r0 / 32 + k] == kDiagIrregular) kb = k;
+    l.own[b] = make_int2(ka, kb);
+    if (vb) {
+      const long room = smem - 2L * l.win_bytes - 3L * l.halo_bytes - (2L * ns + 15) / 16 * 16;
+      l.nres[b] = (int)std::min<long>(ns, room / (vb * W * 32));
+    }
+    std::vector<int> &wt = waits[b];
+    int last = -1;
+    for (int q = ptr[r0]; q < ptr[r1]; q++) {
+      const int c = col[q];
+      if (c >= r0 && c < r1) continue;
+      if (last >= 0 && c >= l.lo[last] && c < l.lo[last + 1]) continue;
+      last = owner(c);
+      wt.push_back(last);
+    }
+    std::sort(wt.begin(), wt.end());
+    wt.erase(std::unique(wt.begin(), wt.end()), wt.end());
+  }
+  if (ring) {  // a ring slot is reused: wait for the readers of the own rows too
+    const std::vector<std::vector<int>> reads(waits);
+    for (int c = 0; c < grid; c++)
+      for (int b : reads[c]) waits[b].push_back(c);
+  }
+  l.dptr.assign(grid + 1, 0);
+  l.didx.clear();
+  for (int b = 0; b < grid; b++) {
+    std::vector<int> &wt = waits[b];
+    std::sort(wt.begin(), wt.end());
+    wt.erase(std::unique(wt.begin(), wt.end()), wt.end());
+    for (int c : wt) {
+      l.didx.push_back(c);
+      l.reach = std::max<long>(l.reach, std::abs(c - b));
+    }
+    l.dptr[b + 1] = (int)l.didx.size();
+  }
+  if (l.didx.empty()) l.didx.push_back(0);
+  l.fits = true;
+  return kOk;
+}
+
+}  // namespace mpkg
