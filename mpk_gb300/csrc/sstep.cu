@@ -158,36 +158,47 @@ __global__ void axpby_kernel(int n, double a, const double *__restrict__ x, doub
 // [4] r.r, [5] p.p.
 constexpr int kScalars = 6;
 
-// r.r and p.p from the per-CTA partial sums (one warp: lane j sums
-// partials j, j+32, ... in order, then a fixed butterfly, so the same bits
-// on every run), and the norms that scale the next basis.
-__global__ void norms_kernel(int nb, const double *__restrict__ part, double *__restrict__ sc) {
-  if (blockIdx.x != 0 || threadIdx.x >= 32) return;
-  const int lane = threadIdx.x;
-  double rr = 0.0, pp = 0.0;
-  for (int k = lane; k < nb; k += 32) {
-    rr += part[k];
-    pp += part[nb + k];
+// r.r and p.p from the per-CTA partial sums, a warp each (lane j sums
+// partials j, j+32, ... in order, eight loads in flight, then a fixed
+// butterfly, so the same bits on every run), and the norms that scale the next
+// basis.  Two warps call it; sc is written by thread 0.
+constexpr int kNormThreads = 64;
+__device__ __forceinline__ void reduce_norms(int nb, const double *__restrict__ part, double *sc) {
+  __shared__ double s_pp;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double *q = part + (warp ? nb : 0);
+  double v = 0.0;
+  for (int k = lane; k < nb; k += 256) {
+    double t[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+      if (k + 32 * u < nb) t[u] = __ldg(q + k + 32 * u);
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+      if (k + 32 * u < nb) v += t[u];
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    rr += __shfl_xor_sync(0xFFFFFFFFu, rr, o);
-    pp += __shfl_xor_sync(0xFFFFFFFFu, pp, o);
-  }
-  if (lane != 0) return;
-  const double pn = sqrt(pp), rn = sqrt(rr);
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+  if (threadIdx.x == 32) s_pp = v;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  const double pp = s_pp, pn = sqrt(pp), rn = sqrt(v);
   sc[0] = pn;
   sc[1] = rn;
   sc[2] = 1.0 / pn;
   sc[3] = 1.0 / rn;
-  sc[4] = rr;
+  sc[4] = v;
   sc[5] = pp;
+}
+
+__global__ void __launch_bounds__(kNormThreads) norms_kernel(int nb, const double *__restrict__ part, double *sc) {
+  reduce_norms(nb, part, sc);
 }
 
 // The whole solve as one graph: a conditional WHILE node whose body is
 // one outer iteration, ended by decide_kernel (one warp), which counts the
 // iteration, records the P block of the Gram matrix for the host's
 // condition number (a ring in page-locked memory, with a progress count),
-// asks for a restart when p.p is not positive, and sets the loop
+// asks for a restart when p.p is not positive (basis_start_kernel), and sets the loop
 // condition: more iterations allowed, progress made, |r| above tol |b|.
 // The count of iterations bounds the loop by max_outer.
 struct LoopState {
@@ -195,20 +206,14 @@ struct LoopState {
 };
 constexpr int kCondRing = 512;
 
-__global__ void restart_kernel(int n, const LoopState *__restrict__ st, const double *__restrict__ r,
-                               double *__restrict__ p, double *__restrict__ sc) {
-  if (!st->restart) return;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = r[i];
-  if (blockIdx.x == 0 && threadIdx.x == 0) {  // |p| = |r|, p.p = r.r
-    sc[0] = sc[1];
-    sc[2] = sc[3];
-    sc[5] = sc[4];
-  }
-}
-
-__global__ void decide_kernel(int s, int m, const int *__restrict__ flag, const double *__restrict__ sc,
-                              const double *__restrict__ g, int max_outer, double rtol, LoopState *st, double *ring,
-                              int *progress, cudaGraphConditionalHandle loop) {
+// The norms of the next iteration, then the decision (warp 0).
+__global__ void __launch_bounds__(kNormThreads) decide_kernel(int nb, const double *__restrict__ part, int s, int m,
+                                                          const int *__restrict__ flag, double *sc,
+                                                          const double *__restrict__ g, int max_outer, double rtol,
+                                                          LoopState *st, double *ring, int *progress,
+                                                          cudaGraphConditionalHandle loop) {
+  reduce_norms(nb, part, sc);
+  if (threadIdx.x >= 32) return;
   const int lane = threadIdx.x, mp = s + 1, o = st->outer;
   double *slot = ring + (size_t)(o % kCondRing) * mp * mp;
   for (int k = lane; k < mp * mp; k += 32) slot[k] = g[(k / mp) * m + k % mp];
@@ -226,12 +231,23 @@ __global__ void decide_kernel(int s, int m, const int *__restrict__ flag, const 
   cudaGraphSetConditional(loop, more ? 1u : 0u);
 }
 
-__global__ void basis_start_kernel(int n, const double *__restrict__ p, const double *__restrict__ r,
-                                   const double *__restrict__ sc, float *__restrict__ y0, float *__restrict__ yr) {
-  const double ip = sc[2], ir = sc[3];
+// The basis' first columns, p / |p| and r / |r|; with st and a restart asked
+// for, p is r first (the scalars of p follow those of r: with a restart no
+// CTA reads the ones that thread 0 rewrites).
+__global__ void basis_start_kernel(int n, double *__restrict__ p, const double *__restrict__ r, double *sc,
+                                   const LoopState *__restrict__ st, float *__restrict__ y0, float *__restrict__ yr) {
+  const bool restart = st && st->restart;
+  const double ir = sc[3], ip = restart ? ir : sc[2];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    y0[i] = (float)(p[i] * ip);
-    yr[i] = (float)(r[i] * ir);
+    const double rv = r[i], pv = restart ? rv : p[i];
+    if (restart) p[i] = rv;
+    y0[i] = (float)(pv * ip);
+    yr[i] = (float)(rv * ir);
+  }
+  if (restart && blockIdx.x == 0 && threadIdx.x == 0) {  // |p| = |r|, p.p = r.r
+    sc[0] = sc[1];
+    sc[2] = sc[3];
+    sc[5] = sc[4];
   }
 }
 
@@ -378,17 +394,29 @@ __global__ void __launch_bounds__(kThreads) basis_wave_kernel(BasisWave w, Sell 
   }
 }
 
-// Gram matrix G = Y^T Y of the FP32 basis.  Every product a*b of two FP32
-// values is exact in FP64 (48-bit mantissa).  F64: the products are
-// summed with FP64 FMAs (the FP64 Gram of the s-step method).  !F64: each
-// product is split exactly into p + e (p = a*b rounded, e = fma(a, b, -p))
-// and summed in double-float on the FP32 pipes (a two-sum on the high
-// parts, errors and low parts added; about 2^-46 relative to the sum of
-// |products|), for GB300 whose FP64 pipe runs at 1/64 of FP32.
-// A CTA stages a tile of rows of all columns in shared memory; thread t
-// accumulates pair t of the upper triangle with four independent sums;
-// per-CTA partials (FP64) are summed in a fixed order by gram_reduce_kernel.
+// Gram matrix G = Y^T Y of the FP32 basis.  A product a*b of two FP32 values
+// is split exactly into p + e (p = a*b rounded, e = fma(a, b, -p)) and summed
+// on the FP32 pipes, since GB300's FP64 pipe runs at 1/64 of FP32: in
+// double-float over all the CTA's rows (!F64: a two-sum on the high parts,
+// errors and low parts added, about 2^-46 relative to the sum of |products|),
+// or (F64, the FP64 Gram of the s-step method) over a tile's 64 products with
+// the errors of every addition kept (gram_acc4), then into FP64.  That is no
+// further from the exact sum than FP64 fused multiply-adds: 17 correlated
+// columns, rms over the pairs relative to the columns' norms, three
+// distributions together, at 1 K / 30 K / 262 K / 885 K rows 4.6e-17 /
+// 5.0e-17 / 5.9e-17 / 5.5e-17 against 5.5e-17 / 5.2e-17 / 8.1e-17 / 2.8e-16.
+// Tiles with a nonzero value outside 2^-45 .. 2^60, where a product or its
+// error could leave the FP32 range, are summed with FP64 fused multiply-adds.
+// A CTA stages a tile of rows of all columns in shared memory, thread t
+// accumulates pair t of the upper triangle; per-CTA partials (FP64) are summed
+// in a fixed order by gram_reduce_kernel.
+//
+// What bounds it: the FP32 instructions, 22 a product (F64).  153 pairs, 262 K
+// rows 45 us, 885 K rows 137 us, against 86 and 268 with FP64 fused
+// multiply-adds, whose pipe bounds those; without the compensation of the low
+// sums (10 instructions) 30 and 86 us, but 5 times further off.
 constexpr int kGramRows = 64;
+constexpr int kGramStride = kGramRows + 4;  // 16-byte rows, eight columns in different banks
 thread_local bool g_gram_f64 = true;  // mpkg_sstep_gram: FP64 (default) or double-float Gram
 thread_local bool g_device_loop = true;  // mpkg_sstep_loop: device-side (default) or host-side outer loop
 thread_local bool g_basis_mpk = false;   // mpkg_sstep_basis: s launches (default) or one matrix powers launch
@@ -401,47 +429,95 @@ __device__ __forceinline__ void gram_acc(float a, float b, float &sh, float &sl)
   sl = __fadd_rn(sl, __fadd_rn(err, e));
 }
 
+// s + b rounded into s; returns the rounding error (two-sum).
+__device__ __forceinline__ float two_sum(float &s, float b) {
+  const float t = __fadd_rn(s, b), bp = __fadd_rn(t, -s);
+  const float err = __fadd_rn(__fadd_rn(s, -__fadd_rn(t, -bp)), __fadd_rn(b, -bp));
+  s = t;
+  return err;
+}
+
+// The sum h + l + m + c of products: h takes the rounded products, l the
+// errors of its additions, m the errors of the products, c those of l and m.
+__device__ __forceinline__ void gram_acc4(float a, float b, float &h, float &l, float &m, float &c) {
+  const float p = __fmul_rn(a, b), e = __fmaf_rn(a, b, -p);
+  const float el = two_sum(l, two_sum(h, p));
+  c = __fadd_rn(c, __fadd_rn(el, two_sum(m, e)));
+}
+
+// Exact float -> double in integer arithmetic (the conversion shares the FP64 pipe).
+__device__ __forceinline__ double ss_widen(float f) {
+  const unsigned int u = __float_as_uint(f);
+  const unsigned int e = (u >> 23) & 0xFF;
+  const unsigned int sgn = u & 0x80000000u;
+  const unsigned int bias = e == 0xFF ? (1792u << 20) : (896u << 20);
+  const unsigned int hi = e == 0 ? sgn : (sgn | (((u >> 3) & 0x0FFFFFFFu) + bias));
+  const unsigned int lo = e == 0 ? 0u : (u << 29);
+  return __hiloint2double((int)hi, (int)lo);
+}
+
 template <bool F64>
 __global__ void __launch_bounds__(kThreads) gram_kernel(int n, int ncol, const float *__restrict__ y,
                                                         double *__restrict__ part) {
-  // one padding word per column: the threads of a warp read up to 17
-  // different columns at the same row, which would otherwise share a bank.
-  // F64 stages the values already widened, so that each is converted once
-  // per tile rather than once per pair (the conversion shares the FP64 pipe)
-  using Stage = typename std::conditional<F64, double, float>::type;
-  __shared__ Stage tile[kMaxCols][kGramRows + 1];
+  __shared__ __align__(16) float tile[kMaxCols * kGramStride];
   const int npair = ncol * (ncol + 1) / 2;
   int pa = 0, pb = 0;
   {
     int t = threadIdx.x, a = 0;
     while (a < ncol && t >= ncol - a) { t -= ncol - a; a++; }
-    pa = a;
-    pb = a + t;
+    pa = a < ncol ? a : 0;
+    pb = a < ncol ? a + t : 0;
   }
+  const float4 *ta = reinterpret_cast<const float4 *>(tile + pa * kGramStride);
+  const float4 *tb = reinterpret_cast<const float4 *>(tile + pb * kGramStride);
   float h[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  double acc = 0.0;
   for (long r0 = (long)blockIdx.x * kGramRows; r0 < n; r0 += (long)gridDim.x * kGramRows) {
     __syncthreads();
+    int wide = 0;
     for (int e = threadIdx.x; e < ncol * kGramRows; e += blockDim.x) {
       const int c = e / kGramRows, rr = e % kGramRows;
-      tile[c][rr] = (Stage)(r0 + rr < n ? y[(size_t)c * n + r0 + rr] : 0.f);
+      const float v = r0 + rr < n ? y[(size_t)c * n + r0 + rr] : 0.f;
+      tile[c * kGramStride + rr] = v;
+      const unsigned int u = __float_as_uint(v) & 0x7FFFFFFFu;
+      wide |= u != 0 && u - (82u << 23) >= (105u << 23);
     }
-    __syncthreads();
-    if ((int)threadIdx.x < npair) {  // four independent partial sums per thread
+    if (F64) wide = __syncthreads_or(wide);
+    else __syncthreads();
+    if ((int)threadIdx.x >= npair) continue;
+    if (F64 && wide) {
+      for (int rr = 0; rr < kGramRows; rr++)
+        acc = fma((double)tile[pa * kGramStride + rr], (double)tile[pb * kGramStride + rr], acc);
+      continue;
+    }
+    if (F64) {
+      float h0 = 0.f, l0 = 0.f, m0 = 0.f, c0 = 0.f;
 #pragma unroll 4
-      for (int rr = 0; rr < kGramRows; rr += 4) {
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          if (F64) acc[u] = fma((double)tile[pa][rr + u], (double)tile[pb][rr + u], acc[u]);
-          else gram_acc((float)tile[pa][rr + u], (float)tile[pb][rr + u], h[u], lo[u]);
-        }
+      for (int q = 0; q < kGramRows / 4; q++) {  // four rows a step
+        const float4 va = ta[q], vb = tb[q];
+        gram_acc4(va.x, vb.x, h0, l0, m0, c0);
+        gram_acc4(va.y, vb.y, h0, l0, m0, c0);
+        gram_acc4(va.z, vb.z, h0, l0, m0, c0);
+        gram_acc4(va.w, vb.w, h0, l0, m0, c0);
+      }
+      acc += ss_widen(h0);
+      acc += (ss_widen(l0) + ss_widen(m0)) + ss_widen(c0);
+    } else {
+#pragma unroll 4
+      for (int q = 0; q < kGramRows / 4; q++) {
+        const float4 va = ta[q], vb = tb[q];
+        gram_acc(va.x, vb.x, h[0], lo[0]);
+        gram_acc(va.y, vb.y, h[1], lo[1]);
+        gram_acc(va.z, vb.z, h[2], lo[2]);
+        gram_acc(va.w, vb.w, h[3], lo[3]);
       }
     }
   }
   if ((int)threadIdx.x < npair) {
-    double s = 0.0;
-    for (int k = 0; k < 4; k++) s += F64 ? acc[k] : (double)h[k] + (double)lo[k];
-    part[(size_t)blockIdx.x * npair + threadIdx.x] = s;
+    double s = acc;
+    if (!F64)
+      for (int k = 0; k < 4; k++) s += (double)h[k] + (double)lo[k];
+    part[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = s;  // [pair][CTA]
   }
 }
 
@@ -453,7 +529,7 @@ __global__ void gram_reduce_kernel(int nblk, int ncol, const double *__restrict_
   const int t = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (t >= npair) return;
   double s = 0.0;
-  for (int b = lane; b < nblk; b += 32) s += part[(size_t)b * npair + t];
+  for (int b = lane; b < nblk; b += 32) s += part[(size_t)t * nblk + b];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
   if (lane == 0) {
     int a = 0, u = t;
@@ -528,16 +604,6 @@ __global__ void coeff_kernel(int s, const double *__restrict__ g, const double *
 // products and their sums in double-float on the FP32 pipes (each
 // coefficient split into two floats; products exact up to the low part's
 // rounding, about 2^-46 relative), then one FP64 add into x per row.
-__device__ __forceinline__ double ss_widen(float f) {  // exact float -> double in integer arithmetic
-  const unsigned int u = __float_as_uint(f);
-  const unsigned int e = (u >> 23) & 0xFF;
-  const unsigned int sgn = u & 0x80000000u;
-  const unsigned int bias = e == 0xFF ? (1792u << 20) : (896u << 20);
-  const unsigned int hi = e == 0 ? sgn : (sgn | (((u >> 3) & 0x0FFFFFFFu) + bias));
-  const unsigned int lo = e == 0 ? 0u : (u << 29);
-  return __hiloint2double((int)hi, (int)lo);
-}
-
 __device__ __forceinline__ void ss_mac(float ch, float cl, float v, float &sh, float &sl) {
   const float p = __fmul_rn(ch, v);
   float e = __fmaf_rn(ch, v, -p);
@@ -1202,9 +1268,9 @@ int mpkg_sstep_cg(int n, const int *ptr, const int *col, const double *val, cons
   }
   // one outer iteration: basis, Gram, coefficient steps, update, true
   // residual, scalars for the next iteration
-  auto iteration = [&](cudaStream_t cs) {
+  auto iteration = [&](cudaStream_t cs, const LoopState *st) {
     float *Y = y.p;
-    basis_start_kernel<<<nb, kThreads, 0, cs>>>(n, dp.p, dr.p, dsc.p, Y, Y + (size_t)(s + 1) * n);
+    basis_start_kernel<<<nb, kThreads, 0, cs>>>(n, dp.p, dr.p, dsc.p, st, Y, Y + (size_t)(s + 1) * n);
     if (basis_mpk) {
       bl.launch(a.sell(), Y, cs);
     } else for (int j = 0; j < s; j++) {
@@ -1214,13 +1280,13 @@ int mpkg_sstep_cg(int n, const int *ptr, const int *col, const double *val, cons
                                                  rstep ? Y + (size_t)(s + 2 + j) * n : nullptr, (float)th[j],
                                                  (float)(1.0 / sg[j]));
     }
-    if (g_gram_f64) gram_kernel<true><<<gblk, kThreads, 0, cs>>>(n, m, Y, gpart.p);
-    else gram_kernel<false><<<gblk, kThreads, 0, cs>>>(n, m, Y, gpart.p);
+    const int gthr = (npair + 31) / 32 * 32;
+    if (g_gram_f64) gram_kernel<true><<<gblk, gthr, 0, cs>>>(n, m, Y, gpart.p);
+    else gram_kernel<false><<<gblk, gthr, 0, cs>>>(n, m, Y, gpart.p);
     gram_reduce_kernel<<<(npair * 32 + kThreads - 1) / kThreads, kThreads, 0, cs>>>(gblk, m, gpart.p, dg.p);
     coeff_kernel<<<1, 32, 0, cs>>>(s, dg.p, dth.p, dsg.p, dsc.p, dxh.p, dph.p, drh.p, dflag.p);
     combine_kernel<<<nb, kThreads, 0, cs>>>(n, m, Y, dxh.p, dph.p, dx.p, dp.p, part.p + nb);
     resid_kernel<<<nb, kThreads, 0, cs>>>(n, a.sell(), dx.p, db.p, dr.p, part.p);
-    norms_kernel<<<1, 32, 0, cs>>>(nb, part.p, dsc.p);
   };
   int outer = 0, steps = 0, breakdowns = 0;
   double cond_max = 0.0;
@@ -1274,10 +1340,10 @@ int mpkg_sstep_cg(int n, const int *ptr, const int *col, const double *val, cons
   if (device_loop) {
     SS_TRY(cudaMemsetAsync(dstate.p, 0, sizeof(LoopState), gr.st));
     device_loop = build_device_loop(gr, [&](cudaStream_t cs, cudaGraphConditionalHandle h) {
-      restart_kernel<<<nb, kThreads, 0, cs>>>(n, reinterpret_cast<const LoopState *>(dstate.p), dr.p, dp.p, dsc.p);
-      iteration(cs);
-      decide_kernel<<<1, 32, 0, cs>>>(s, m, dflag.p, dsc.p, dg.p, max_outer, rtol,
-                                       reinterpret_cast<LoopState *>(dstate.p), lh.d_ring, lh.d_progress, h);
+      LoopState *st = reinterpret_cast<LoopState *>(dstate.p);
+      iteration(cs, st);
+      decide_kernel<<<1, kNormThreads, 0, cs>>>(nb, part.p, s, m, dflag.p, dsc.p, dg.p, max_outer, rtol, st, lh.d_ring,
+                                            lh.d_progress, h);
     });
   }
   if (device_loop) {
@@ -1317,7 +1383,8 @@ int mpkg_sstep_cg(int n, const int *ptr, const int *col, const double *val, cons
     // with one copy back of the flags, r.r, p.p and the Gram matrix
     cudaStream_t cs = gr.st;
     SS_TRY(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-    iteration(cs);
+    iteration(cs, nullptr);
+    norms_kernel<<<1, kNormThreads, 0, cs>>>(nb, part.p, dsc.p);
     cudaMemcpyAsync(hbuf.p, dflag.p, sizeof(int) * 2, cudaMemcpyDeviceToHost, cs);
     cudaMemcpyAsync(reinterpret_cast<char *>(hbuf.p) + hb_sc, dsc.p + 4, sizeof(double) * 2, cudaMemcpyDeviceToHost,
                     cs);
