@@ -52,12 +52,14 @@ __global__ void __launch_bounds__(256) spmv_level_kernel(int n, const int *__res
   const int j0 = ptr[i], j1 = ptr[i + 1];
   const double a = VALUED ? 0.0 : coef[i];  // 1/deg, rounded on the host exactly as 1.0/deg
   double s = 0.0;
-  if (j0 < j1) s = row_first<ARITH>(VALUED ? coef[j0] : a, x[col[j0]]);
-  int j = j0 + 1;
+  int j = j0;
   if (ARITH == MPKG_ARITH_SEPARATE) {
     // three products of four on the integer pipes, the fourth beside them on
     // the FP64 pipe (97 x 96 x 95 diffusion, 6 levels: 175 us with all on the
-    // FP64 pipe, 136 with none, 125 so; of 2, 3, 5, 6: 164, 130, 129, 152)
+    // FP64 pipe, 136 with none, 128 so; groups of 2, 3, 5, 6: 164, 130, 129,
+    // 152).  With the first product ahead of the groups that is 124, but small
+    // launches, bound by the row's chain of loads, lose a fifth (100 x 101
+    // 1/deg, 6 levels: 25 / 31); so do FMA rows, which keep the plain loop.
     constexpr int G = 4;
     for (; j + G <= j1; j += G) {
       double xv[G], v[G];
@@ -66,8 +68,9 @@ __global__ void __launch_bounds__(256) spmv_level_kernel(int n, const int *__res
         xv[u] = x[col[j + u]];
         v[u] = VALUED ? coef[j + u] : a;
       }
+      s = j == j0 ? row_first<ARITH>(v[0], xv[0]) : row_next<ARITH>(s, v[0], xv[0]);
 #pragma unroll
-      for (int u = 0; u < G; u++) s = u < G - 1 ? row_next<ARITH>(s, v[u], xv[u]) : row_term<ARITH>(s, v[u], xv[u]);
+      for (int u = 1; u < G; u++) s = u < G - 1 ? row_next<ARITH>(s, v[u], xv[u]) : row_term<ARITH>(s, v[u], xv[u]);
     }
   }
   for (; j < j1; j++) s = row_next<ARITH>(s, VALUED ? coef[j] : a, x[col[j]]);
