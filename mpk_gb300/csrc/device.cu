@@ -2078,7 +2078,7 @@ struct mpkg_plan {
   bool wave_uni = false;  // pattern-compressed offsets (plans with matrix values)
   DiagArgs dg{};          // rows on a few diagonals: the diagonal wavefront
   bool dg_on = false;
-  int dg_form = 0, dg_w = 0, dg_gl = 0, dg_threads = 0;
+  int dg_form = 0, dg_w = 0, dg_mode = 0, dg_threads = 0;
   // batched block-vector form
   BatchArgs batch{};
   int batch_lpr = 0, batch_vw = 0, batch_nmat = 0;
@@ -2385,7 +2385,7 @@ int launch_diag(mpkg_plan *p, double *vv, double *hv, float *vf, float scale, in
   a.base = p->wave.base; a.stall = p->wave.stall; a.flags = p->wave.flags; a.err = err;
   a.vv = vv; a.hv = hv; a.vf = vf; a.scale = scale;
   void *args[] = {&a};
-  CUDA_TRY(cudaLaunchCooperativeKernel(diag_kernel_ptr(p->dg_form, p->dg_w, p->dg_gl), dim3(a.nblk),
+  CUDA_TRY(cudaLaunchCooperativeKernel(diag_kernel_ptr(p->dg_form, p->dg_w, p->dg_mode), dim3(a.nblk),
                                        dim3(p->dg_threads), args, (size_t)a.smem, st));
   return kOk;
 }
@@ -3467,15 +3467,15 @@ int diag_setup(mpkg_plan *p, int form, const int *ptr, const int *col, const dou
   if (!coop) return kOk;
   const int smem = optin - 1024;  // less the kernel's static part
   DiagLayout l;
-  int rc = diag_layout(n, ptr, col, form, nsm, smem, &l);
+  int rc = diag_layout(n, ptr, col, p->nlevel, form, nsm, smem, &l);
   if (rc || !l.fits) return rc;
-  const void *fn = diag_kernel_ptr(form, l.w, l.gl);
+  const void *fn = diag_kernel_ptr(form, l.w, l.mode);
   CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kDiagThreads, smem));
   if ((long)per_sm * nsm < l.grid) return kOk;
   DiagArgs &a = p->dg;
-  a.n = n; a.nlevel = p->nlevel; a.nblk = l.grid; a.halo = l.halo; a.smem = smem; a.win_bytes = l.win_bytes;
-  a.halo_bytes = l.halo_bytes;
+  a.n = n; a.nlevel = p->nlevel; a.nblk = l.grid; a.halo = l.halo; a.smem = smem;
+  a.depth = l.depth; a.grow = l.grow; a.win_at = l.win_at; a.second = l.second;
   a.ring_all = l.irregular > 0;
   for (int u = 0; u < l.w; u++) {
     a.d[u] = l.d[u];
@@ -3550,11 +3550,9 @@ int diag_setup(mpkg_plan *p, int form, const int *ptr, const int *col, const dou
   p->wave_grid = l.grid;
   p->pipe_grid = l.grid;
   p->pipe_reach = (int)l.reach;
-  p->rows_computed = (long)n * p->nlevel;
-  p->dg_form = form; p->dg_w = l.w; p->dg_gl = l.gl;
-  int slices = 0;  // a warp per slice, as far as they go
-  for (int b = 0; b < l.grid; b++) slices = std::max(slices, (l.lo[b + 1] - l.lo[b] + 31) / 32);
-  p->dg_threads = std::min(kDiagThreads, std::max(128, 32 * slices));
+  p->rows_computed = l.rows;
+  p->dg_form = form; p->dg_w = l.w; p->dg_mode = l.mode;
+  p->dg_threads = std::min(kDiagThreads, std::max(128, 32 * l.slices));  // a warp per slice, as far as they go
   p->dg_on = true;
   *done = true;
   return kOk;

@@ -17,6 +17,15 @@
 // [slice][diagonal][lane]; shared memory keeps as many slices of them as fit
 // beside the windows for the whole call.
 //
+// A level costs some 4.5 K cycles of hand-over between CTAs, whatever its
+// size.  Where the rows reach few slices a CTA exchanges every `depth` levels
+// instead: it fetches depth times the halo and computes the levels between on
+// so many slices of its neighbours too, as many levels as the cost below
+// prefers (us with 1, 2, 3, 4 levels: 100^2 1/deg k = 4 12.4 / 8.7 / 10.2 /
+// 8.4; 200 x 201 k = 6 18.5 / 14.4 / 15.0 / 16.4; mixed FP32 9-point 120 x 110
+// k = 8 20.6 / 14.4 / 13.9 / 12.4; FP64 9-point 1023 x 769 k = 6 80 / 85 / 92 /
+// 100).
+//
 // Row sums run over the entries in CSR order with the arithmetic of
 // wave_kernel, wave_df_kernel and wave_mix_kernel: the same bits.
 //
@@ -26,9 +35,9 @@
 // hand-over (release after the barrier 1.5-3 K, the neighbours' flags 1-2 K,
 // the halo 1 K).  Against the general wavefront, which reads every index and
 // its columns through L1 (us): 128^3 1/deg k = 8 228 / 249; 100^2 1/deg k = 4
-// 12.3 / 14.6; 9-point FP64 1400 x 1300 k = 8 264 / 293; double-float 1/deg
-// 101 x 97 x 89 k = 8 79 / 105; mixed FP32 120 x 110 x 100 k = 8 69 / 141, BF16
-// 9-point 701 x 699 k = 4 18.4 / 40.8.
+// 8.2 / 15.1; 9-point FP64 1400 x 1300 k = 8 266 / 293; double-float 1/deg
+// 101 x 97 x 89 k = 8 79 / 105; mixed FP32 120 x 110 x 100 k = 8 68 / 141, BF16
+// 9-point 701 x 699 k = 4 17.7 / 40.9.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -138,12 +147,14 @@ __device__ __forceinline__ void diag_publish(const DiagArgs &a, int b, unsigned 
 
 constexpr int kXGroups = 8;  // host execution: CTA groups that copy x in turn (as wave_kernel)
 
-template <int F, int W, int GL>
+// MODE: kDiagAll, kDiagPair or kDiagDeep.
+template <int F, int W, int MODE>
 __global__ void __launch_bounds__(kDiagThreads, 1) diag_kernel(const __grid_constant__ DiagArgs a) {
   using FM = Form<F>;
   using E = typename FM::Elem;
   using V = typename FM::Val;
   constexpr bool kDf = FM::kArith == MPKG_ARITH_DF64, kMix = FM::kArith < 0;
+  constexpr bool kPair = MODE == kDiagPair, kDeep = MODE == kDiagDeep;
   extern __shared__ __align__(128) unsigned char dg_smem[];
   __shared__ int s_abort;
   __shared__ __align__(8) unsigned long long s_bar;
@@ -152,26 +163,30 @@ __global__ void __launch_bounds__(kDiagThreads, 1) diag_kernel(const __grid_cons
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nt = blockDim.x, nw = nt >> 5;
   // shared memory: patterns, values, then the two windows at the end
   unsigned short *s_pat = reinterpret_cast<unsigned short *>(dg_smem);
-  V *s_val = reinterpret_cast<V *>(dg_smem + ((2 * ns + 15) & ~15));
+  // slices before and after the own ones that it computes too at the first
+  // level after an exchange
+  const int depth = kDeep ? a.depth : 1, more = (depth - 1) * a.grow;
+  const int xlo = min(s0, more), xhi = min(((a.n + 31) >> 5) - s0 - ns, more);
+  s_pat += xlo;  // of the first own slice, as s_val and vals
+  V *s_val = reinterpret_cast<V *>(dg_smem + ((2 * (xlo + ns + xhi) + 15) & ~15)) + xlo * W * 32;
   const V *vals = reinterpret_cast<const V *>(a.vals) + (size_t)s0 * W * 32;
-  const int nres = FM::kVal ? a.nres[b] : 0;
-  // halo, window A, halo, window B, halo: the middle one serves both
-  unsigned char *wins = dg_smem + a.smem - 2 * a.win_bytes - 2 * a.halo_bytes;
+  const int nres = FM::kVal ? a.nres[b] - xlo : 0;
+  unsigned char *wins = dg_smem + a.win_at;
   const int w0 = max(0, r0 - a.halo), w1 = min(a.n, r1 + a.halo);
   if (threadIdx.x == 0) {
     s_abort = 0;
     if (FM::kVal) {  // the values stream in while the window is filled
       mbar_init(&s_bar);
-      const unsigned bytes = (unsigned)(nres * W * 32 * (int)sizeof(V));
-      mbar_expect(&s_bar, bytes);
-      for (unsigned o = 0; o < bytes; o += 32768)
+      constexpr int kSlice = W * 32 * (int)sizeof(V);
+      mbar_expect(&s_bar, (unsigned)((nres + xlo) * kSlice));
+      for (int o = -xlo * kSlice; o < nres * kSlice; o += 32768)
         bulk_g2s(reinterpret_cast<unsigned char *>(s_val) + o, reinterpret_cast<const unsigned char *>(vals) + o,
-                 min(32768u, bytes - o), &s_bar);
+                 (unsigned)min(32768, nres * kSlice - o), &s_bar);
     }
   }
-  for (int k = threadIdx.x; k < ns; k += nt) s_pat[k] = a.pat[s0 + k];
+  for (int k = (int)threadIdx.x - xlo; k < ns + xhi; k += nt) s_pat[k] = a.pat[s0 + k];
   auto level = [&](int l) -> const E * {  // where other CTAs' rows of level l are read
-    if constexpr (kDf) return a.ring + (size_t)(l % 3) * a.n;
+    if constexpr (kDf) return a.ring + (size_t)(l / depth % 3) * a.n;
     else if constexpr (kMix) return a.vf + (size_t)l * a.n;
     else return a.vv + (size_t)l * a.n;
   };
@@ -211,39 +226,45 @@ __global__ void __launch_bounds__(kDiagThreads, 1) diag_kernel(const __grid_cons
   if constexpr (kDf && !FM::kVal) coef2 = __ldg(a.lut2 + W);
   __syncthreads();
   if (FM::kVal && !tr_wait(&s_bar, 0, a.err)) return;
-  for (int l = 1; l <= a.nlevel; l++) {
-    const int second = a.win_bytes + a.halo_bytes;
-    E *in = reinterpret_cast<E *>(wins + (l & 1 ? 0 : second)) - r0;
-    E *out = reinterpret_cast<E *>(wins + (l & 1 ? second : 0)) - r0;
+  for (int l = 1, left = -1; l <= a.nlevel; l++, left--) {
+    // `left` levels follow before the next exchange; each needs a.grow slices
+    // more of this one on either side
+    const bool exchange = !kDeep || left < 0;
+    if (exchange) left = min(depth, a.nlevel + 1 - l) - 1;
+    const int lo = kDeep ? -min(xlo, left * a.grow) : 0, hi = ns + (kDeep ? min(xhi, left * a.grow) : 0);
+    E *in = reinterpret_cast<E *>(wins + (l & 1 ? 0 : a.second)) - r0;
+    E *out = reinterpret_cast<E *>(wins + (l & 1 ? a.second : 0)) - r0;
     const E *prev = level(l - 1);
     auto far = [&](int i) -> E { return kDf && l == 1 ? first(i) : __ldcg(prev + i); };
+    const bool wait = exchange && l > 1;
     for (int part = 0; part < 2; part++) {
-      // part 0: slices [own0, own1), which read own rows only; part 1: the
-      // others, once the CTAs that own their columns have published them
-      const int cnt = part == 0 ? own1 - own0 : ns - (own1 - own0);
-      auto at = [&](int j) { return part == 0 ? own0 + j : j < own0 ? j : j + (own1 - own0); };
+      // part 0: slices [own0, own1), which read own rows only; part 1: the others,
+      // once the CTAs that own the rows around them have published those
+      const int cut = part == 0 ? own1 : own0, end = part == 0 ? own1 : hi - (own1 - own0);
+      auto at = [&](int j) { return j < cut ? j : j + (own1 - own0); };
+      const int j0 = (part == 0 ? own0 : lo) + warp;
       E g0{}, g1{};
       auto fetch = [&](int j) {  // the far entries of slice j
-        if (GL > 0 && j < cnt) {
-          const int i = r0 + 32 * at(j) + lane, lo = i + a.d[0], hi = i + a.d[W - 1];
-          if (lo >= 0 && i < r1) g0 = far(lo);
-          if (hi < a.n) g1 = far(hi);  // hi > i
+        if (kPair && j < end) {
+          const int i = r0 + 32 * at(j) + lane, c0 = i + a.d[0], c1 = i + a.d[W - 1];
+          if (c0 >= 0 && i < a.n) g0 = far(c0);
+          if (c1 < a.n) g1 = far(c1);  // c1 > i
         }
       };
-      if (part == 1 && l > 1) {
+      if (part == 1 && wait) {
         if (!diag_wait(a, a.dep_idx, a.dep_ptr[b], a.dep_ptr[b + 1], a.base + (unsigned)(l - 1), &s_abort)) return;
-        fetch(warp);
+        fetch(j0);
         for (int i = w0 + (int)threadIdx.x; i < r0; i += nt) in[i] = __ldcg(prev + i);
         for (int i = r1 + (int)threadIdx.x; i < w1; i += nt) in[i] = __ldcg(prev + i);
         __syncthreads();
       } else {
-        fetch(warp);
+        fetch(j0);
       }
-      for (int j = warp; j < cnt; j += nw) {
+      for (int j = j0; j < end; j += nw) {
         const int k = at(j), i = r0 + 32 * k + lane;
         const E x0 = g0, x1 = g1;
         fetch(j + nw);
-        if (i >= r1) continue;
+        if (i >= a.n) continue;
         const int pat = s_pat[k];
         Sum<F> s;
         int len = W;
@@ -251,7 +272,7 @@ __global__ void __launch_bounds__(kDiagThreads, 1) diag_kernel(const __grid_cons
           const int m = pat == 0 ? (1 << W) - 1 : __ldg(a.mask + 32 * pat + lane);
           const unsigned char *own = reinterpret_cast<const unsigned char *>(in + i);
           auto entry = [&](int u) -> E {
-            return GL > 0 && u == 0 ? x0 : GL > 0 && u == W - 1 ? x1 : *reinterpret_cast<const E *>(own + a.db[u]);
+            return kPair && u == 0 ? x0 : kPair && u == W - 1 ? x1 : *reinterpret_cast<const E *>(own + a.db[u]);
           };
           auto row = [&](auto value) {  // value(u): from shared memory, or from global memory
             if (pat == 0) {
@@ -273,7 +294,7 @@ __global__ void __launch_bounds__(kDiagThreads, 1) diag_kernel(const __grid_cons
           if (!FM::kVal || k < nres) {
             row([&](int u) { return v[32 * u]; });
           } else {
-            const V *vg = vals + (size_t)k * W * 32 + lane;
+            const V *vg = vals + (ptrdiff_t)k * W * 32 + lane;
             V w[W];
 #pragma unroll
             for (int u = 0; u < W; u++) w[u] = __ldg(vg + 32 * u);
@@ -294,45 +315,55 @@ __global__ void __launch_bounds__(kDiagThreads, 1) diag_kernel(const __grid_cons
           if (!FM::kVal)
             r = df_scale(pat == 0 ? coef2 : len < 256 ? __ldg(a.lut2 + len) : static_cast<const float2 *>(a.coef)[i], r);
           out[i] = r;
-          // others read the rows near the ends, with far diagonals any
-          if (GL > 0 || i - r0 < a.halo || r1 - i <= a.halo || a.ring_all) a.ring[(size_t)(l % 3) * a.n + i] = r;
+          if (kDeep && (unsigned)k >= (unsigned)ns) continue;
+          // at an exchange others read the rows near the ends, with far diagonals any
+          if ((!kDeep || left == 0) && l < a.nlevel && (kPair || i - r0 < a.halo || r1 - i <= a.halo || a.ring_all))
+            a.ring[(size_t)(l / depth % 3) * a.n + i] = r;
           __stcs((host ? a.hv : a.vv) + (size_t)l * a.n + i, df_to_double(r));
         } else if constexpr (kMix) {
           const float y = s.s * a.scale;
           out[i] = y;
+          if (kDeep && (unsigned)k >= (unsigned)ns) continue;
           __stcs(a.vf + (size_t)l * a.n + i, y);
         } else {
           out[i] = s.s;
+          if (kDeep && (unsigned)k >= (unsigned)ns) continue;
           __stcs(a.vv + (size_t)l * a.n + i, s.s);
           if (host) a.hv[(size_t)l * a.n + i] = s.s;
         }
       }
     }
-    if (l < a.nlevel) diag_publish(a, b, a.base + (unsigned)l);
+    if (kDeep && left > 0) __syncthreads();
+    else if (l < a.nlevel) diag_publish(a, b, a.base + (unsigned)l);
   }
 }
 
+template <int F, int W>
+const void *kernel_of(int mode) {
+  if (mode == kDiagAll) return (const void *)diag_kernel<F, W, kDiagAll>;
+  if (mode == kDiagDeep) return (const void *)diag_kernel<F, W, kDiagDeep>;
+  if constexpr (W < 9) return (const void *)diag_kernel<F, W, kDiagPair>;
+  return nullptr;
+}
 template <int F>
-const void *kernel_of(int w, int gl) {
-  if (w == 5) return gl ? (const void *)diag_kernel<F, 5, 1> : (const void *)diag_kernel<F, 5, 0>;
-  if (w == 7) return gl ? (const void *)diag_kernel<F, 7, 1> : (const void *)diag_kernel<F, 7, 0>;
-  return w == 9 && !gl ? (const void *)diag_kernel<F, 9, 0> : nullptr;
+const void *kernel_of(int w, int mode) {
+  return w == 5 ? kernel_of<F, 5>(mode) : w == 7 ? kernel_of<F, 7>(mode) : kernel_of<F, 9>(mode);
 }
 
 }  // namespace
 
 namespace mpkg {
 
-const void *diag_kernel_ptr(int form, int w, int gl) {
+const void *diag_kernel_ptr(int form, int w, int mode) {
   switch (form) {
-    case kDiagFma: return kernel_of<kDiagFma>(w, gl);
-    case kDiagFmaVal: return kernel_of<kDiagFmaVal>(w, gl);
-    case kDiagSep: return kernel_of<kDiagSep>(w, gl);
-    case kDiagSepVal: return kernel_of<kDiagSepVal>(w, gl);
-    case kDiagDf: return kernel_of<kDiagDf>(w, gl);
-    case kDiagDfVal: return kernel_of<kDiagDfVal>(w, gl);
-    case kDiagF32: return kernel_of<kDiagF32>(w, gl);
-    case kDiagBf16: return kernel_of<kDiagBf16>(w, gl);
+    case kDiagFma: return kernel_of<kDiagFma>(w, mode);
+    case kDiagFmaVal: return kernel_of<kDiagFmaVal>(w, mode);
+    case kDiagSep: return kernel_of<kDiagSep>(w, mode);
+    case kDiagSepVal: return kernel_of<kDiagSepVal>(w, mode);
+    case kDiagDf: return kernel_of<kDiagDf>(w, mode);
+    case kDiagDfVal: return kernel_of<kDiagDfVal>(w, mode);
+    case kDiagF32: return kernel_of<kDiagF32>(w, mode);
+    case kDiagBf16: return kernel_of<kDiagBf16>(w, mode);
   }
   return nullptr;
 }
@@ -347,17 +378,20 @@ int diag_value_bytes(int form) {
   return 0;
 }
 
-int diag_layout(int n, const int *ptr, const int *col, int form, int nsm, int smem, DiagLayout *out) {
+int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int nsm, int smem, DiagLayout *out) {
   DiagLayout &l = *out;
   l.fits = false;
   const int nslice = (n + 31) / 32;
   const bool ring = form == kDiagDf || form == kDiagDfVal;
   const long eb = diag_elem_bytes(form), vb = diag_value_bytes(form);
-  // the diagonals that more than half of 64 rows all over the matrix have
+  // the diagonals that more than half of 256 rows all over the matrix have
   std::map<int, int> seen;
-  const int probes = std::min(n, 64);
+  const int probes = std::min(n, 256);
+  unsigned long long mix = 1;
   for (int t = 0; t < probes; t++) {
-    const int i = (int)((0x9E3779B9ull * (unsigned long long)(t + 1)) % (unsigned long long)n);  // spread over all residues
+    // rows at random: a constant distance can keep to a mesh's planes
+    mix = mix * 6364136223846793005ull + 1442695040888963407ull;
+    const int i = n <= 256 ? t : (int)((mix >> 33) % (unsigned long long)n);
     if (ptr[i + 1] - ptr[i] > 2 * kDiagMax) return kOk;
     for (int q = ptr[i]; q < ptr[i + 1]; q++) seen[col[q] - i]++;
   }
@@ -377,26 +411,6 @@ int diag_layout(int n, const int *ptr, const int *col, int form, int nsm, int sm
   l.lo.assign(grid + 1, 0);
   for (int b = 1; b <= grid; b++) l.lo[b] = (int)std::min<long>(n, 32L * ((long)nslice * b / grid));
   const int own = 32 * ((nslice + grid - 1) / grid);
-  // the halo holds all the diagonals or all but the outermost pair: the first
-  // fetches 2 halo rows per CTA and level, the second two per own row, so a
-  // halo beyond the own rows is taken only where the second does not do
-  const bool pair = W < 9 && l.d[0] < 0 && l.d[W - 1] > 0;
-  l.win_bytes = (int)((own * eb + 15) / 16 * 16);
-  int gl = -1;
-  for (const int t : {0, 1, 2}) {
-    const int g = t & 1;
-    if (g && !pair) continue;
-    const long halo = std::max({0, -l.d[g], l.d[W - 1 - g]});
-    if (t == 0 && pair && halo > own) continue;
-    const long hb = (halo * eb + 15) / 16 * 16;
-    if (2L * l.win_bytes + 3 * hb + (2L * own / 32 + 16) > smem) continue;
-    gl = g;
-    l.halo = (int)halo;
-    l.halo_bytes = (int)hb;
-    break;
-  }
-  if (gl < 0) return kOk;
-  l.gl = gl;
   // patterns
   l.pat.assign(nslice, 0);
   std::map<std::vector<unsigned short>, int> known;
@@ -436,6 +450,46 @@ int diag_layout(int n, const int *ptr, const int *col, int form, int nsm, int sm
     known[m] = l.pat[sl];
     l.mask.insert(l.mask.end(), m.begin(), m.end());
   }
+  // Levels per exchange and the halo.  With one level, not 9 diagonals, the
+  // halo holds all of them or all but the outermost pair: the first fetches 2
+  // halo rows per CTA and level, the second two per own row, so a halo beyond
+  // the own rows is taken only where the second does not do.  With more levels
+  // it holds all.  A call's time in cycles, as measured: a hand-over 4500 and
+  // the halo's rows, a barrier 200, a slice its share of the FP64 or issue
+  // slots, a level at least the latency of one slice; once, the values of the
+  // neighbours' slices.
+  const bool pair = W < 9 && l.d[0] < 0 && l.d[W - 1] > 0;
+  const bool fp64 = eb == 8 && !ring;
+  const double per_slice = (fp64 ? 20.0 : ring ? 9.0 : 4.5) * W, least = fp64 ? 120.0 * W : ring ? 80.0 * W : 500.0;
+  const long reach = std::max({0, -l.d[0], l.d[W - 1]}), ns_max = own / 32;
+  l.win_bytes = (int)((own * eb + 15) / 16 * 16);
+  l.grow = (int)((reach + 31) / 32);
+  double best = -1;
+  auto consider = [&](int depth, int g) {  // false: does not fit
+    const long halo = 32L * (depth - 1) * l.grow + (g ? std::max({0, -l.d[1], l.d[W - 2]}) : reach);
+    const long hb = (halo * eb + 15) / 16 * 16, most = ns_max + 2L * (depth - 1) * l.grow;
+    if (2L * l.win_bytes + (depth > 1 ? 4 : 3) * hb + (2 * most + 16) > smem) return false;
+    double cost = 0.4 * halo * ((nlevel + depth - 1) / depth) + 2.0 * (depth - 1) * l.grow * W * 32 * vb / 24;
+    for (int lev = 0; lev < nlevel; lev++) {
+      const int left = std::min(depth, nlevel - lev / depth * depth) - 1 - lev % depth;
+      cost += (lev == 0 ? 0 : lev % depth == 0 ? 4500 : 200) +
+              std::max(least, per_slice * std::min<long>(nslice, ns_max + 2L * left * l.grow));
+    }
+    if (best >= 0 && cost > 0.95 * best) return true;
+    best = cost;
+    l.depth = depth;
+    l.mode = g ? kDiagPair : depth > 1 ? kDiagDeep : kDiagAll;
+    l.halo = (int)std::min<long>(halo, n);
+    l.halo_bytes = (int)hb;
+    l.second = (int)(l.win_bytes + (depth > 1 ? 2 : 1) * hb);
+    l.win_at = (int)(smem - l.second - l.win_bytes - hb);
+    return true;
+  };
+  const bool near = !pair || reach <= own;
+  if (!(near && consider(1, 0)) && !(pair && consider(1, 1)) && !consider(1, 0)) return kOk;
+  if (!irregular)
+    for (int depth = 2; depth <= std::min(nlevel, kDiagMaxDepth) && consider(depth, 0); depth++) {
+    }
   // per CTA: slice ranges, resident values, dependencies
   l.own.assign(grid, make_int2(0, 0));
   l.nres.assign(grid, 0);
@@ -449,9 +503,16 @@ int diag_layout(int n, const int *ptr, const int *col, int form, int nsm, int sm
     for (int k = ka; k < kb; k++)
       if (l.pat[r0 / 32 + k] == kDiagIrregular) kb = k;
     l.own[b] = make_int2(ka, kb);
+    const int s0 = r0 / 32, more = (l.depth - 1) * l.grow;
+    const long all = std::min(s0, more) + ns + std::min(nslice - s0 - ns, more);
+    l.slices = std::max(l.slices, (int)all);
+    for (int lev = 0; lev < nlevel; lev++) {
+      const int left = std::min(l.depth, nlevel - lev / l.depth * l.depth) - 1 - lev % l.depth, g = left * l.grow;
+      l.rows += std::min<long>(n, 32L * (s0 + ns + std::min(nslice - s0 - ns, g))) - 32L * (s0 - std::min(s0, g));
+    }
     if (vb) {
-      const long room = smem - 2L * l.win_bytes - 3L * l.halo_bytes - (2L * ns + 15) / 16 * 16;
-      l.nres[b] = (int)std::min<long>(ns, room / (vb * W * 32));
+      const long room = l.win_at - l.halo_bytes - (2 * all + 15) / 16 * 16;
+      l.nres[b] = (int)std::min<long>(all, room / (vb * W * 32));
     }
     std::vector<int> &wt = waits[b];
     int last = -1;
@@ -462,6 +523,12 @@ int diag_layout(int n, const int *ptr, const int *col, int form, int nsm, int sm
       last = owner(c);
       wt.push_back(last);
     }
+    if (l.depth > 1)  // the rows of the halo
+      for (const int end : {0, 1}) {
+        const int c0 = end ? r1 : std::max(0, r0 - l.halo), c1 = end ? std::min(n, r1 + l.halo) : r0;
+        if (c0 < c1)
+          for (int o = owner(c0); o <= owner(c1 - 1); o++) wt.push_back(o);
+      }
     std::sort(wt.begin(), wt.end());
     wt.erase(std::unique(wt.begin(), wt.end()), wt.end());
   }

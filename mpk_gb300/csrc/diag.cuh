@@ -18,7 +18,13 @@ enum DiagForm {
   kDiagF32, kDiagBf16,    // mixed: FP32 or BF16 values
 };
 
+// How rows of other CTAs are read: from the halo; the outermost diagonal on
+// either side from global memory and the others from the halo; from a halo for
+// several levels.
+enum DiagMode { kDiagAll, kDiagPair, kDiagDeep };
+
 constexpr int kDiagMax = 9;  // diagonals
+constexpr int kDiagMaxDepth = 8;
 
 struct DiagArgs {
   int n, nlevel, nblk;
@@ -26,6 +32,7 @@ struct DiagArgs {
   int d[kDiagMax];        // the diagonals, ascending column offsets ...
   int db[kDiagMax];       // ... and in bytes of a window
   int halo;               // rows kept of the CTAs on either side
+  int depth, grow;        // levels per exchange; slices that a level takes more on either side for the next
   const int *row_lo, *dep_ptr, *dep_idx;
   unsigned int *flags;
   int *err;
@@ -46,7 +53,7 @@ struct DiagArgs {
   float scale;
   double *hv;                  // host mapping of vv, or null (as WaveArgs; double-float: vv is the host's)
   int smem;                    // dynamic shared memory
-  int win_bytes, halo_bytes;   // of one window, of one halo
+  int win_at, second;          // bytes: the own rows of window A, and of window B after those
 };
 
 constexpr unsigned short kDiagIrregular = 0xFFFF;
@@ -55,10 +62,12 @@ constexpr int kFlagStride = 32;  // flags lie in cache lines of their own
 // Host side of a layout.
 struct DiagLayout {
   bool fits = false;
-  int w = 0, gl = 0;           // diagonals; the outermost gl on either side are always read from global memory
+  int w = 0, mode = kDiagAll;  // diagonals; DiagMode
   int d[kDiagMax] = {};
   int halo = 0, win_bytes = 0, halo_bytes = 0, grid = 0;
-  long reach = 0, irregular = 0;
+  int depth = 1, grow = 0, win_at = 0, second = 0;
+  int slices = 0;              // the most that a CTA computes at a level
+  long reach = 0, irregular = 0, rows = 0;  // rows: computed by a call
   std::vector<int> lo, dptr, didx, nres;
   std::vector<int2> own;
   std::vector<unsigned short> pat, mask;
@@ -67,7 +76,7 @@ struct DiagLayout {
 // The layout of the diagonal wavefront for `nsm` CTAs with `smem` bytes of
 // dynamic shared memory; fits is false where the structure or the sizes do
 // not suit it.  ring: dependencies both ways.
-int diag_layout(int n, const int *ptr, const int *col, int form, int nsm, int smem, DiagLayout *out);
+int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int nsm, int smem, DiagLayout *out);
 
 // Values along the layout's diagonals, [slice][diagonal][lane], zero where a
 // row has no entry (and in irregular slices): conv(entry) in type T.
@@ -84,7 +93,7 @@ void diag_values(int n, const int *ptr, const int *col, const DiagLayout &l, F &
   }
 }
 
-const void *diag_kernel_ptr(int form, int w, int gl);
+const void *diag_kernel_ptr(int form, int w, int mode);
 constexpr int kDiagThreads = 1024;
 int diag_elem_bytes(int form);   // of a window element
 int diag_value_bytes(int form);  // of a matrix value, 0 for 1/deg

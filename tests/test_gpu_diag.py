@@ -2,9 +2,10 @@
 against the general wavefront (the same plan with a cap on its CTAs per SM)
 bit for bit in FP64 and double-float, and against the oracle's FP32 chain in
 the mixed form: meshes whose far diagonals lie inside and outside a CTA's own
-rows, rows short of a slice, rows without some or all of the diagonals, rows
-with other columns, unsorted and repeated columns, one level and many, and
-host execution on page-locked and pageable memory."""
+rows, several levels per exchange of neighbouring rows, rows short of a slice,
+rows without some or all of the diagonals, rows with other columns, unsorted
+and repeated columns, one level and many, and host execution on page-locked and
+pageable memory."""
 import numpy as np
 import pytest
 
@@ -38,6 +39,12 @@ CASES = {
     "box7_thin": (lambda: M.Csr.laplacian(11, 9, 1201), 5),
     "tiny": (lambda: M.Csr.laplacian(5, 5), 1),
     "few_slices": (lambda: M.Csr.laplacian(9, 11), 31),
+    # several levels per exchange: all of them, and a short last block
+    "deep5": (lambda: M.Csr.laplacian(60, 61), 7),
+    "deep5_one_slice": (lambda: M.Csr.laplacian(31, 170), 5),
+    "deep9": (lambda: M.Csr.diffusion(91, 33, sigma=1.0, seed=6), 8),
+    "deep9_many": (lambda: M.Csr.diffusion(150, 301, sigma=1.0, seed=6), 11),
+    "deep7": (lambda: M.Csr.laplacian(20, 21, 22), 5),
     "odd_rows": (lambda: _odd(M.Csr.laplacian(60, 61, 20), 3, 4001, 53, 2503), 4),
     "odd_rows_2d": (lambda: _odd(M.Csr.laplacian(150, 149), 4, 1999, 31, 1777), 5),
 }
