@@ -405,8 +405,11 @@ __global__ void __launch_bounds__(kThreads) basis_wave_kernel(BasisWave w, Sell 
 // columns, rms over the pairs relative to the columns' norms, three
 // distributions together, at 1 K / 30 K / 262 K / 885 K rows 4.6e-17 /
 // 5.0e-17 / 5.9e-17 / 5.5e-17 against 5.5e-17 / 5.2e-17 / 8.1e-17 / 2.8e-16.
-// Tiles with a nonzero value outside 2^-45 .. 2^60, where a product or its
-// error could leave the FP32 range, are summed with FP64 fused multiply-adds.
+// A tile's columns are scaled by powers of two to a largest value in [1, 2),
+// so that products and their errors stay in the FP32 range; tiles with
+// infinities or NaN are summed with FP64 fused multiply-adds.  (Unscaled, a
+// monomial basis, whose columns shrink, left that range: 181 us an outer
+// iteration on 64^3 diffusion, 136 so.)
 // A CTA stages a tile of rows of all columns in shared memory, thread t
 // accumulates pair t of the upper triangle; per-CTA partials (FP64) are summed
 // in a fixed order by gram_reduce_kernel.
@@ -415,7 +418,7 @@ __global__ void __launch_bounds__(kThreads) basis_wave_kernel(BasisWave w, Sell 
 // rows 45 us, 885 K rows 137 us, against 86 and 268 with FP64 fused
 // multiply-adds, whose pipe bounds those; without the compensation of the low
 // sums (10 instructions) 30 and 86 us, but 5 times further off.
-constexpr int kGramRows = 64;
+constexpr int kGramRows = 64;  // two per lane of the warp that stages a column
 constexpr int kGramStride = kGramRows + 4;  // 16-byte rows, eight columns in different banks
 thread_local bool g_gram_f64 = true;  // mpkg_sstep_gram: FP64 (default) or double-float Gram
 thread_local bool g_device_loop = true;  // mpkg_sstep_loop: device-side (default) or host-side outer loop
@@ -445,12 +448,13 @@ __device__ __forceinline__ void gram_acc4(float a, float b, float &h, float &l, 
   c = __fadd_rn(c, __fadd_rn(el, two_sum(m, e)));
 }
 
-// Exact float -> double in integer arithmetic (the conversion shares the FP64 pipe).
-__device__ __forceinline__ double ss_widen(float f) {
+// f * 2^k, exact, in integer arithmetic (the conversion shares the FP64 pipe);
+// subnormals as zero.
+__device__ __forceinline__ double ss_widen(float f, int k = 0) {
   const unsigned int u = __float_as_uint(f);
   const unsigned int e = (u >> 23) & 0xFF;
   const unsigned int sgn = u & 0x80000000u;
-  const unsigned int bias = e == 0xFF ? (1792u << 20) : (896u << 20);
+  const unsigned int bias = (unsigned)(e == 0xFF ? 1792 : 896 + k) << 20;
   const unsigned int hi = e == 0 ? sgn : (sgn | (((u >> 3) & 0x0FFFFFFFu) + bias));
   const unsigned int lo = e == 0 ? 0u : (u << 29);
   return __hiloint2double((int)hi, (int)lo);
@@ -460,6 +464,7 @@ template <bool F64>
 __global__ void __launch_bounds__(kThreads) gram_kernel(int n, int ncol, const float *__restrict__ y,
                                                         double *__restrict__ part) {
   __shared__ __align__(16) float tile[kMaxCols * kGramStride];
+  __shared__ int s_exp[kMaxCols];  // F64: the tile's columns are scaled by 2^-s_exp
   const int npair = ncol * (ncol + 1) / 2;
   int pa = 0, pb = 0;
   {
@@ -471,23 +476,46 @@ __global__ void __launch_bounds__(kThreads) gram_kernel(int n, int ncol, const f
   const float4 *ta = reinterpret_cast<const float4 *>(tile + pa * kGramStride);
   const float4 *tb = reinterpret_cast<const float4 *>(tile + pb * kGramStride);
   float h[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
+  const int lane = threadIdx.x & 31;
   double acc = 0.0;
   for (long r0 = (long)blockIdx.x * kGramRows; r0 < n; r0 += (long)gridDim.x * kGramRows) {
     __syncthreads();
     int wide = 0;
-    for (int e = threadIdx.x; e < ncol * kGramRows; e += blockDim.x) {
-      const int c = e / kGramRows, rr = e % kGramRows;
-      const float v = r0 + rr < n ? y[(size_t)c * n + r0 + rr] : 0.f;
-      tile[c * kGramStride + rr] = v;
-      const unsigned int u = __float_as_uint(v) & 0x7FFFFFFFu;
-      wide |= u != 0 && u - (82u << 23) >= (105u << 23);
+    for (int c = threadIdx.x >> 5; c < ncol; c += blockDim.x >> 5) {  // a warp per column
+      float v[2];
+      unsigned int top = 0;
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const long i = r0 + lane + 32 * q;
+        v[q] = i < n ? y[(size_t)c * n + i] : 0.f;
+        top = max(top, __float_as_uint(v[q]) & 0x7FFFFFFFu);
+      }
+      float up = 1.f;
+      if (F64) {
+        top = __reduce_max_sync(0xFFFFFFFFu, top);
+        int e = (int)(top >> 23), sub = 0;
+        if (e == 0 && top != 0) {  // subnormal
+          sub = 64;
+          v[0] *= 0x1p64f;
+          v[1] *= 0x1p64f;
+          e = (int)(__float_as_uint(__uint_as_float(top) * 0x1p64f) >> 23);
+        }
+        wide |= e == 255;
+        if (e > 0 && e < 255) up = __uint_as_float(e < 254 ? (unsigned)(254 - e) << 23 : 1u << 22);  // 2^(127 - e)
+        if (lane == 0) s_exp[c] = e > 0 && e < 255 ? e - 127 - sub : 0;
+      }
+      tile[c * kGramStride + lane] = v[0] * up;
+      tile[c * kGramStride + lane + 32] = v[1] * up;
     }
     if (F64) wide = __syncthreads_or(wide);
     else __syncthreads();
     if ((int)threadIdx.x >= npair) continue;
+    const int k = F64 ? s_exp[pa] + s_exp[pb] : 0;
     if (F64 && wide) {
+      double t = 0.0;
       for (int rr = 0; rr < kGramRows; rr++)
-        acc = fma((double)tile[pa * kGramStride + rr], (double)tile[pb * kGramStride + rr], acc);
+        t = fma((double)tile[pa * kGramStride + rr], (double)tile[pb * kGramStride + rr], t);
+      acc += scalbn(t, k);
       continue;
     }
     if (F64) {
@@ -500,8 +528,8 @@ __global__ void __launch_bounds__(kThreads) gram_kernel(int n, int ncol, const f
         gram_acc4(va.z, vb.z, h0, l0, m0, c0);
         gram_acc4(va.w, vb.w, h0, l0, m0, c0);
       }
-      acc += ss_widen(h0);
-      acc += (ss_widen(l0) + ss_widen(m0)) + ss_widen(c0);
+      acc += ss_widen(h0, k);
+      acc += (ss_widen(l0, k) + ss_widen(m0, k)) + ss_widen(c0, k);
     } else {
 #pragma unroll 4
       for (int q = 0; q < kGramRows / 4; q++) {
