@@ -226,6 +226,8 @@ __global__ void __launch_bounds__(kDiagThreads, 1) diag_kernel(const __grid_cons
   if constexpr (kDf && !FM::kVal) coef2 = __ldg(a.lut2 + W);
   __syncthreads();
   if (FM::kVal && !tr_wait(&s_bar, 0, a.err)) return;
+  // the test hook's wait, also where no level waits
+  if (kDeep && a.stall && !diag_wait(a, a.dep_idx, a.dep_ptr[b], a.dep_ptr[b + 1], a.base + 1, &s_abort)) return;
   for (int l = 1, left = -1; l <= a.nlevel; l++, left--) {
     // `left` levels follow before the next exchange; each needs a.grow slices
     // more of this one on either side
