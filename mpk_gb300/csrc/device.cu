@@ -2468,10 +2468,16 @@ bool host_parallel(int count, F &&fn) {
 
 // Groups of consecutive matrices within `budget` bytes (matrix + two
 // levels of vectors); per group, CTA row ranges of equal nonzeros and the
-// CTAs owning each range's columns.  A group of fewer rows than the grid
-// has row slots (`threads` / lpr per CTA) takes fewer CTAs, so that each has
-// one pass of its threads: a level costs a hand-over between CTAs whatever
-// its size, and matrices of up to two passes stay whole, with none.
+// CTAs owning each range's columns.  A small group takes fewer CTAs, and its
+// ranges end with its matrices, since a level costs a hand-over between CTAs
+// (some 5 K cycles) whatever its size, and a matrix that stays whole has none.
+// CSR kernel: groups of fewer rows than the grid has row slots (`threads` /
+// lpr per CTA, a pass of the CTA's threads); a pass per CTA, matrices of up to
+// two passes whole.  Windows: by work, of which 10 units a row slot take as
+// long as a hand-over; a CTA has that much or more, matrices of up to one and
+// a half hand-overs stay whole (41 matrices of 335-2744 rows, 4 right-hand
+// sides, 4 levels, one CTA per SM: 23 us, by rows as above 48, for parts and
+// whole matrices of twice that 28 and more; 20 of 500-2500, 16 sides: 23 / 28).
 int batch_ranges(const BatchHost &h, int nrhs, long budget, bool windows, int grid, int threads, int lpr,
                  BatchLayout *out) {
   const int nmat = (int)h.mat_row0.size() - 1;
@@ -2512,10 +2518,23 @@ int batch_ranges(const BatchHost &h, int nrhs, long budget, bool windows, int gr
     const long a = h.mat_row0[g0[g]], z = h.mat_row0[g0[g + 1]];
     const long pass = std::max(1, threads / lpr);  // rows of one pass
     std::vector<long> cut(1, a);
-    if (z - a <= pass * grid) {
+    const long share = (work(z) - work(a)) / grid + 1;
+    long part = std::max(10 * pass, share);
+    auto parts_of = [&](int m) {
+      const long r0 = h.mat_row0[m], r1 = h.mat_row0[m + 1], w = work(r1) - work(r0);
+      if (windows) return w <= std::max(15 * pass, part) ? 1L : (w + part - 1) / part;
+      return r1 - r0 <= 2 * pass ? 1L : (r1 - r0 + pass - 1) / pass;
+    };
+    auto parts_all = [&] {
+      long n = 0;
+      for (int m = g0[g]; m < g0[g + 1]; m++) n += parts_of(m);
+      return n;
+    };
+    const bool few = windows ? g0[g + 1] - g0[g] <= grid && share <= 40 * pass : z - a <= pass * grid;
+    if (few) {
+      while (windows && parts_all() > grid) part += part / 8 + 1;
       for (int m = g0[g]; m < g0[g + 1]; m++) {
-        const long r0 = h.mat_row0[m], r1 = h.mat_row0[m + 1];
-        const long parts = r1 - r0 <= 2 * pass ? 1 : (r1 - r0 + pass - 1) / pass;
+        const long r0 = h.mat_row0[m], r1 = h.mat_row0[m + 1], parts = parts_of(m);
         const long q0 = work(r0), nz = work(r1) - q0;
         for (long t = 1; t < parts; t++) cut.push_back(std::max(std::min(row_at(q0 + nz * t / parts, r0, r1), r1), cut.back()));
         cut.push_back(r1);

@@ -2,7 +2,8 @@
 the oracle's FP32 chain: rows short of a slice and of a pair of entries,
 empty rows, rows of every length in one matrix, columns beyond the window,
 the matrix resident in shared memory and streamed past it, one row per
-matrix; and plans of different windows alive together."""
+matrix, matrices whole and in parts, more of them than thread blocks; and plans
+of different windows alive together."""
 import numpy as np
 import pytest
 
@@ -45,6 +46,8 @@ EDGES = {
     "empty_rows": lambda: [_random(300, [0, 5, 0, 1, 8], 1, 40), _random(65, [0, 0, 3], 2)],
     "all_lengths": lambda: [_random(1500, list(range(70)), 3, 64)],
     "anywhere": lambda: [_random(9000, [4, 9, 1], 4), M.Csr.laplacian(30, 30, 30)],
+    "whole_and_parts": lambda: [_random(n, [9, 13, 30], n, 64) for n in (300, 760, 64, 1500, 4000, 2900)],
+    "more_than_ctas": lambda: [_random(1 + n % 9, [2, 3], n) for n in range(160)],
     "long_rows": lambda: [_random(700, [2, 2, 2, 600], 5), _random(257, [257], 6)],
 }
 
