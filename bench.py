@@ -510,7 +510,7 @@ def bench_sstep(M):
     # outer iteration (the default builds it with one launch per step)
     _, out["learned_shifts_mpk_basis"] = M.sstep_cg(a, b, 8, shifts=sh, basis=M.SSTEP_BASIS_MPK)
     out["basis"] = "one FP32 SpMV launch per Newton step, both blocks per launch (mpk_basis: one wavefront launch)"
-    out["gram"] = "FP64 FMAs over the exact FP64 products of the FP32 basis (df64: double-float sums)"
+    out["gram"] = "FP64, from FP32 sums of the exact products with their errors kept (df64: double-float sums)"
     # the same solve with the outer loop driven from the host (one graph
     # launch and synchronisation per outer iteration)
     _, out["learned_shifts_host_loop"] = M.sstep_cg(a, b, 8, shifts=sh, loop=M.SSTEP_HOST_LOOP)
@@ -719,13 +719,14 @@ def main():
     peak, peak_kind = peaks()
     B = algorithmic_bytes(n, nnz, k, valued=False)
     achieved = B / (ms * 1e-3) / 1e9
-    kname = {"pipe": "flow_kernel", "wave": "wave_kernel", "tiles": "tiles_kernel", "tasks": "tasks_kernel",
+    # the wavefront of a mesh in its natural order is the diagonal one
+    kname = {"pipe": "flow_kernel", "wave": "diag_kernel", "tiles": "tiles_kernel", "tasks": "tasks_kernel",
              "spmv": "spmv_level_kernel"}[args.exec]
     if args.arith == "df64":
-        kname = {"pipe": "flow_df_kernel", "wave": "wave_df_kernel", "tiles": "tiles_df_kernel"}.get(args.exec, kname)
+        kname = {"pipe": "flow_df_kernel", "tiles": "tiles_df_kernel"}.get(args.exec, kname)
     if args.arith == "fixed":
         kname = "wave_fix_kernel"
-    traffic = profile_traffic(kname)
+    traffic = profile_traffic(f"{kname} {args.arith}" if kname == "diag_kernel" else kname)
     rows = info["rows_computed"]
     fmas = nnz * k * (rows / (n * k))
     rate = fp64_rate()
