@@ -8,6 +8,8 @@
 //   pipe   - zero-redundancy level pipeline: chunks of rows keep their
 //            matrix rows in shared memory and advance level by level once
 //            the neighbouring chunks have finished the previous level;
+//   wave   - persistent wavefront: row ranges at every level, waits for the
+//            neighbours only (diag.cu for rows on a few diagonals);
 //   spmv   - k separate SpMV launches (baseline, spmv_exec_*).
 // All executors evaluate each row sum over the stored columns in CSR order,
 // so for a given arithmetic mode every executor produces the same bits.
