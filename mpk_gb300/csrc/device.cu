@@ -2147,6 +2147,14 @@ int dev_alloc(mpkg_plan *p, T **dst, size_t count) {
   return kOk;
 }
 
+// Clears device memory before it returns: cudaMemset does not wait for the
+// device, and the streams that plans and callers launch on do not wait for its.
+int dev_clear(void *q, size_t bytes) {
+  CUDA_TRY(cudaMemset(q, 0, bytes));
+  CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+  return kOk;
+}
+
 int check_csr(int n, const int *ptr, const int *col) {
   if (n <= 0 || !ptr || !col) return fail(kEInval, "empty matrix or null arrays");
   if (ptr[0] != 0) return fail(kEInval, "ptr[0] must be 0");
@@ -2197,8 +2205,7 @@ int plan_common(mpkg_plan *p, int n, const int *ptr, const int *col, const doubl
     CUDA_TRY(cudaStreamSynchronize(p->stream));
   }
   if ((rc = dev_alloc(p, &p->d_err, 1))) return rc;
-  CUDA_TRY(cudaMemset(p->d_err, 0, sizeof(int)));
-  return kOk;
+  return dev_clear(p->d_err, sizeof(int));
 }
 
 int build_task_device(mpkg_plan *p, int npart, int nphase, const long *off, const long *idx) {
@@ -3256,7 +3263,7 @@ int mpkg_plan_pipe(int n, const int *ptr, const int *col, const double *val, int
       a.coef2 = p->d_coef2;
     }
     if (!rc) {
-      cudaMemset(counts, 0, sizeof(unsigned int) * ncount);
+      rc = dev_clear(counts, sizeof(unsigned int) * ncount);
       a.gdep_lo = dlo; a.gdep_hi = dhi; a.ticket = ticket; a.counts = counts;
       a.ptr = p->d_ptr; a.col = p->d_col; a.coef = p->d_coef; a.err = p->d_err;
       a.bulk_ok = true;  // cudaMalloc'd arrays are 256-byte aligned
@@ -3431,7 +3438,7 @@ int mpkg_plan_bufs(const char *dir, int npart, int arith, mpkg_plan **out) {
   if (!rc) rc = dev_copy(p, &p->b_gcol, gcol.data(), gcol.size());
   if (!rc) rc = dev_copy(p, &p->b_gval, gval.data(), gval.size());
   if (!rc) rc = dev_alloc(p, &p->d_err, 1);
-  if (!rc && cudaMemset(p->d_err, 0, sizeof(int)) != cudaSuccess) rc = fail(kECuda, "memset failed");
+  if (!rc) rc = dev_clear(p->d_err, sizeof(int));
   p->b_nin = (long)in_dst.size();
   p->b_nout = (long)out_src.size();
   p->b_cm_off = cm_off;
@@ -3799,8 +3806,7 @@ int plan_wave_impl(int n, const int *ptr, const int *col, const double *val, int
       for (int d = 2; d < 256; d++) mul[d] = ~0ull / (unsigned long long)d + 1;  // ceil(2^64 / d)
       rc = dev_copy(p, (unsigned long long **)&w.fix_mul, mul.data(), mul.size());
       if (!rc) rc = dev_alloc(p, &w.fix_word, 1);
-      if (!rc && cudaMemset(w.fix_word, 0, sizeof(unsigned long long)) != cudaSuccess)
-        rc = fail(kECuda, "memset failed");
+      if (!rc) rc = dev_clear(w.fix_word, sizeof(unsigned long long));
     }
     w.row_lo = d_lo; w.dep_ptr = d_dlo; w.dep_idx = d_dhi;
     p->pipe_reach = (int)reach;
@@ -3859,7 +3865,7 @@ int batch_configure(mpkg_plan *p, const BatchHost &h, const BatchCand &c, const 
   if (!rc) rc = dev_copy(p, &d_dlo, lay.dptr.data(), lay.dptr.size());
   if (!rc) rc = dev_copy(p, &d_dhi, lay.didx.data(), lay.didx.size());
   if (!rc) rc = dev_alloc(p, &d_flags, (size_t)c.grid);
-  if (!rc && cudaMemset(d_flags, 0, sizeof(unsigned int) * (size_t)c.grid) != cudaSuccess) rc = fail(kECuda, "memset failed");
+  if (!rc) rc = dev_clear(d_flags, sizeof(unsigned int) * (size_t)c.grid);
   if (!rc && c.staged) {
     BatchUnit *unit = nullptr;
     int4 *iv = nullptr;
@@ -3943,7 +3949,7 @@ int mpkg_plan_batch(int nmat, const int *n, const int *const *ptr, const int *co
   BatchArgs &a = p->batch;
   a.N = h.N; a.nrhs = nrhs; a.nlevel = nlevel;
   if (!rc) rc = dev_alloc(p, &p->d_err, 1);
-  if (!rc && cudaMemset(p->d_err, 0, sizeof(int)) != cudaSuccess) rc = fail(kECuda, "memset failed");
+  if (!rc) rc = dev_clear(p->d_err, sizeof(int));
   a.err = p->d_err;
   int nsm = 0, sm_per_sm = 0, sm_optin = 0;
   if (!rc &&
@@ -4156,7 +4162,7 @@ int mpkg_plan_pdmpk(int npart, const char *const *buf_paths, const char *const *
   if (!rc) rc = dev_copy(p, &p->b_gcol, m.gcol.data(), m.gcol.size());
   if (!rc) rc = dev_copy(p, &p->b_gval, m.gval.data(), m.gval.size());
   if (!rc) rc = dev_alloc(p, &p->d_err, 1);
-  if (!rc && cudaMemset(p->d_err, 0, sizeof(int)) != cudaSuccess) rc = fail(kECuda, "memset failed");
+  if (!rc) rc = dev_clear(p->d_err, sizeof(int));
   p->b_nin = (long)m.in_dst.size();
   p->b_nout = (long)m.out_src.size();
   p->b_cm_off = m.cm_off;
@@ -4352,8 +4358,8 @@ int mpkg_plan_mixed(int n, const int *ptr, const int *col, const double *val, in
   if (!rc) rc = dev_alloc(p, &counts, (size_t)(nlevel + 1) * pp.nchunk);
   if (!rc) rc = dev_alloc(p, &p->d_err, 1);
   if (!rc) {
-    cudaMemset(counts, 0, sizeof(unsigned) * (size_t)(nlevel + 1) * pp.nchunk);
-    cudaMemset(p->d_err, 0, sizeof(int));
+    rc = dev_clear(counts, sizeof(unsigned) * (size_t)(nlevel + 1) * pp.nchunk);
+    if (!rc) rc = dev_clear(p->d_err, sizeof(int));
     m.gdep_lo = dlo; m.gdep_hi = dhi; m.ptr = p->d_ptr; m.col = p->d_col; m.ticket = ticket; m.counts = counts;
     m.err = p->d_err;
     m.bulk_ok = true;
@@ -4693,7 +4699,7 @@ int mpkg_plan_mixed_tiles(int n, const int *ptr, const int *col, const double *v
   if (!rc) rc = dev_alloc(p, &ticket, 1);
   if (!rc) rc = dev_alloc(p, &p->d_err, 1);
   if (!rc) {
-    cudaMemset(p->d_err, 0, sizeof(int));
+    rc = dev_clear(p->d_err, sizeof(int));
     a.order = order; a.slot_off = slot_off; a.shell = shell; a.slot_vert = slot_vert; a.slot_coef = slot_coef;
     a.slice_off = slice_off; a.ell_off = ell_off; a.ell_col = ell_col; a.ell_width = ell_width;
     a.ticket = ticket; a.err = p->d_err;
@@ -4731,7 +4737,7 @@ int mpkg_plan_mixed_tiles_tuned(int n, const int *ptr, const int *col, const dou
   float *scratch = nullptr;
   if (cudaMalloc(&scratch, sizeof(float) * (size_t)n * (nlevel + 1)) != cudaSuccess)
     return fail(kENoMem, "autotune scratch");
-  cudaMemset(scratch, 0, sizeof(float) * (size_t)n * (nlevel + 1));  // timing only: the values do not matter
+  dev_clear(scratch, sizeof(float) * (size_t)n * (nlevel + 1));  // timing only: the values do not matter
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -4927,16 +4933,17 @@ int mpkg_sync(mpkg_plan *p, void *stream) {
   int err = 0;
   CUDA_TRY(cudaMemcpy(&err, p->d_err, sizeof(int), cudaMemcpyDeviceToHost));
   if (err) {
-    cudaMemset(p->d_err, 0, sizeof(int));
+    CUDA_TRY(cudaMemsetAsync(p->d_err, 0, sizeof(int), st));
     if ((p->exec == MPKG_EXEC_PIPE || p->exec == MPKG_EXEC_MIXED) && p->pipe.counts) {  // counters are
       // inconsistent after an abort
-      cudaMemset(p->pipe.counts, 0, sizeof(unsigned int) * (size_t)(p->nlevel + 1) * p->pipe.ngroups);
+      CUDA_TRY(cudaMemsetAsync(p->pipe.counts, 0, sizeof(unsigned int) * (size_t)(p->nlevel + 1) * p->pipe.ngroups, st));
       p->epoch = 0;
     }
     if (p->exec == MPKG_EXEC_WAVE) p->wave.base = 0;  // flags restart from zero on the next call
     if (p->inner) p->inner->wave.base = 0;
     if (p->exec == MPKG_EXEC_BATCH && p->batch.flags)  // left behind by an abort
-      cudaMemset(p->batch.flags, 0, sizeof(unsigned int) * (size_t)p->batch.nblk);
+      CUDA_TRY(cudaMemsetAsync(p->batch.flags, 0, sizeof(unsigned int) * (size_t)p->batch.nblk, st));
+    CUDA_TRY(cudaStreamSynchronize(st));  // the next call may be on another stream
     if (err == kErrTimeout) return fail(kETimeout, "a device-side wait exceeded its spin limit");
     return fail(kERange, "device-side bounds check failed");
   }

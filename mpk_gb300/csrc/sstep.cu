@@ -950,6 +950,7 @@ struct BasisLayout {
     SS_TRY(cudaMemcpy(dep_ptr.p, dp.data(), sizeof(int) * (nblk + 1), cudaMemcpyHostToDevice));
     if (!di.empty()) SS_TRY(cudaMemcpy(dep_idx.p, di.data(), sizeof(int) * di.size(), cudaMemcpyHostToDevice));
     SS_TRY(cudaMemset(err.p, 0, sizeof(int)));
+    SS_TRY(cudaStreamSynchronize(cudaStreamLegacy));  // the solve's stream does not wait for that one
     w.n = n; w.s = s; w.nblk = nblk; w.stall = g_basis_stall;
     w.row_lo = row_lo.p; w.dep_ptr = dep_ptr.p; w.dep_idx = dep_idx.p; w.flags = flags.p; w.err = err.p;
     for (int j = 0; j < s; j++) {
