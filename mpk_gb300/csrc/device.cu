@@ -2134,6 +2134,7 @@ int dev_copy(mpkg_plan *p, T **dst, const T *src, size_t count) {
   p->owned.push_back(*dst);
   p->device_bytes += (long)(sizeof(T) * count);
   CUDA_TRY(cudaMemcpy(*dst, src, sizeof(T) * count, cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));  // the copy from pageable memory may still be on its way
   return kOk;
 }
 

@@ -1282,6 +1282,7 @@ int mpkg_sstep_cg(int n, const int *ptr, const int *col, const double *val, cons
   double rr;
   if ((rc = sum_parts(part.p, nb, &rr))) return rc;
   SS_TRY(cudaMemcpy(dp.p, dr.p, sizeof(double) * n, cudaMemcpyDeviceToDevice));
+  SS_TRY(cudaStreamSynchronize(cudaStreamLegacy));  // the solve's stream does not wait for that one
   double pp = rr;
   GraphRun gr;
   SS_TRY(cudaStreamCreateWithFlags(&gr.st, cudaStreamNonBlocking));

@@ -1,8 +1,9 @@
-"""Device memory that a call or a plan clears is cleared before any kernel can
-read it.  cudaMemset works on the legacy default stream and returns before the
-device has done it, while plans and callers launch on streams that do not wait
-for that one: between a cudaMemset and the next launch, or the return to the
-caller, something must wait for it."""
+"""Device memory that a call or a plan clears or fills is ready before any
+kernel can read it.  cudaMemset, and cudaMemcpy from pageable or device memory,
+work on the legacy default stream and may return before the device has done
+them, while plans and callers launch on streams that do not wait for that one:
+between them and the next launch, or the return to the caller, something must
+wait."""
 import pytest
 
 import fake_cudart
@@ -30,7 +31,7 @@ def _check(log):
     """Follows the legacy stream: what is pending on it at each launch on another stream and at each mark."""
     pending = None
     for w in log:
-        if w[0] == "memset" and w[2] == "legacy":
+        if w[-1] == "legacy" and (w[0] == "memset" or w[0] == "memcpy" and w[1] in ("1", "3")):  # up, or on the device
             pending = w
         elif w[0] == "memcpy" and w[3] == "legacy" or w[0] == "sync" and w[1] in ("legacy", "device"):
             pending = None
@@ -60,4 +61,16 @@ mark("returned")
 """)
     at = log.index(["mark", "sync"])
     assert any(w[0] == "memset" for w in log[at:])
+    _check(log)
+
+
+@pytest.mark.parametrize("basis", ["M.SSTEP_BASIS_MPK", "M.SSTEP_BASIS_STEPS"])
+def test_solve_starts_from_what_it_uploaded(basis, tmp_path):
+    """The solver's own stream, up to the point where the fake runtime has no graphs."""
+    log = fake_cudart.run(str(tmp_path), SETUP + f"""
+try: M.sstep_cg(V, np.ones(V.n), 4, scale=1.0, basis={basis})
+except M.MpkError: pass
+mark("returned")
+""")
+    assert any(w[0] == "launch" for w in log)
     _check(log)
