@@ -200,14 +200,20 @@ __global__ void __launch_bounds__(kDiagThreads, 1) diag_kernel(const __grid_cons
         const int c0 = (int)(((long)(grp - 1) * a.nblk + kXGroups - 1) / kXGroups);
         const int c1 = (int)(((long)grp * a.nblk + kXGroups - 1) / kXGroups);
         __syncthreads();
-        if (!diag_wait(a, nullptr, c0, c1, a.base, &s_abort)) return;
+        if (!diag_wait(a, nullptr, c0, c1, a.base, &s_abort)) {
+          if (FM::kVal) tr_wait(&s_bar, 0, a.err);  // the values are on their way
+          return;
+        }
       }
       for (int i = r0 + (int)threadIdx.x; i < r1; i += nt) {
         if constexpr (kDf) a.ring[i] = df_split(a.hv[i]);
         else a.vv[i] = a.hv[i];
       }
       diag_publish(a, b, a.base);
-      if (!diag_wait(a, a.dep_idx, a.dep_ptr[b], a.dep_ptr[b + 1], a.base, &s_abort)) return;
+      if (!diag_wait(a, a.dep_idx, a.dep_ptr[b], a.dep_ptr[b + 1], a.base, &s_abort)) {
+        if (FM::kVal) tr_wait(&s_bar, 0, a.err);
+        return;
+      }
     }
   }
   auto first = [&](int i) -> E {  // row i of level 0
