@@ -1725,7 +1725,7 @@ __global__ void __launch_bounds__(256) batch_kernel(BatchArgs a) {
       }
     }
   }
-  if (threadIdx.x == 0) a.flags[b] = base + (unsigned)a.ngroup * (unsigned)(a.nlevel + 1);
+  if (threadIdx.x == 0) st_release(a.flags + b, base + (unsigned)a.ngroup * (unsigned)(a.nlevel + 1));
 }
 
 // The batched rows with the previous level in shared memory and the matrix
@@ -1932,7 +1932,7 @@ __global__ void __launch_bounds__(1024) batch_pack_kernel(BatchArgs a) {
       }
     }
   }
-  if (threadIdx.x == 0) a.flags[b] = base + (unsigned)a.ngroup * (unsigned)(a.nlevel + 1);
+  if (threadIdx.x == 0) st_release(a.flags + b, base + (unsigned)a.ngroup * (unsigned)(a.nlevel + 1));
 }
 
 // One pdmpk batch of every rank (Buffers::DoComp, pdmpk/buffers.cc:76-97):

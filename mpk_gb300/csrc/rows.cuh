@@ -82,6 +82,10 @@ __device__ __forceinline__ unsigned int ld_acquire(const unsigned int *p) {
   return v;
 }
 
+__device__ __forceinline__ void st_release(unsigned int *p, unsigned int v) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
 // ------------------------------------------------------------------------
 // Double-float ("df64") arithmetic on the FP32 pipes.  A value is an
 // unevaluated sum h + l of two floats with |l| <= ulp(h)/2 after

@@ -78,6 +78,12 @@ def test_no_return_with_copies_on_the_way(f, k, body):
     assert not _leaves_early(body)
 
 
+@pytest.mark.parametrize("f,k,body", KERNELS, ids=[f"{f}-{k}" for f, k, _ in KERNELS])
+def test_flags_are_released(f, k, body):
+    """Words that other blocks poll with acquire loads are never stored plainly."""
+    assert not re.search(r"\bflags\s*\[[^;]*?\]\s*=[^=]", body)
+
+
 def test_the_check_sees_an_early_return():
     assert _leaves_early("mbar_expect(&b, 16); if (gave_up) return; tr_wait(&b, 0);")
     assert _leaves_early("for (;;) { if (gave_up) { g(); return; } tr_wait(&b, 0); f(); mbar_expect(&b, 16); }")
