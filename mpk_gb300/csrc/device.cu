@@ -2486,16 +2486,20 @@ bool host_parallel(int count, F &&fn) {
 
 // Groups of consecutive matrices within `budget` bytes (matrix + two
 // levels of vectors); per group, CTA row ranges of equal nonzeros and the
-// CTAs owning each range's columns.  A small group takes fewer CTAs, and its
-// ranges end with its matrices, since a level costs a hand-over between CTAs
-// (some 5 K cycles) whatever its size, and a matrix that stays whole has none.
-// CSR kernel: groups of fewer rows than the grid has row slots (`threads` /
-// lpr per CTA, a pass of the CTA's threads); a pass per CTA, matrices of up to
-// two passes whole.  Windows: by work, of which 10 units a row slot take as
-// long as a hand-over; a CTA has that much or more, matrices of up to one and
-// a half hand-overs stay whole (41 matrices of 335-2744 rows, 4 right-hand
-// sides, 4 levels, one CTA per SM: 23 us, by rows as above 48, for parts and
-// whole matrices of twice that 28 and more; 20 of 500-2500, 16 sides: 23 / 28).
+// CTAs owning each range's columns.
+// With windows (a CTA holds one copy of a level's rows), a small group takes
+// fewer CTAs, and its ranges end with its matrices, since a level costs a
+// hand-over between CTAs (some 5 K cycles) whatever its size, and a matrix
+// that stays whole has none: by work, of which 10 units a row slot (`threads` /
+// lpr per CTA, a pass of the CTA's threads) take as long as a hand-over; a CTA
+// has that much or more, matrices of up to one and a half hand-overs stay
+// whole (41 matrices of 335-2744 rows, 4 right-hand sides, 4 levels, one CTA
+// per SM: 23 us, with a pass of rows per CTA and matrices of up to two whole
+// 48; 20 of 500-2500, 16 sides: 23 / 28).  The CSR kernel reads from L2 at
+// every entry and has several small CTAs per SM: it is fastest spread over all
+// of them whatever the size (a pass of rows per CTA, matrices of up to two
+// passes whole: 6 matrices of 300-3000 rows, 2 sides, 4 levels 55 -> 76 us,
+// 40000 rows, 1 side 43 -> 77).
 int batch_ranges(const BatchHost &h, int nrhs, long budget, bool windows, int grid, int threads, int lpr,
                  BatchLayout *out) {
   const int nmat = (int)h.mat_row0.size() - 1;
@@ -2540,17 +2544,15 @@ int batch_ranges(const BatchHost &h, int nrhs, long budget, bool windows, int gr
     long part = std::max(10 * pass, share);
     auto parts_of = [&](int m) {
       const long r0 = h.mat_row0[m], r1 = h.mat_row0[m + 1], w = work(r1) - work(r0);
-      if (windows) return w <= std::max(15 * pass, part) ? 1L : (w + part - 1) / part;
-      return r1 - r0 <= 2 * pass ? 1L : (r1 - r0 + pass - 1) / pass;
+      return w <= std::max(15 * pass, part) ? 1L : (w + part - 1) / part;
     };
     auto parts_all = [&] {
       long n = 0;
       for (int m = g0[g]; m < g0[g + 1]; m++) n += parts_of(m);
       return n;
     };
-    const bool few = windows ? g0[g + 1] - g0[g] <= grid && share <= 40 * pass : z - a <= pass * grid;
-    if (few) {
-      while (windows && parts_all() > grid) part += part / 8 + 1;
+    if (windows && g0[g + 1] - g0[g] <= grid && share <= 40 * pass) {
+      while (parts_all() > grid) part += part / 8 + 1;
       for (int m = g0[g]; m < g0[g + 1]; m++) {
         const long r0 = h.mat_row0[m], r1 = h.mat_row0[m + 1], parts = parts_of(m);
         const long q0 = work(r0), nz = work(r1) - q0;

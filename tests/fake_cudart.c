@@ -11,6 +11,8 @@
 static FILE *out;
 static size_t live, peak, limit = (size_t)-1; /* bytes of device memory */
 static int status;                            /* what the next int read from the device says, once */
+static struct { void *to; size_t bytes; } up[4096]; /* the latest copies to the device */
+static int nup;
 static const void *fun[512];
 static const char *name[512];
 static int nfun;
@@ -29,6 +31,11 @@ void fake_limit(size_t bytes) { limit = bytes; }
 void fake_status(int s) { status = s; }
 size_t fake_live(void) { return live; }
 size_t fake_peak(void) { return peak; }
+void *fake_upload(size_t bytes, int back) { /* where the latest copy of that size went, but `back` */
+  for (int i = nup; i-- > 0 && i > nup - 4096;)
+    if (up[i % 4096].bytes == bytes && back-- == 0) return up[i % 4096].to;
+  return NULL;
+}
 void fake_mark(const char *what) { fprintf(log_file(), "mark %s\n", what); }
 
 /* ---- registration ---- */
@@ -147,6 +154,10 @@ cudaError_t cudaPointerGetAttributes(struct cudaPointerAttributes *a, const void
 }
 cudaError_t cudaGetSymbolAddress(void **p, const void *s) { return cudaErrorNotSupported; }
 static void copied(void *d, size_t n, enum cudaMemcpyKind k) {
+  if (k == cudaMemcpyHostToDevice) {
+    up[nup % 4096].to = d;
+    up[nup++ % 4096].bytes = n;
+  }
   if (status && k == cudaMemcpyDeviceToHost && n == sizeof(int)) {
     *(int *)d = status;
     status = 0;

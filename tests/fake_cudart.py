@@ -15,6 +15,10 @@ import mpk_gb300 as M
 fake = C.CDLL(None)
 fake.fake_limit.argtypes = [C.c_size_t]
 fake.fake_live.restype = fake.fake_peak.restype = C.c_size_t
+fake.fake_upload.argtypes, fake.fake_upload.restype = [C.c_size_t, C.c_int], C.c_void_p
+def upload(count, dtype, back=0):
+    p = fake.fake_upload(count * np.dtype(dtype).itemsize, back)
+    return np.ctypeslib.as_array((C.c_byte * (count * np.dtype(dtype).itemsize)).from_address(p)).view(dtype)
 def mark(s): fake.fake_mark(s.encode())
 def live(): return int(fake.fake_live())
 def peak(): return int(fake.fake_peak())
