@@ -1657,23 +1657,26 @@ struct VecF<4> {
 };
 
 template <int LPR, int VW>
-__global__ void __launch_bounds__(256) batch_kernel(BatchArgs a) {
+__global__ void __launch_bounds__(256, VW == 4 ? 6 : 8) batch_kernel(BatchArgs a) {
   __shared__ int s_abort;
-  if (threadIdx.x == 0) s_abort = 0;
+  __shared__ unsigned s_base;  // where the last call left every flag
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    s_base = a.flags[blockIdx.x];
+  }
   __syncthreads();
   const int b = blockIdx.x, nrhs = LPR * VW;
   const int lane = (int)threadIdx.x % LPR, rpp = (int)blockDim.x / LPR;
-  const unsigned base = a.flags[b];  // where the last call left every flag
   for (int g = 0; g < a.ngroup; g++) {
     const int r0 = a.row_lo[(size_t)g * (a.nblk + 1) + b], r1 = a.row_lo[(size_t)g * (a.nblk + 1) + b + 1];
-    const unsigned tag = base + (unsigned)g * (unsigned)(a.nlevel + 1);
     const int dlo = a.dep_ptr[(size_t)g * a.nblk + b], dhi = a.dep_ptr[(size_t)g * a.nblk + b + 1];
     for (int l = 1; l <= a.nlevel; l++) {
       if (l > 1) {  // the CTAs owning this range's columns have published level l-1 of group g
+        const unsigned want = s_base + (unsigned)(g * (a.nlevel + 1) + l - 1) + a.stall;
         for (int k = dlo + (int)threadIdx.x; k < dhi; k += blockDim.x) {
           const int c = a.dep_idx[k];
           long spins = 0;
-          while ((int)(ld_acquire(a.flags + c) - (tag + (unsigned)(l - 1) + a.stall)) < 0) {
+          while ((int)(ld_acquire(a.flags + c) - want) < 0) {
             if (++spins > kSpinLimit || *((volatile int *)a.err)) {
               atomicCAS(a.err, 0, kErrTimeout);
               s_abort = 1;
@@ -1719,13 +1722,13 @@ __global__ void __launch_bounds__(256) batch_kernel(BatchArgs a) {
         }
         VecF<VW>::st(dst + (size_t)i * nrhs, acc);
       }
-      __syncthreads();  // as in wave_publish: the release store is cumulative
-      if (threadIdx.x == 0) {
-        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.flags + b), "r"(tag + (unsigned)l) : "memory");
+      if (l < a.nlevel) {  // nobody waits for the last level
+        __syncthreads();   // as in wave_publish: the release store is cumulative
+        if (threadIdx.x == 0) st_release(a.flags + b, s_base + (unsigned)(g * (a.nlevel + 1) + l));
       }
     }
   }
-  if (threadIdx.x == 0) st_release(a.flags + b, base + (unsigned)a.ngroup * (unsigned)(a.nlevel + 1));
+  if (threadIdx.x == 0) st_release(a.flags + b, s_base + (unsigned)(a.ngroup * (a.nlevel + 1)));
 }
 
 // The batched rows with the previous level in shared memory and the matrix
@@ -1920,9 +1923,9 @@ __global__ void __launch_bounds__(1024) batch_pack_kernel(BatchArgs a) {
         for (int t = 0; t < kBpRing; t++) fetch(t, t);
       }
       __syncthreads();  // rows written and the window read; the release store is cumulative
-      if (threadIdx.x == 0) {
-        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.flags + b), "r"(tag + (unsigned)l) : "memory");
-        if (l < a.nlevel && un.iv1 > un.iv0) {
+      if (threadIdx.x == 0 && l < a.nlevel) {  // nobody waits for the last level
+        st_release(a.flags + b, tag + (unsigned)l);
+        if (un.iv1 > un.iv0) {
           // the next level's own rows, while the neighbours finish theirs:
           // the release above has ordered the CTA's writes before the copies
           asm volatile("fence.proxy.async;" ::: "memory");
