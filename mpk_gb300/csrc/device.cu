@@ -743,11 +743,16 @@ __device__ __forceinline__ int ld_off(const short *p) {
 
 // One row's sum over its entries (CSR order): the row's int16 offsets are
 // RS apart (32: per-lane layout, a constant after inlining; 1: a slice's
-// shared list), values and int32 columns 32 apart.  The first 8 (12 for FP32)
-// entries have all their loads in flight together, whatever the row's
-// length; the first product runs on the integer pipes (128^3 1/deg, 8 levels:
-// 270 -> 249 us; 9-point diffusion 1400 x 1300 in FP64, whose rows of 9 used
-// to load entry by entry: 360 -> 293 us).
+// shared list), values and int32 columns 32 apart.  The first 8 entries have
+// all their loads in flight together, whatever the row's length; the first
+// product runs on the integer pipes (128^3 1/deg, 8 levels: 270 -> 249 us;
+// 9-point diffusion 1400 x 1300 in FP64, whose rows of 9 used to load entry by
+// entry: 360 -> 293 us).  The others go four at a time: written out for fused
+// multiply-adds with values, where the compiler's own unrolling spills, and
+// left to the compiler otherwise, where it is the faster (us before this loop
+// was unrolled / 8 loads in flight only / so, 6 levels: 27-point 31^3 with
+// values 67 / 76 / 65, 40 entries a row, 5000 rows 61 / 63 / 47; 1/deg 27-point
+// 40^3, separate rounding, 85 / 88 / 76, 64^3 244 / 227 / 171).
 template <int ARITH, bool VALUED, bool REL, bool STAGE>
 __device__ __forceinline__ double fp_row(int len, int RS, double cf, const short *cr, const int *cc,
                                          const double *cv, const double *xb, const double *src) {
@@ -764,9 +769,25 @@ __device__ __forceinline__ double fp_row(int len, int RS, double cf, const short
 #pragma unroll
   for (int u = 1; u < 8; u++)
     if (u < len) s = u < kIntTerms ? row_next<ARITH>(s, v[u], x[u]) : row_term<ARITH>(s, v[u], x[u]);
-  for (int t = 8; t < len; t++)
-    s = row_term<ARITH>(s, VALUED ? __ldg(cv + 32L * t) : cf,
-                        REL ? xb[ld_off<STAGE>(cr + RS * t)] : src[__ldg(cc + 32L * t)]);
+  auto x_at = [&](int t) { return REL ? xb[ld_off<STAGE>(cr + RS * t)] : src[__ldg(cc + 32L * t)]; };
+  int t = 8;
+  if (VALUED && ARITH != MPKG_ARITH_SEPARATE) {
+    for (; t + 4 <= len; t += 4) {
+      double y[4], w[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        y[u] = x_at(t + u);
+        w[u] = __ldg(cv + 32L * (t + u));
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) s = row_term<ARITH>(s, w[u], y[u]);
+    }
+#pragma unroll 1
+    for (; t < len; t++) s = row_term<ARITH>(s, __ldg(cv + 32L * t), x_at(t));
+  } else {
+#pragma unroll 4
+    for (; t < len; t++) s = row_term<ARITH>(s, VALUED ? __ldg(cv + 32L * t) : cf, x_at(t));
+  }
   return s;
 }
 

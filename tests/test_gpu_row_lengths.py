@@ -1,0 +1,41 @@
+"""Rows of every length around the groups that the FP64 row sums go in (8
+entries ahead, then fours; fours and their remainder in the k-SpMV), in the
+general wavefront and in k-SpMV launches of fewer and of more blocks than SMs,
+bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+import mpk_gb300 as M
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(n, uniform, seed):
+    """Row i has (i + i // 32) % 46 entries (slices of one length each if `uniform`), columns near it."""
+    rng = np.random.default_rng(seed)
+    i = np.arange(n)
+    length = np.where(i // 32 % 2 == 0, i // 64 % 46, (i + i // 32) % 46) if not uniform else i // 32 % 46
+    ptr = np.concatenate([[0], np.cumsum(length)]).astype(np.int32)
+    row = np.repeat(i, length)
+    off = np.arange(ptr[-1]) - ptr[row]
+    col = np.clip(row + 3 * off - 60 - rng.integers(0, 3, n)[row], None, n - 1)
+    col = np.where(col < 0, off, col).astype(np.int32)
+    return M.Csr(ptr, col, rng.normal(size=int(ptr[-1])))
+
+
+@pytest.mark.parametrize("plan", ["wave", "spmv"])
+@pytest.mark.parametrize("n,uniform", [(3001, False), (20011, True), (60013, False)])
+@pytest.mark.parametrize("valued", [False, True])
+@pytest.mark.parametrize("arith", [M.ARITH_FMA, M.ARITH_SEPARATE])
+def test_every_row_length(plan, n, uniform, valued, arith, gpu):
+    a = _matrix(n, uniform, 3)
+    a = a if valued else M.Csr(a.ptr, a.col)
+    k = 3
+    x = M.uniform(5, n)
+    p = M.Plan.wave(a, k, arith=arith) if plan == "wave" else M.Plan.spmv(a, k, arith=arith)
+    vv = np.zeros((k + 1) * n)
+    vv[:n] = x
+    p.exec_host(vv)
+    want = O.mpk(a.ptr, a.col, a.val, x, k, O.MODE_FMA if arith == M.ARITH_FMA else O.MODE_SEPARATE)
+    assert vv.tobytes() == want.tobytes()
