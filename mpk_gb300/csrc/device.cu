@@ -43,7 +43,8 @@ __device__ __forceinline__ double ld_cg(const double *p) { return __ldcg(p); }
 // ------------------------------------------------------------------------
 // k-SpMV: one launch per level, one thread per row.
 // ------------------------------------------------------------------------
-template <int ARITH, bool VALUED>
+// INT: the launch keeps the FP64 pipe busy (launch_spmv).
+template <int ARITH, bool VALUED, bool INT>
 __global__ void __launch_bounds__(256) spmv_level_kernel(int n, const int *__restrict__ ptr,
                                                          const int *__restrict__ col,
                                                          const double *__restrict__ coef,
@@ -55,13 +56,11 @@ __global__ void __launch_bounds__(256) spmv_level_kernel(int n, const int *__res
   const double a = VALUED ? 0.0 : coef[i];  // 1/deg, rounded on the host exactly as 1.0/deg
   double s = 0.0;
   int j = j0;
-  if (ARITH == MPKG_ARITH_SEPARATE) {
+  if (INT) {
     // three products of four on the integer pipes, the fourth beside them on
     // the FP64 pipe (97 x 96 x 95 diffusion, 6 levels: 175 us with all on the
     // FP64 pipe, 136 with none, 128 so; groups of 2, 3, 5, 6: 164, 130, 129,
-    // 152).  With the first product ahead of the groups that is 124, but small
-    // launches, bound by the row's chain of loads, lose a fifth (100 x 101
-    // 1/deg, 6 levels: 25 / 31); so do FMA rows, which keep the plain loop.
+    // 152)
     constexpr int G = 4;
     for (; j + G <= j1; j += G) {
       double xv[G], v[G];
@@ -75,7 +74,8 @@ __global__ void __launch_bounds__(256) spmv_level_kernel(int n, const int *__res
       for (int u = 1; u < G; u++) s = u < G - 1 ? row_next<ARITH>(s, v[u], xv[u]) : row_term<ARITH>(s, v[u], xv[u]);
     }
   }
-  for (; j < j1; j++) s = row_next<ARITH>(s, VALUED ? coef[j] : a, x[col[j]]);
+  for (; j < j1; j++)
+    s = INT ? row_next<ARITH>(s, VALUED ? coef[j] : a, x[col[j]]) : row_term<ARITH>(s, VALUED ? coef[j] : a, x[col[j]]);
   y[i] = s;
 }
 
@@ -2938,17 +2938,21 @@ int batch_launch(mpkg_plan *p, float *d_vb, cudaStream_t st) {
 int launch_spmv(int n, const int *ptr, const int *col, const double *coef, bool valued, int nlevel,
                 double *vv, int arith, cudaStream_t st) {
   dim3 blk(256), grd((n + 255) / 256);
-  for (int l = 1; l <= nlevel; l++) {
-    const double *x = vv + (long)(l - 1) * n;
-    double *y = vv + (long)l * n;
-    if (arith == MPKG_ARITH_SEPARATE) {
-      if (valued) spmv_level_kernel<MPKG_ARITH_SEPARATE, true><<<grd, blk, 0, st>>>(n, ptr, col, coef, x, y);
-      else spmv_level_kernel<MPKG_ARITH_SEPARATE, false><<<grd, blk, 0, st>>>(n, ptr, col, coef, x, y);
-    } else {
-      if (valued) spmv_level_kernel<MPKG_ARITH_FMA, true><<<grd, blk, 0, st>>>(n, ptr, col, coef, x, y);
-      else spmv_level_kernel<MPKG_ARITH_FMA, false><<<grd, blk, 0, st>>>(n, ptr, col, coef, x, y);
-    }
-  }
+  // With separate rounding a level of more blocks than SMs is bound by the FP64
+  // pipe, which products on the integer pipes relieve; up to there by each
+  // row's chain of loads and sums, which they lengthen (7-point 43^3, 6
+  // levels: 46 us without and 41 with them; 27-point 31^3 55 and 64, 36^3 78
+  // and 66; 20000 rows of 5-30 entries 54 and 65, 40000 rows 79 and 66).
+  int dev = 0, nsm = 0;
+  CUDA_TRY(cudaGetDevice(&dev));
+  CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const bool ints = arith == MPKG_ARITH_SEPARATE && (int)grd.x > nsm;
+  auto kernel = arith != MPKG_ARITH_SEPARATE
+                    ? (valued ? spmv_level_kernel<MPKG_ARITH_FMA, true, false> : spmv_level_kernel<MPKG_ARITH_FMA, false, false>)
+                : ints ? (valued ? spmv_level_kernel<MPKG_ARITH_SEPARATE, true, true> : spmv_level_kernel<MPKG_ARITH_SEPARATE, false, true>)
+                       : (valued ? spmv_level_kernel<MPKG_ARITH_SEPARATE, true, false> : spmv_level_kernel<MPKG_ARITH_SEPARATE, false, false>);
+  for (int l = 1; l <= nlevel; l++)
+    kernel<<<grd, blk, 0, st>>>(n, ptr, col, coef, vv + (long)(l - 1) * n, vv + (long)l * n);
   CUDA_TRY(cudaGetLastError());
   return kOk;
 }
