@@ -413,12 +413,49 @@ int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int
   const int W = l.w;
   // slice-aligned row ranges of equal length: a slice costs the same with
   // and without its holes
-  for (int i = 0; i < n; i++)
-    if (ptr[i + 1] - ptr[i] > 65535) return kOk;  // refused by the general wavefront
   const int grid = l.grid = std::min(nsm, nslice);
   l.lo.assign(grid + 1, 0);
   for (int b = 1; b <= grid; b++) l.lo[b] = (int)std::min<long>(n, 32L * ((long)nslice * b / grid));
   const int own = 32 * ((nslice + grid - 1) / grid);
+  // Levels per exchange and the halo.  With one level, not 9 diagonals, the
+  // halo holds all of them or all but the outermost pair: the first fetches 2
+  // halo rows per CTA and level, the second two per own row, so a halo beyond
+  // the own rows is taken only where the second does not do.  With more levels
+  // it holds all.  A call's time in cycles, as measured: a hand-over 4500 and
+  // the halo's rows, a barrier 200, a slice its share of the FP64 or issue
+  // slots, a level at least the latency of one slice; once, the values of the
+  // neighbours' slices.
+  const bool pair = W < 9 && l.d[0] < 0 && l.d[W - 1] > 0;
+  const bool fp64 = eb == 8 && !ring;
+  const double per_slice = (fp64 ? 20.0 : ring ? 9.0 : 4.5) * W, least = fp64 ? 120.0 * W : ring ? 80.0 * W : 500.0;
+  const long reach = std::max({0, -l.d[0], l.d[W - 1]}), ns_max = own / 32;
+  l.win_bytes = (int)((own * eb + 15) / 16 * 16);
+  l.grow = (int)((reach + 31) / 32);
+  double best = -1;
+  auto consider = [&](int depth, int g) {  // false: does not fit
+    const long halo = 32L * (depth - 1) * l.grow + (g ? std::max({0, -l.d[1], l.d[W - 2]}) : reach);
+    const long hb = (halo * eb + 15) / 16 * 16, most = ns_max + 2L * (depth - 1) * l.grow;
+    if (2L * l.win_bytes + (depth > 1 ? 4 : 3) * hb + (2 * most + 16) > smem) return false;
+    double cost = 0.4 * halo * ((nlevel + depth - 1) / depth) + 2.0 * (depth - 1) * l.grow * W * 32 * vb / 24;
+    for (int lev = 0; lev < nlevel; lev++) {
+      const int left = std::min(depth, nlevel - lev / depth * depth) - 1 - lev % depth;
+      cost += (lev == 0 ? 0 : lev % depth == 0 ? 4500 : 200) +
+              std::max(least, per_slice * std::min<long>(nslice, ns_max + 2L * left * l.grow));
+    }
+    if (best >= 0 && cost > 0.95 * best) return true;
+    best = cost;
+    l.depth = depth;
+    l.mode = g ? kDiagPair : depth > 1 ? kDiagDeep : kDiagAll;
+    l.halo = (int)std::min<long>(halo, n);
+    l.halo_bytes = (int)hb;
+    l.second = (int)(l.win_bytes + (depth > 1 ? 2 : 1) * hb);
+    l.win_at = (int)(smem - l.second - l.win_bytes - hb);
+    return true;
+  };
+  const bool near = !pair || reach <= own;
+  if (!(near && consider(1, 0)) && !(pair && consider(1, 1)) && !consider(1, 0)) return kOk;  // too large
+  for (int i = 0; i < n; i++)
+    if (ptr[i + 1] - ptr[i] > 65535) return kOk;  // refused by the general wavefront
   // patterns
   l.pat.assign(nslice, 0);
   std::map<std::vector<unsigned short>, int> known;
@@ -458,44 +495,7 @@ int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int
     known[m] = l.pat[sl];
     l.mask.insert(l.mask.end(), m.begin(), m.end());
   }
-  // Levels per exchange and the halo.  With one level, not 9 diagonals, the
-  // halo holds all of them or all but the outermost pair: the first fetches 2
-  // halo rows per CTA and level, the second two per own row, so a halo beyond
-  // the own rows is taken only where the second does not do.  With more levels
-  // it holds all.  A call's time in cycles, as measured: a hand-over 4500 and
-  // the halo's rows, a barrier 200, a slice its share of the FP64 or issue
-  // slots, a level at least the latency of one slice; once, the values of the
-  // neighbours' slices.
-  const bool pair = W < 9 && l.d[0] < 0 && l.d[W - 1] > 0;
-  const bool fp64 = eb == 8 && !ring;
-  const double per_slice = (fp64 ? 20.0 : ring ? 9.0 : 4.5) * W, least = fp64 ? 120.0 * W : ring ? 80.0 * W : 500.0;
-  const long reach = std::max({0, -l.d[0], l.d[W - 1]}), ns_max = own / 32;
-  l.win_bytes = (int)((own * eb + 15) / 16 * 16);
-  l.grow = (int)((reach + 31) / 32);
-  double best = -1;
-  auto consider = [&](int depth, int g) {  // false: does not fit
-    const long halo = 32L * (depth - 1) * l.grow + (g ? std::max({0, -l.d[1], l.d[W - 2]}) : reach);
-    const long hb = (halo * eb + 15) / 16 * 16, most = ns_max + 2L * (depth - 1) * l.grow;
-    if (2L * l.win_bytes + (depth > 1 ? 4 : 3) * hb + (2 * most + 16) > smem) return false;
-    double cost = 0.4 * halo * ((nlevel + depth - 1) / depth) + 2.0 * (depth - 1) * l.grow * W * 32 * vb / 24;
-    for (int lev = 0; lev < nlevel; lev++) {
-      const int left = std::min(depth, nlevel - lev / depth * depth) - 1 - lev % depth;
-      cost += (lev == 0 ? 0 : lev % depth == 0 ? 4500 : 200) +
-              std::max(least, per_slice * std::min<long>(nslice, ns_max + 2L * left * l.grow));
-    }
-    if (best >= 0 && cost > 0.95 * best) return true;
-    best = cost;
-    l.depth = depth;
-    l.mode = g ? kDiagPair : depth > 1 ? kDiagDeep : kDiagAll;
-    l.halo = (int)std::min<long>(halo, n);
-    l.halo_bytes = (int)hb;
-    l.second = (int)(l.win_bytes + (depth > 1 ? 2 : 1) * hb);
-    l.win_at = (int)(smem - l.second - l.win_bytes - hb);
-    return true;
-  };
-  const bool near = !pair || reach <= own;
-  if (!(near && consider(1, 0)) && !(pair && consider(1, 1)) && !consider(1, 0)) return kOk;
-  if (!irregular)
+  if (!irregular)  // more levels per exchange
     for (int depth = 2; depth <= std::min(nlevel, kDiagMaxDepth) && consider(depth, 0); depth++) {
     }
   // per CTA: slice ranges, resident values, dependencies
