@@ -463,6 +463,24 @@ int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int
   std::vector<unsigned short> m(32);
   known[std::vector<unsigned short>(32, all)] = 0;
   l.mask.assign(32, all);
+  // Rows of irregular slices run one entry after another, from the CSR, where
+  // the general wavefront has 8 entries in flight.  That costs 350 cycles an
+  // entry for these 8 (double-float 650, and 250 for each further one, which
+  // the other forms take no slower than the general wavefront), and a CTA one
+  // cycle for each of its irregular slices' entries (of a row's first 8), six
+  // for those outside its window.  It has to stay below what the other slices
+  // gain, of which columns beyond 16 bits, which the general wavefront reads
+  // as 32, make 1.6 times as much; and one slice in twenty may be irregular.  us,
+  // 5 levels, general / with any such rows / by this rule: 110^3 1/deg, every
+  // 25th slice with one row of columns anywhere 168 / 104 / 104, the first 1 %
+  // of the rows so 175 / 1024 / 175, the first 4 % with columns within 3000
+  // 164 / 239 / 164; 100^2, 32 rows of columns anywhere 22.6 / 25.9 / 22.6;
+  // double-float 110^3 212 / 116 / 116, 188 / 924 / 188, 197 / 295 / 197.
+  const double spare = fp64 ? std::max(std::min(8000.0, 1900 + 130.0 * ns_max), 0.25 * per_slice * ns_max)
+                            : std::max(std::min(12000.0, 2500 + 200.0 * ns_max), 0.45 * per_slice * ns_max);
+  int cta = 0;
+  long loads = 0, worst = 0;  // of CTA `cta`, of all
+  bool wide = false;
   long &irregular = l.irregular = 0;
   for (int sl = 0; sl < nslice; sl++) {
     bool ok = true;
@@ -479,9 +497,22 @@ int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int
       m[i & 31] = (unsigned short)bits;
       full &= bits == all;
     }
-    if (!ok) {  // its rows run one entry after another: at most one slice in twenty
+    if (!ok) {
       l.pat[sl] = kDiagIrregular;
       if (++irregular * 20 > nslice) return kOk;
+      while (l.lo[cta + 1] <= sl * 32) {
+        cta++;
+        loads = 0;
+      }
+      for (int i = sl * 32; i < std::min(n, sl * 32 + 32); i++) {
+        const int len = ptr[i + 1] - ptr[i], ahead = std::min(len, 8);
+        loads += ahead;
+        for (int q = ptr[i]; q < ptr[i + 1]; q++) {
+          if (q < ptr[i] + ahead && (col[q] < l.lo[cta] - l.halo || col[q] >= l.lo[cta + 1] + l.halo)) loads += 5;
+          wide |= std::abs(col[q] - i) > 32767;
+        }
+        worst = std::max({worst, loads, ahead * (ring ? 650L : 350L) + (ring ? (len - ahead) * 250L : 0L)});
+      }
       continue;
     }
     if (full) continue;
@@ -495,6 +526,7 @@ int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int
     known[m] = l.pat[sl];
     l.mask.insert(l.mask.end(), m.begin(), m.end());
   }
+  if (worst > (wide ? 1.6 : 1.0) * spare) return kOk;
   if (!irregular)  // more levels per exchange
     for (int depth = 2; depth <= std::min(nlevel, kDiagMaxDepth) && consider(depth, 0); depth++) {
     }
