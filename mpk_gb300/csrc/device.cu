@@ -3537,11 +3537,12 @@ int diag_setup(mpkg_plan *p, int form, const int *ptr, const int *col, const dou
   int rc = diag_layout(n, ptr, col, p->nlevel, form, nsm, smem, &l);
   if (rc || !l.fits) return rc;
   const void *fn = diag_kernel_ptr(form, l.w, l.mode);
+  // the limit of a function is the largest that any plan uses
   CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kDiagThreads, smem));
+  CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kDiagThreads, l.smem));
   if ((long)per_sm * nsm < l.grid) return kOk;
   DiagArgs &a = p->dg;
-  a.n = n; a.nlevel = p->nlevel; a.nblk = l.grid; a.halo = l.halo; a.smem = smem;
+  a.n = n; a.nlevel = p->nlevel; a.nblk = l.grid; a.halo = l.halo; a.smem = l.smem;
   a.depth = l.depth; a.grow = l.grow; a.win_at = l.win_at; a.second = l.second;
   a.ring_all = l.irregular > 0;
   for (int u = 0; u < l.w; u++) {

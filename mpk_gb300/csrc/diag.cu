@@ -533,6 +533,7 @@ int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int
   // per CTA: slice ranges, resident values, dependencies
   l.own.assign(grid, make_int2(0, 0));
   l.nres.assign(grid, 0);
+  long used = 0;  // bytes below the windows
   std::vector<std::vector<int>> waits(grid);
   auto owner = [&](int c) { return (int)(std::upper_bound(l.lo.begin(), l.lo.end() - 1, c) - l.lo.begin()) - 1; };
   for (int b = 0; b < grid; b++) {
@@ -550,10 +551,9 @@ int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int
       const int left = std::min(l.depth, nlevel - lev / l.depth * l.depth) - 1 - lev % l.depth, g = left * l.grow;
       l.rows += std::min<long>(n, 32L * (s0 + ns + std::min(nslice - s0 - ns, g))) - 32L * (s0 - std::min(s0, g));
     }
-    if (vb) {
-      const long room = l.win_at - l.halo_bytes - (2 * all + 15) / 16 * 16;
-      l.nres[b] = (int)std::min<long>(all, room / (vb * W * 32));
-    }
+    const long pats = (2 * all + 15) / 16 * 16, room = l.win_at - l.halo_bytes - pats;
+    if (vb) l.nres[b] = (int)std::min<long>(all, room / (vb * W * 32));
+    used = std::max(used, pats + l.nres[b] * vb * W * 32);
     std::vector<int> &wt = waits[b];
     int last = -1;
     for (int q = ptr[r0]; q < ptr[r1]; q++) {
@@ -572,6 +572,10 @@ int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int
     std::sort(wt.begin(), wt.end());
     wt.erase(std::unique(wt.begin(), wt.end()), wt.end());
   }
+  // what no CTA needs is left to other kernels
+  const long slack = (l.win_at - l.halo_bytes - used) / 128 * 128;
+  l.win_at -= (int)slack;
+  l.smem = smem - (int)slack;
   if (ring) {  // a ring slot is reused: wait for the readers of the own rows too
     const std::vector<std::vector<int>> reads(waits);
     for (int c = 0; c < grid; c++)

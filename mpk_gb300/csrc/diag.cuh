@@ -66,6 +66,7 @@ struct DiagLayout {
   int d[kDiagMax] = {};
   int halo = 0, win_bytes = 0, halo_bytes = 0, grid = 0;
   int depth = 1, grow = 0, win_at = 0, second = 0;
+  int smem = 0;                // dynamic shared memory that it needs
   int slices = 0;              // the most that a CTA computes at a level
   long reach = 0, irregular = 0, rows = 0;  // rows: computed by a call
   std::vector<int> lo, dptr, didx, nres;
@@ -73,9 +74,9 @@ struct DiagLayout {
   std::vector<unsigned short> pat, mask;
 };
 
-// The layout of the diagonal wavefront for `nsm` CTAs with `smem` bytes of
-// dynamic shared memory; fits is false where the structure or the sizes do
-// not suit it.  ring: dependencies both ways.
+// The layout of the diagonal wavefront for `nsm` CTAs with up to `smem` bytes
+// of dynamic shared memory; fits is false where the structure or the sizes do
+// not suit it.
 int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int nsm, int smem, DiagLayout *out);
 
 // Values along the layout's diagonals, [slice][diagonal][lane], zero where a

@@ -23,7 +23,7 @@ int main(int argc, char **argv) {
                                    std::atoi(argv[5]), &l);
   const double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   std::printf("{\"rc\": %d, \"ms\": %.3f, \"fits\": %d, \"w\": %d, \"mode\": %d, \"depth\": %d, \"halo\": %d, \"grid\": %d, "
-              "\"irregular\": %ld, \"rows\": %ld, \"scanned\": %zu, \"patterns\": %zu}\n",
-              rc, ms, (int)l.fits, l.w, l.mode, l.depth, l.halo, l.grid, l.irregular, l.rows, l.pat.size(),
+              "\"smem\": %d, \"win_at\": %d, \"irregular\": %ld, \"rows\": %ld, \"scanned\": %zu, \"patterns\": %zu}\n",
+              rc, ms, (int)l.fits, l.w, l.mode, l.depth, l.halo, l.grid, l.smem, l.win_at, l.irregular, l.rows, l.pat.size(),
               l.mask.size() / 32);
 }

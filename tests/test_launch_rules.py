@@ -20,3 +20,19 @@ p.exec_host(np.zeros(4 * a.n))
     got = _kernels(log, "spmv_level_kernel")
     want = f"spmv_level_kernelILi{code}ELb1ELb{int(ints and arith == 'SEPARATE')}E"
     assert len(got) == 3 and all(want in w[0] for w in got), got
+
+
+@pytest.mark.parametrize("make,k,most", [
+    ("M.Plan.wave(M.Csr.laplacian(100, 100).pattern(), 4)", 4, 20000),
+    ("M.Plan.wave(M.Csr.laplacian(100, 100), 4, arith=M.ARITH_DF64)", 4, 60000),
+    ("M.Plan.wave(M.Csr.laplacian(60, 60, 60).pattern(), 4)", 4, 40000),
+    ("M.Plan.wave(M.Csr.laplacian(128, 128, 128).pattern(), 4)", 4, 231424),
+])
+def test_diagonal_wavefront_takes_the_shared_memory_it_needs(make, k, most, tmp_path):
+    """A small plan leaves room on every SM, so that plans on several streams run side by side."""
+    log = fake_cudart.run(str(tmp_path), f"""
+p = {make}
+p.exec_host(np.zeros({k + 1} * p.n))
+""")
+    (kernel, blocks, threads, smem, _), = _kernels(log, "diag_kernel")
+    assert blocks <= 152 and smem <= most
