@@ -2180,6 +2180,12 @@ int dev_alloc(mpkg_plan *p, T **dst, size_t count) {
   return kOk;
 }
 
+void dev_free(mpkg_plan *p, void *q, size_t bytes) {  // of dev_copy or dev_alloc
+  p->owned.erase(std::find(p->owned.begin(), p->owned.end(), q));
+  p->device_bytes -= (long)bytes;
+  cudaFree(q);
+}
+
 // Clears device memory before it returns: cudaMemset does not wait for the
 // device, and the streams that plans and callers launch on do not wait for its.
 int dev_clear(void *q, size_t bytes) {
@@ -3579,6 +3585,9 @@ int diag_setup(mpkg_plan *p, int form, const int *ptr, const int *col, const dou
       float2 *v2 = nullptr;
       rc = dev_alloc(p, &v2, nv);
       if (!rc) split_kernel<<<592, 256, 0, p->stream>>>(v, v2, (long)nv);
+      if (!rc && (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(p->stream) != cudaSuccess))
+        rc = fail(kECuda, "split of the diagonal values failed");
+      dev_free(p, v, sizeof(double) * nv);  // the pairs take its place
       a.vals = v2;
     }
   } else if (!rc && form == kDiagF32) {
