@@ -3936,14 +3936,25 @@ int batch_configure(mpkg_plan *p, const BatchHost &h, const BatchCand &c, const 
   p->owned.resize(owned0);
   p->batch_bytes = p->device_bytes - bytes0;
   if (!rc && !c.staged && !a.ptr) {  // batch_kernel reads the CSR
+    const size_t csr0 = p->owned.size();
+    const long csr_bytes0 = p->device_bytes;
     int *d_ptr = nullptr, *d_col = nullptr;
     float *d_val = nullptr;
     rc = dev_copy(p, &d_ptr, h.ptr.data(), h.ptr.size());
     if (!rc) rc = dev_copy(p, &d_col, h.col.data(), h.col.size());
     if (!rc) rc = dev_copy(p, &d_val, h.val.data(), h.val.size());
-    a.ptr = d_ptr; a.col = d_col; a.val = d_val;
+    if (!rc) {
+      a.ptr = d_ptr; a.col = d_col; a.val = d_val;
+    } else {
+      for (size_t q = csr0; q < p->owned.size(); q++) cudaFree(p->owned[q]);
+      p->owned.resize(csr0);
+      p->device_bytes = csr_bytes0;
+    }
   }
-  if (rc) return rc;
+  if (rc) {
+    cudaGetLastError();
+    return rc;
+  }
   a.row_lo = d_lo; a.dep_ptr = d_dlo; a.dep_idx = d_dhi; a.flags = d_flags;
   a.nblk = grid; a.ngroup = lay.ngroup;
   p->batch_lpr = c.lpr; p->batch_vw = c.vw; p->batch_group_bytes = c.budget;
@@ -4058,7 +4069,7 @@ int mpkg_plan_batch(int nmat, const int *n, const int *const *ptr, const int *co
   if (!rc && cands.empty()) rc = fail(kEInval, "no kernel configuration for this nrhs");
   BatchCand best = cands.empty() ? BatchCand{1, 1, 0, 1, false, 256, 0} : cands[0];
   BatchLayout lay;
-  bool laid = false;  // lay is best's
+  bool laid = false, configured = false;  // lay is best's, and the plan's
   if (!rc && tune >= MPKG_BATCH_STAGED) {  // untimed staged configuration
     const int want_threads = tune == MPKG_BATCH_STAGED ? 1024 : tune == MPKG_BATCH_STAGED2 ? 512 : 256;
     bool found = false;
@@ -4072,18 +4083,19 @@ int mpkg_plan_batch(int nmat, const int *n, const int *const *ptr, const int *co
   } else if (!rc && tune == MPKG_BATCH_DEFAULT && packable) {
     // one CTA per SM (the least halo; two and four measure the same on large
     // batches and more on small ones); where its windows miss a fourth of the
-    // columns, the CSR kernel
+    // columns, or it cannot be made, the CSR kernel
     if (best.staged) {
-      rc = batch_build_layout(h, nrhs, best, &lay);
-      laid = !rc;
+      laid = batch_build_layout(h, nrhs, best, &lay) == kOk && 4 * lay.far <= nnz &&
+             batch_configure(p, h, best, lay) == kOk;
+      clear_error();
     }
-    if (!rc && (!best.staged || 4 * lay.far > nnz))
+    if (!laid)
       for (const BatchCand &c : cands)
         if (!c.staged) {
           best = c;
-          laid = false;
           break;
         }
+    configured = laid;
   } else if (!rc && tune == MPKG_BATCH_TUNE && cands.size() > 1) {
     // time every candidate on the plan's own matrices (zero input; the
     // arithmetic does not depend on the values)
@@ -4100,7 +4112,9 @@ int mpkg_plan_batch(int nmat, const int *n, const int *const *ptr, const int *co
     for (const BatchCand &c : cands) {
       if (rc) break;
       BatchLayout l;
-      if ((rc = batch_build_layout(h, nrhs, c, &l)) || (rc = batch_configure(p, h, c, l))) break;
+      // one that cannot be made (for want of memory, say) leaves it to the others
+      if (batch_build_layout(h, nrhs, c, &l) != kOk || batch_configure(p, h, c, l) != kOk) continue;
+      clear_error();
       for (int w = 0; w < 2 && !rc; w++) rc = batch_launch_raw(p, scratch, p->stream);
       if (!rc && cudaEventRecord(e0, p->stream) != cudaSuccess) rc = fail(kECuda, "event record");
       for (int w = 0; w < 3 && !rc; w++) rc = batch_launch_raw(p, scratch, p->stream);
@@ -4115,6 +4129,7 @@ int mpkg_plan_batch(int nmat, const int *n, const int *const *ptr, const int *co
         laid = true;
       }
     }
+    if (!rc && !laid) rc = fail(kENoMem, "no kernel configuration of this batch could be made");
     p->batch_tune_ms =
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
     if (e0) cudaEventDestroy(e0);
@@ -4123,7 +4138,7 @@ int mpkg_plan_batch(int nmat, const int *n, const int *const *ptr, const int *co
   }
   if (!rc && !laid) rc = batch_build_layout(h, nrhs, best, &lay);
   p->batch_candidates = (int)cands.size();
-  if (!rc) rc = batch_configure(p, h, best, lay);
+  if (!rc && !configured) rc = batch_configure(p, h, best, lay);
   if (rc) { mpkg_plan_destroy(p); return rc; }
   *out = p;
   return kOk;

@@ -22,3 +22,35 @@ for ctas in (0, 32):
     assert live() == 0
 assert held[0] <= held[1], held
 """)
+
+
+@pytest.mark.parametrize("mode", ["DEFAULT", "TUNE"])
+def test_batch_takes_the_csr_kernel_where_the_packed_matrix_finds_no_memory(mode, tmp_path):
+    """Rows of one entry take twice their CSR bytes when packed; a plan that
+    has a choice of kernels is made of those that fit, and refused where none does."""
+    fake_cudart.run(str(tmp_path), f"""
+n = 200000
+i = np.arange(n, dtype=np.int32)
+mats = [M.Csr(np.arange(n + 1, dtype=np.int32), i[::-1].copy() if q else i, np.ones(n)) for q in range(2)]
+vectors = 3 * 2 * n * 4 * 4 if "{mode}" == "TUNE" else 0
+p = M.Plan.batch(mats, 4, 2, tune=M.BATCH_STAGED)
+packed = live()
+p.close()
+csr = 2 * n * 12
+assert packed > csr + 1000000
+fake.fake_limit(csr + 500000)
+raises(M.ECUDA, lambda: M.Plan.batch(mats, 4, 2, tune=M.BATCH_STAGED))
+fake.fake_limit(csr + 500000 + vectors)
+p = M.Plan.batch(mats, 4, 2, tune=M.BATCH_{mode})
+assert not p.batch_info()["staged"] and live() == p.batch_info()["device_bytes"]
+p.exec_batch_device(1 << 20)
+p.close()
+fake.fake_limit(csr // 2 + vectors)
+assert live() == 0
+try:
+    M.Plan.batch(mats, 4, 2, tune=M.BATCH_{mode})
+    raise AssertionError("no error")
+except M.MpkError as e:
+    assert e.code in (M.ECUDA, M.ENOMEM) and str(e)
+assert live() == 0
+""")
