@@ -4477,7 +4477,9 @@ int mpkg_plan_mixed(int n, const int *ptr, const int *col, const double *val, in
       if (cudaStreamCreateWithFlags(&w->stream, cudaStreamNonBlocking) != cudaSuccess) rc = fail(kECuda, "stream creation failed");
       if (!rc && diag_setup(w, value_type == MPKG_VALUE_F32 ? kDiagF32 : kDiagBf16, ptr, col, val, &diag) != kOk)
         clear_error();  // the general wavefront, or the chunk pipeline
-      if (!diag) {
+      if (diag) {
+        p->rows_computed = w->rows_computed;  // with several levels per exchange some twice
+      } else {
         mpkg_plan_destroy(w);
         p->inner = nullptr;
       }

@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 
 import diag_probe as D
+import fake_cudart
 import mpk_gb300 as M
 
 
@@ -51,3 +52,16 @@ def test_irregular_rows_on_small_meshes():
     assert D.layout(a, D.FMA, 5)["fits"] and D.layout(a, D.FMA, 5)["mode"] == D.DEEP
     for form in (D.FMA, D.SEP, D.DF):
         assert not D.layout(_with_rows(a, [4321], None), form, 5)["fits"]
+
+
+@pytest.mark.parametrize("make", ["M.Csr.diffusion(120, 110, 1, sigma=0.5, seed=1)", "M.Csr.diffusion(40, 41, 42, sigma=0.5, seed=1)"])
+@pytest.mark.parametrize("vt,form", [("F32", D.F32), ("BF16", D.BF16)])
+def test_mixed_plans_count_the_rows_they_compute(make, vt, form, tmp_path):
+    """With several levels per exchange a block computes rows of its neighbours too."""
+    a = eval(make)
+    rows = D.layout(a, form, 8)["rows"]
+    assert rows > 8 * a.n or a.n > 20000
+    fake_cudart.run(str(tmp_path), f"""
+p = M.Plan.mixed({make}, 8, M.VALUE_{vt})
+assert p.info()["rows_computed"] == {rows}, (p.info(), {rows})
+""")
