@@ -405,6 +405,12 @@ void mpkg_plan_destroy(mpkg_plan *p);
  * MPKG_ETIMEOUT with the context still usable; 0 restores normal waits. */
 int mpkg_debug_pipe_stall(mpkg_plan *p, int extra_levels);
 
+/* Test hook: 1 when the plan runs the diagonal wavefront, with its mode (0:
+ * neighbours' rows from the halo, 1: the outermost pair of diagonals from
+ * global memory, 2: several levels per exchange), its levels per exchange and
+ * its slices of 32 rows with columns off the diagonals; else 0. */
+int mpkg_debug_plan_diag(const mpkg_plan *p, int *mode, int *depth, int *irregular);
+
 /* Allocation-free pipeline (no counterpart in the reference).  For callers
  * that must not allocate device memory themselves, e.g. a solver plug-in
  * running inside an application whose memory pool owns the whole device, or

@@ -118,6 +118,7 @@ def _declare(L):
         "mpkg_exec_device": (I, [P, P, P]),
         "mpkg_sync": (I, [P, P]),
         "mpkg_plan_destroy": (None, [P]),
+        "mpkg_debug_plan_diag": (I, [P, P, P, P]),
         "mpkg_debug_pipe_stall": (I, [P, I]),
         "mpkg_spmv_chain_device": (I, [I, P, P, P, I, P, I, P]),
         "mpkg_read_metis": (I, [C.c_char_p, C.POINTER(I), C.POINTER(Lg), pp, pp]),
@@ -678,6 +679,12 @@ class Plan:
         """Test hook: pipeline waits target `extra_levels` beyond the real
         level (0 restores normal behaviour)."""
         _check(lib().mpkg_debug_pipe_stall(self._h, extra_levels))
+
+    def debug_diag(self):
+        """Test hook: (mode, levels per exchange, irregular slices) of a plan
+        on the diagonal wavefront, None for the others."""
+        v = [C.c_int() for _ in range(3)]
+        return tuple(x.value for x in v) if lib().mpkg_debug_plan_diag(self._h, *(C.byref(x) for x in v)) else None
 
     def close(self):
         if self._h is not None and self._h.value:

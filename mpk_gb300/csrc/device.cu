@@ -2112,7 +2112,7 @@ struct mpkg_plan {
   bool wave_uni = false;  // pattern-compressed offsets (plans with matrix values)
   DiagArgs dg{};          // rows on a few diagonals: the diagonal wavefront
   bool dg_on = false;
-  int dg_form = 0, dg_w = 0, dg_mode = 0, dg_threads = 0;
+  int dg_form = 0, dg_w = 0, dg_mode = 0, dg_threads = 0, dg_irregular = 0;
   // batched block-vector form
   BatchArgs batch{};
   int batch_lpr = 0, batch_vw = 0, batch_nmat = 0;
@@ -3628,7 +3628,7 @@ int diag_setup(mpkg_plan *p, int form, const int *ptr, const int *col, const dou
   p->pipe_grid = l.grid;
   p->pipe_reach = (int)l.reach;
   p->rows_computed = l.rows;
-  p->dg_form = form; p->dg_w = l.w; p->dg_mode = l.mode;
+  p->dg_form = form; p->dg_w = l.w; p->dg_mode = l.mode; p->dg_irregular = (int)l.irregular;
   p->dg_threads = std::min(kDiagThreads, std::max(128, 32 * l.slices));  // a warp per slice, as far as they go
   p->dg_on = true;
   *done = true;
@@ -4943,6 +4943,16 @@ int mpkg_exec_mixed_device(mpkg_plan *p, float *d_vv, void *stream) {
   CUDA_TRY(cudaGetLastError());
   p->launches = 1;
   return kOk;
+}
+
+int mpkg_debug_plan_diag(const mpkg_plan *p, int *mode, int *depth, int *irregular) {
+  if (!p || !mode || !depth || !irregular) return 0;
+  if (p->inner) p = p->inner;
+  if (!p->dg_on) return 0;
+  *mode = p->dg_mode;
+  *depth = p->dg.depth;
+  *irregular = p->dg_irregular;
+  return 1;
 }
 
 int mpkg_debug_pipe_stall(mpkg_plan *p, int extra_levels) {
