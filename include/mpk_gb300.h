@@ -229,6 +229,9 @@ int mpkg_cg(int n, const int *ptr, const int *col, const double *val, const doub
 #define MPKG_GRAM_FP64 0
 #define MPKG_GRAM_DF64 1
 int mpkg_sstep_gram(int mode);
+/* Test hook: the Gram matrix g (ncol x ncol, ncol <= 21) of the columns y
+ * (ncol x n, host arrays) in the mode of the calling thread's solves. */
+int mpkg_debug_gram(int n, int ncol, const float *y, double *g);
 /* Where the calling thread's later mpkg_sstep_cg calls run their outer
  * loop: MPKG_SSTEP_DEVICE_LOOP (default; the whole solve is one CUDA graph
  * launch, a conditional WHILE node deciding on the device after each

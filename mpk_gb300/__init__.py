@@ -138,6 +138,7 @@ def _declare(L):
                                 C.POINTER(Lg)]),
         "mpkg_lapjv": (I, [P, I, P]),
         "mpkg_sstep_gram": (I, [I]),
+        "mpkg_debug_gram": (I, [I, I, P, P]),
         "mpkg_sstep_loop": (I, [I]),
         "mpkg_sstep_basis": (I, [I]),
         "mpkg_sstep_debug_stall": (I, [I]),
@@ -719,6 +720,19 @@ def cg(a: Csr, b, x0=None, tol=1e-8, max_iter=10000):
 GRAM_FP64, GRAM_DF64 = 0, 1
 SSTEP_DEVICE_LOOP, SSTEP_HOST_LOOP = 0, 1
 SSTEP_BASIS_MPK, SSTEP_BASIS_STEPS = 0, 1
+
+
+def debug_gram(y: np.ndarray, gram=GRAM_FP64) -> np.ndarray:
+    """Test hook: the s-step method's Gram matrix of the columns y (ncol x n,
+    float32)."""
+    y = np.ascontiguousarray(y, dtype=np.float32)
+    g = np.zeros((len(y), len(y)))
+    _check(lib().mpkg_sstep_gram(gram))
+    try:
+        _check(lib().mpkg_debug_gram(y.shape[1], len(y), _ptr(y), _ptr(g)))
+    finally:
+        _check(lib().mpkg_sstep_gram(GRAM_FP64))
+    return g
 
 
 def sstep_cg(a: Csr, b, s=8, shifts=None, scale=None, x0=None, tol=1e-8, max_outer=2000, gram=GRAM_FP64,

@@ -409,10 +409,15 @@ __global__ void __launch_bounds__(kThreads) basis_wave_kernel(BasisWave w, Sell 
 // distributions together, at 1 K / 30 K / 262 K / 885 K rows 4.6e-17 /
 // 5.0e-17 / 5.9e-17 / 5.5e-17 against 5.5e-17 / 5.2e-17 / 8.1e-17 / 2.8e-16.
 // A tile's columns are scaled by powers of two to a largest value in [1, 2),
-// so that products and their errors stay in the FP32 range; tiles with
-// infinities or NaN are summed with FP64 fused multiply-adds.  (Unscaled, a
+// so that products and their errors stay in the FP32 range.  (Unscaled, a
 // monomial basis, whose columns shrink, left that range: 181 us an outer
-// iteration on 64^3 diffusion, 136 so.)
+// iteration on 64^3 diffusion, 136 so.)  Tiles with infinities or NaN, or with
+// a column whose nonzero values lie more than 2^38 apart, are summed with FP64
+// fused multiply-adds: within 2^38 every value is a multiple of 2^-61 of its
+// column's scale, so every product, error and sum is one of 2^-122 and none
+// is subnormal.  (A point source, whose basis decays over many orders, 64^3 to
+// 1e-9: 28 ms a solve, 30 with all tiles in FP64, 23 with none but then with
+// the low bits of small products lost.)
 // A CTA stages a tile of rows of all columns in shared memory, thread t
 // accumulates pair t of the upper triangle; per-CTA partials (FP64) are summed
 // in a fixed order by gram_reduce_kernel.
@@ -423,6 +428,7 @@ __global__ void __launch_bounds__(kThreads) basis_wave_kernel(BasisWave w, Sell 
 // sums (10 instructions) 30 and 86 us, but 5 times further off.
 constexpr int kGramRows = 64;  // two per lane of the warp that stages a column
 constexpr int kGramStride = kGramRows + 4;  // 16-byte rows, eight columns in different banks
+constexpr int kGramWide = kGramRows + 1;
 thread_local bool g_gram_f64 = true;  // mpkg_sstep_gram: FP64 (default) or double-float Gram
 thread_local bool g_device_loop = true;  // mpkg_sstep_loop: device-side (default) or host-side outer loop
 thread_local bool g_basis_mpk = false;   // mpkg_sstep_basis: s launches (default) or one matrix powers launch
@@ -468,6 +474,7 @@ __global__ void __launch_bounds__(kThreads) gram_kernel(int n, int ncol, const f
                                                         double *__restrict__ part) {
   __shared__ __align__(16) float tile[kMaxCols * kGramStride];
   __shared__ int s_exp[kMaxCols];  // F64: the tile's columns are scaled by 2^-s_exp
+  __shared__ double wtile[F64 ? kMaxCols * kGramWide : 1];  // ... and, for FP64 sums, widened
   const int npair = ncol * (ncol + 1) / 2;
   int pa = 0, pb = 0;
   {
@@ -486,39 +493,56 @@ __global__ void __launch_bounds__(kThreads) gram_kernel(int n, int ncol, const f
     int wide = 0;
     for (int c = threadIdx.x >> 5; c < ncol; c += blockDim.x >> 5) {  // a warp per column
       float v[2];
-      unsigned int top = 0;
+      unsigned int top = 0, low = 0xFFFFFFFFu;  // largest and smallest magnitude (not zero)
 #pragma unroll
       for (int q = 0; q < 2; q++) {
         const long i = r0 + lane + 32 * q;
         v[q] = i < n ? y[(size_t)c * n + i] : 0.f;
-        top = max(top, __float_as_uint(v[q]) & 0x7FFFFFFFu);
+        const unsigned int u = __float_as_uint(v[q]) & 0x7FFFFFFFu;
+        top = max(top, u);
+        low = min(low, u - 1u);  // zero goes to the top
       }
       float up = 1.f;
       if (F64) {
         top = __reduce_max_sync(0xFFFFFFFFu, top);
+        low = __reduce_min_sync(0xFFFFFFFFu, low) + 1u;
         int e = (int)(top >> 23), sub = 0;
-        if (e == 0 && top != 0) {  // subnormal
+        if (e == 0 && top != 0) {  // subnormal, all of them
           sub = 64;
           v[0] *= 0x1p64f;
           v[1] *= 0x1p64f;
           e = (int)(__float_as_uint(__uint_as_float(top) * 0x1p64f) >> 23);
         }
-        wide |= e == 255;
-        if (e > 0 && e < 255) up = __uint_as_float(e < 254 ? (unsigned)(254 - e) << 23 : 1u << 22);  // 2^(127 - e)
-        if (lane == 0) s_exp[c] = e > 0 && e < 255 ? e - 127 - sub : 0;
+        // a subnormal beside others counts as the smallest there is
+        const bool far = e == 255 || (sub == 0 && e > 0 && e - (low >> 23 ? (int)(low >> 23) : -22) > 38);
+        wide |= far;
+        const bool scaled = e > 0 && !far;
+        if (scaled) up = __uint_as_float(e < 254 ? (unsigned)(254 - e) << 23 : 1u << 22);  // 2^(127 - e)
+        if (lane == 0) s_exp[c] = scaled ? e - 127 - sub : 0;
       }
       tile[c * kGramStride + lane] = v[0] * up;
       tile[c * kGramStride + lane + 32] = v[1] * up;
     }
     if (F64) wide = __syncthreads_or(wide);
     else __syncthreads();
+    if (F64 && wide) {  // each value converted once
+      for (int q = threadIdx.x; q < ncol * kGramRows; q += blockDim.x) {
+        const float f = tile[q / kGramRows * kGramStride + q % kGramRows];
+        const unsigned int u = __float_as_uint(f) & 0x7FFFFFFFu;
+        wtile[q / kGramRows * kGramWide + q % kGramRows] = u - 1u < 0x7FFFFFu ? (double)f : ss_widen(f);
+      }
+      __syncthreads();
+    }
     if ((int)threadIdx.x >= npair) continue;
     const int k = F64 ? s_exp[pa] + s_exp[pb] : 0;
     if (F64 && wide) {
-      double t = 0.0;
-      for (int rr = 0; rr < kGramRows; rr++)
-        t = fma((double)tile[pa * kGramStride + rr], (double)tile[pb * kGramStride + rr], t);
-      acc += scalbn(t, k);
+      const double *wa = wtile + pa * kGramWide, *wb = wtile + pb * kGramWide;
+      double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+      for (int rr = 0; rr < kGramRows; rr += 4)
+#pragma unroll
+        for (int q = 0; q < 4; q++) t[q] = fma(wa[rr + q], wb[rr + q], t[q]);
+      acc += scalbn((t[0] + t[1]) + (t[2] + t[3]), k);
       continue;
     }
     if (F64) {
@@ -568,6 +592,16 @@ __global__ void gram_reduce_kernel(int nblk, int ncol, const double *__restrict_
     g[a * ncol + a + u] = s;
     g[(a + u) * ncol + a] = s;
   }
+}
+
+int gram_blocks(int n) { return (int)std::min<long>(1216, ((long)n + kGramRows - 1) / kGramRows); }
+
+// G (ncol x ncol) of the basis y; part: gram_blocks(n) sums for each pair.
+void launch_gram(int n, int ncol, const float *y, double *part, double *g, cudaStream_t cs) {
+  const int npair = ncol * (ncol + 1) / 2, thr = (npair + 31) / 32 * 32, gblk = gram_blocks(n);
+  if (g_gram_f64) gram_kernel<true><<<gblk, thr, 0, cs>>>(n, ncol, y, part);
+  else gram_kernel<false><<<gblk, thr, 0, cs>>>(n, ncol, y, part);
+  gram_reduce_kernel<<<(npair * 32 + kThreads - 1) / kThreads, kThreads, 0, cs>>>(gblk, ncol, part, g);
 }
 
 // The s inner CG steps in coefficient space (FP64, one warp; lane c holds
@@ -1225,6 +1259,22 @@ int mpkg_sstep_gram(int mode) {
   return kOk;
 }
 
+int mpkg_debug_gram(int n, int ncol, const float *y, double *g) {
+  clear_error();
+  if (n <= 0 || ncol <= 0 || ncol > kMaxCols || !y || !g) return fail(kEInval, "bad argument");
+  const int npair = ncol * (ncol + 1) / 2, gblk = gram_blocks(n);
+  DevBuf<float> dy;
+  DevBuf<double> part, dg;
+  int rc;
+  if ((rc = dy.alloc((size_t)n * ncol)) || (rc = part.alloc((size_t)gblk * npair)) || (rc = dg.alloc(ncol * ncol)))
+    return rc;
+  SS_TRY(cudaMemcpy(dy.p, y, sizeof(float) * (size_t)n * ncol, cudaMemcpyHostToDevice));
+  launch_gram(n, ncol, dy.p, part.p, dg.p, 0);
+  SS_TRY(cudaGetLastError());
+  SS_TRY(cudaMemcpy(g, dg.p, sizeof(double) * ncol * ncol, cudaMemcpyDeviceToHost));
+  return kOk;
+}
+
 int mpkg_sstep_basis(int mode) {
   if (mode != MPKG_SSTEP_BASIS_MPK && mode != MPKG_SSTEP_BASIS_STEPS) return fail(kEInval, "unknown basis mode");
   g_basis_mpk = mode == MPKG_SSTEP_BASIS_MPK;
@@ -1254,7 +1304,7 @@ int mpkg_sstep_cg(int n, const int *ptr, const int *col, const double *val, cons
   int rc = a.upload(n, ptr, col, val, true);
   if (rc) return rc;
   const int nb = blocks_for(n), m = 2 * s + 1, npair = m * (m + 1) / 2;
-  const int gblk = (int)std::min<long>(1216, (n + kGramRows - 1) / kGramRows);
+  const int gblk = gram_blocks(n);
   DevBuf<double> dx, db, dr, dp, part, gpart, dg, dth, dsg, dxh, dph, drh;
   DevBuf<float> y;
   DevBuf<int> dflag;
@@ -1315,10 +1365,7 @@ int mpkg_sstep_cg(int n, const int *ptr, const int *col, const double *val, cons
                                                  rstep ? Y + (size_t)(s + 2 + j) * n : nullptr, (float)th[j],
                                                  (float)(1.0 / sg[j]));
     }
-    const int gthr = (npair + 31) / 32 * 32;
-    if (g_gram_f64) gram_kernel<true><<<gblk, gthr, 0, cs>>>(n, m, Y, gpart.p);
-    else gram_kernel<false><<<gblk, gthr, 0, cs>>>(n, m, Y, gpart.p);
-    gram_reduce_kernel<<<(npair * 32 + kThreads - 1) / kThreads, kThreads, 0, cs>>>(gblk, m, gpart.p, dg.p);
+    launch_gram(n, m, Y, gpart.p, dg.p, cs);
     coeff_kernel<<<1, 32, 0, cs>>>(s, dg.p, dth.p, dsg.p, dsc.p, dxh.p, dph.p, drh.p, dflag.p);
     combine_kernel<<<nb, kThreads, 0, cs>>>(n, m, Y, dxh.p, dph.p, dx.p, dp.p, part.p + nb);
     resid_kernel<<<nb, kThreads, 0, cs>>>(n, a.sell(), dx.p, db.p, dr.p, part.p);
