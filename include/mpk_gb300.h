@@ -169,7 +169,10 @@ int mpkg_plan_wave_ctas(int n, const int *ptr, const int *col, const double *val
  * windows reach three quarters of the entries, else the CSR kernel;
  * MPKG_BATCH_STAGED / MPKG_BATCH_STAGED2 / MPKG_BATCH_STAGED4 the staged
  * kernel at one, two or four CTAs per SM untimed (EINVAL when nrhs is not a
- * multiple of 4).  All configurations give the same bits. */
+ * multiple of 4).  All configurations give the same bits.  The packed matrix
+ * is made on the host, for this set of matrices, as part of the plan: with 16
+ * cores 0.6 ms of 2.3 for 170 thousand entries, 15 ms of 40 for 4.8 million
+ * (the rest a plan of the CSR kernel takes too). */
 enum {
   MPKG_BATCH_DEFAULT = 0,
   MPKG_BATCH_TUNE = 1,

@@ -2198,10 +2198,12 @@ int check_csr(int n, const int *ptr, const int *col) {
   if (n <= 0 || !ptr || !col) return fail(kEInval, "empty matrix or null arrays");
   if (ptr[0] != 0) return fail(kEInval, "ptr[0] must be 0");
   if (ptr[n] <= 0) return fail(kEInval, "the matrix has no entries");
-  for (int i = 0; i < n; i++)
-    if (ptr[i + 1] < ptr[i]) return fail(kEInval, "ptr must be non-decreasing");
-  for (long j = 0; j < ptr[n]; j++)
-    if (col[j] < 0 || col[j] >= n) return fail(kERange, "column index out of range");
+  int bad = 0;  // no exit from the loops: they vectorise
+  for (int i = 0; i < n; i++) bad |= ptr[i + 1] < ptr[i];
+  if (bad) return fail(kEInval, "ptr must be non-decreasing");
+  const long nnz = ptr[n];
+  for (long j = 0; j < nnz; j++) bad |= (unsigned)col[j] >= (unsigned)n;
+  if (bad) return fail(kERange, "column index out of range");
   return kOk;
 }
 
@@ -2490,30 +2492,6 @@ struct BatchLayout {
   bool resident = false; // every unit's streams have room beside its window
 };
 
-// Runs fn(0..count-1) on all host threads, the caller's among them; false
-// when a call threw (out of memory).
-template <typename F>
-bool host_parallel(int count, F &&fn) {
-  const int nth = (int)std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-  std::atomic<int> next{0};
-  std::atomic<bool> ok{true};
-  auto work = [&] {
-    try {
-      for (int q; ok && (q = next.fetch_add(1)) < count;) fn(q);
-    } catch (const std::exception &) {
-      ok = false;
-    }
-  };
-  std::vector<std::thread> pool;
-  try {
-    for (int t = 1; t < nth && t < count; t++) pool.emplace_back(work);
-  } catch (const std::exception &) {  // no more threads: the caller's thread does the rest
-  }
-  work();
-  for (auto &th : pool) th.join();
-  return ok;
-}
-
 // Groups of consecutive matrices within `budget` bytes (matrix + two
 // levels of vectors); per group, CTA row ranges of equal nonzeros and the
 // CTAs owning each range's columns.
@@ -2601,10 +2579,13 @@ int batch_ranges(const BatchHost &h, int nrhs, long budget, bool windows, int gr
   // the exact set of other CTAs whose rows CTA b reads (its own rows of
   // the previous level are ordered by its barrier)
   std::vector<std::vector<int>> dep((size_t)ng * grid);
-  const bool ok = host_parallel(ng, [&](int g) {
+  const int part = 16;  // CTAs a task
+  const int per_group = (grid + part - 1) / part;
+  const bool ok = host_parallel(ng * per_group, (long)h.col.size(), 50000, [&](int t) {
+    const int g = t / per_group, b0 = t % per_group * part;
     const int *lo = out->row_lo.data() + (size_t)g * (grid + 1);
     std::vector<int> seen(grid, -1);
-    for (int b = 0; b < grid; b++) {
+    for (int b = b0; b < std::min(grid, b0 + part); b++) {
       std::vector<int> &d = dep[(size_t)g * grid + b];
       for (long q = h.ptr[lo[b]]; q < h.ptr[lo[b + 1]]; q++) {
         const int c = h.col[q];
@@ -2632,13 +2613,27 @@ int batch_ranges(const BatchHost &h, int nrhs, long budget, bool windows, int gr
 // the rows do not fit, the intervals nearest the CTA's own rows are kept and
 // the entries of the others read global memory.
 struct RowSpan { int lo, hi; };  // rows [lo, hi)
-void batch_window(const BatchHost &h, int r0, int r1, long cap_rows, std::vector<int> *cols, std::vector<RowSpan> *win) {
+void batch_window(const BatchHost &h, int r0, int r1, long cap_rows, std::vector<int> *cols, std::vector<char> *marks,
+                  std::vector<RowSpan> *win) {
   cols->clear();
   win->clear();
-  for (long q = h.ptr[r0]; q < h.ptr[r1]; q++) cols->push_back(h.col[q]);
-  if (cols->empty()) return;
-  std::sort(cols->begin(), cols->end());
-  cols->erase(std::unique(cols->begin(), cols->end()), cols->end());
+  const long q0 = h.ptr[r0], q1 = h.ptr[r1];
+  if (q0 == q1) return;
+  int lo = h.col[q0], hi = lo;  // the distinct columns: marked where they lie close, else sorted
+  for (long q = q0; q < q1; q++) {
+    lo = std::min(lo, h.col[q]);
+    hi = std::max(hi, h.col[q]);
+  }
+  if ((long)hi - lo < 16 * (q1 - q0)) {
+    marks->assign((size_t)hi - lo + 1, 0);
+    for (long q = q0; q < q1; q++) (*marks)[h.col[q] - lo] = 1;
+    for (int c = lo; c <= hi; c++)
+      if ((*marks)[c - lo]) cols->push_back(c);
+  } else {
+    cols->assign(h.col.begin() + q0, h.col.begin() + q1);
+    std::sort(cols->begin(), cols->end());
+    cols->erase(std::unique(cols->begin(), cols->end()), cols->end());
+  }
   for (int gap : {32, 0}) {
     win->clear();
     long rows = 0;
@@ -2698,8 +2693,11 @@ void batch_window(const BatchHost &h, int r0, int r1, long cap_rows, std::vector
 // The packed form of a layout for CTAs of `threads` threads and `smem` bytes
 // of shared memory: windows, slices of rows sorted by length, and the units'
 // blobs (batch_pack_kernel).  `resident`: the resident form; out->resident
-// tells whether it fits (if not, the layout is not complete).
-int batch_pack(const BatchHost &h, int grid, int lpr, int threads, long smem, bool resident, BatchLayout *out) {
+// tells whether it fits (if not, the layout is not complete).  With more than
+// far_limit entries outside their windows the layout is not completed either;
+// out->far is above the limit then.
+int batch_pack(const BatchHost &h, int grid, int lpr, int threads, long smem, bool resident, long far_limit,
+               BatchLayout *out) {
   const int ng = out->ngroup, rps = 32 / lpr, nw = threads / 32;
   const size_t nu = (size_t)ng * grid;
   const long row_bytes = (long)lpr * 16;
@@ -2720,8 +2718,10 @@ int batch_pack(const BatchHost &h, int grid, int lpr, int threads, long smem, bo
   auto pairs_of_row = [&](int i) { return (h.ptr[i + 1] - h.ptr[i] + 1) / 2; };
   auto pairs_of = [&](const Unit &x, int sl) { return pairs_of_row(x.rows[(size_t)sl * rps]); };
   std::atomic<bool> fits{true};
-  bool ok = host_parallel(ntask, [&](int t) {
-    std::vector<int> cols, sorted;
+  std::atomic<long> far{0};
+  bool ok = host_parallel(ntask, (long)h.col.size(), 20000, [&](int t) {
+    std::vector<int> cols, sorted, first;
+    std::vector<char> marks;
     std::vector<RowSpan> win;
     std::vector<int4> ivs;
     for (size_t u = (size_t)t * chunk; u < std::min(nu, (size_t)(t + 1) * chunk); u++) {
@@ -2736,7 +2736,7 @@ int batch_pack(const BatchHost &h, int grid, int lpr, int threads, long smem, bo
       d.head = (int)head;
       d.staged = resident || head <= (smem - base) / 4 ? (int)head : 0;
       long pos = base;
-      batch_window(h, r0, r1, std::max(0L, (smem - base - d.staged) / row_bytes), &cols, &win);
+      batch_window(h, r0, r1, std::max(0L, (smem - base - d.staged) / row_bytes), &cols, &marks, &win);
       auto add = [&](int a, int z) {
         if (a >= z) return;
         x.iv.push_back(make_int4(a, z - a, (int)pos, 0));
@@ -2753,39 +2753,57 @@ int batch_pack(const BatchHost &h, int grid, int lpr, int threads, long smem, bo
       std::sort(ivs.begin(), ivs.end(), [](const int4 &p, const int4 &q) { return p.x < q.x; });
       const long q0 = h.ptr[r0];
       x.off.resize(h.ptr[r1] - q0);
+      const int4 *v = nullptr;  // interval of the last column
       for (size_t q = 0; q < x.off.size(); q++) {
         const int c = h.col[q0 + q];
-        auto v = std::upper_bound(ivs.begin(), ivs.end(), c, [](int cc, const int4 &z) { return cc < z.x; });
-        if (v != ivs.begin() && c < v[-1].x + v[-1].y) {
-          x.off[q] = (unsigned)(v[-1].z + (c - v[-1].x) * row_bytes);
+        if (!v || c < v->x || c >= v->x + v->y) {
+          auto n = std::upper_bound(ivs.begin(), ivs.end(), c, [](int cc, const int4 &z) { return cc < z.x; });
+          v = n != ivs.begin() && c < n[-1].x + n[-1].y ? &n[-1] : nullptr;
+        }
+        if (v) {
+          x.off[q] = (unsigned)(v->z + (c - v->x) * row_bytes);
         } else {
           x.off[q] = 0x80000000u | (unsigned)c;
           x.far++;
         }
       }
-      sorted.resize(r1 - r0);
-      for (int i = r0; i < r1; i++) sorted[i - r0] = i;
-      std::stable_sort(sorted.begin(), sorted.end(),
-                       [&](int i, int j) { return h.ptr[i + 1] - h.ptr[i] > h.ptr[j + 1] - h.ptr[j]; });
+      if ((far += x.far) > far_limit) {
+        fits = false;
+        return;
+      }
+      sorted.resize(r1 - r0);  // longest first, in order within a length
+      int longest = 0;
+      for (int i = r0; i < r1; i++) longest = std::max(longest, h.ptr[i + 1] - h.ptr[i]);
+      if (longest <= 4096) {
+        first.assign(longest + 2, 0);
+        for (int i = r0; i < r1; i++) first[longest - (h.ptr[i + 1] - h.ptr[i]) + 1]++;
+        for (int k = 0; k <= longest; k++) first[k + 1] += first[k];
+        for (int i = r0; i < r1; i++) sorted[first[longest - (h.ptr[i + 1] - h.ptr[i])]++] = i;
+      } else {
+        for (int i = r0; i < r1; i++) sorted[i - r0] = i;
+        std::stable_sort(sorted.begin(), sorted.end(),
+                         [&](int i, int j) { return h.ptr[i + 1] - h.ptr[i] > h.ptr[j + 1] - h.ptr[j]; });
+      }
       // a quarter warp reads `quad` rows at once, 128 bytes when they lie in
       // different banks: of the next rows of the same length, each place
       // takes the one whose entries meet the fewest of the places before it
       const int quad = std::max(1, 8 / lpr);
+      const unsigned banks = (unsigned)(16 * 8 - 16 * lpr) & 0x70u;
       auto meets = [&](int i, int j) {
         const unsigned *p = x.off.data() + (h.ptr[i] - q0), *q = x.off.data() + (h.ptr[j] - q0);
         const int len = std::min(h.ptr[i + 1] - h.ptr[i], h.ptr[j + 1] - h.ptr[j]);
         int m = 0;
-        for (int e = 0; e < len; e++) m += p[e] != q[e] && ((p[e] ^ q[e]) & (unsigned)(16 * 8 - 16 * lpr) & 0x70u) == 0;
+        for (int e = 0; e < len; e++) m += (int)(p[e] != q[e]) & (int)(((p[e] ^ q[e]) & banks) == 0);
         return m;
       };
       for (size_t k = 0; quad > 1 && k < sorted.size(); k++) {
-        const size_t first = k - k % quad;
-        if (k == first) continue;
+        const size_t begin = k - k % quad;
+        if (k == begin) continue;
         size_t best = k;
         int least = INT32_MAX;
         for (size_t z = k; z < std::min(sorted.size(), k + 16) && pairs_of_row(sorted[z]) == pairs_of_row(sorted[k]); z++) {
           int m = 0;
-          for (size_t y = first; y < k; y++) m += meets(sorted[y], sorted[z]);
+          for (size_t y = begin; y < k && m < least; y++) m += meets(sorted[y], sorted[z]);
           if (m < least) {
             least = m;
             best = z;
@@ -2819,7 +2837,8 @@ int batch_pack(const BatchHost &h, int grid, int lpr, int threads, long smem, bo
     }
   });
   out->resident = resident && fits;
-  if (ok && resident && !fits) return kOk;
+  out->far = far;
+  if (ok && !fits) return kOk;
   if (!ok) return fail(kENoMem, "batch layout");
   long total = 0;  // 16-byte words of all blobs
   out->iv.clear();
@@ -2838,7 +2857,7 @@ int batch_pack(const BatchHost &h, int grid, int lpr, int threads, long smem, bo
   out->blob_words = (size_t)std::max(1L, total);
   out->blob.reset(new (std::nothrow) uint4[out->blob_words]);
   if (!out->blob) return fail(kENoMem, "batch layout");
-  ok = host_parallel(ntask, [&](int t) {
+  ok = host_parallel(ntask, (long)h.col.size(), 100000, [&](int t) {
     for (size_t u = (size_t)t * chunk; u < std::min(nu, (size_t)(t + 1) * chunk); u++) {
       Unit &x = un[u];
       const BatchUnit &d = out->unit[u];
@@ -2880,8 +2899,6 @@ int batch_pack(const BatchHost &h, int grid, int lpr, int threads, long smem, bo
     }
   });
   if (!ok) return fail(kENoMem, "batch layout");
-  out->far = 0;
-  for (const Unit &x : un) out->far += x.far;
   return kOk;
 }
 
@@ -3572,9 +3589,7 @@ int diag_setup(mpkg_plan *p, int form, const int *ptr, const int *col, const dou
   auto upload = [&](auto zero, auto conv, auto **dst) -> int {
     using T = decltype(zero);
     std::unique_ptr<T[]> v(new (std::nothrow) T[nv]);
-    if (!v) return fail(kENoMem, "diagonal values");
-    std::fill(v.get(), v.get() + nv, zero);
-    diag_values(n, ptr, col, l, conv, v.get());
+    if (!v || !diag_values(n, ptr, col, l, zero, conv, v.get())) return fail(kENoMem, "diagonal values");
     return dev_copy(p, dst, v.get(), nv);
   };
   if (!rc && val && diag_value_bytes(form) == 8) {
@@ -3882,7 +3897,7 @@ struct BatchCand {
   size_t smem;  // shared memory per CTA
 };
 
-int batch_build_layout(const BatchHost &h, int nrhs, const BatchCand &c, BatchLayout *lay) {
+int batch_build_layout(const BatchHost &h, int nrhs, const BatchCand &c, BatchLayout *lay, long far_limit = LONG_MAX) {
   int rc = batch_ranges(h, nrhs, c.budget, c.staged, c.grid, c.threads, c.lpr, lay);
   if (rc || !c.staged) return rc;
   // the resident form where the matrix, the windows (a tenth of them halo)
@@ -3890,10 +3905,10 @@ int batch_build_layout(const BatchHost &h, int nrhs, const BatchCand &c, BatchLa
   const long need = 9L * (long)h.col.size() + h.N * (4L * nrhs * 11 / 10 + 10) +
                     (long)c.grid * (c.threads / 32) * bp_chunk_bytes(c.lpr) / 2;
   if (lay->ngroup == 1 && need < (long)(0.93 * c.grid * (double)c.smem)) {
-    rc = batch_pack(h, c.grid, c.lpr, c.threads, (long)c.smem, true, lay);
-    if (rc || lay->resident) return rc;
+    rc = batch_pack(h, c.grid, c.lpr, c.threads, (long)c.smem, true, far_limit, lay);
+    if (rc || lay->resident || lay->far > far_limit) return rc;
   }
-  return batch_pack(h, c.grid, c.lpr, c.threads, (long)c.smem, false, lay);
+  return batch_pack(h, c.grid, c.lpr, c.threads, (long)c.smem, false, far_limit, lay);
 }
 
 // The device state of a configuration, in place of the one before it.  It
@@ -3990,18 +4005,17 @@ int mpkg_plan_batch(int nmat, const int *n, const int *const *ptr, const int *co
   h.ptr.resize(h.N + 1);
   h.col.resize(nnz);
   h.val.resize(nnz);
-  long q = 0;
-  for (int m = 0; m < nmat; m++) {
+  std::vector<long> q0(nmat + 1, 0);
+  for (int m = 0; m < nmat; m++) q0[m + 1] = q0[m] + ptr[m][n[m]];
+  host_parallel(nmat, nnz, 100000, [&](int m) {
     const long r0 = h.mat_row0[m];
-    for (int i = 0; i < n[m]; i++) {
-      h.ptr[r0 + i] = (int)q;
-      for (int t = ptr[m][i]; t < ptr[m][i + 1]; t++, q++) {
-        h.col[q] = (int)(col[m][t] + r0);
-        h.val[q] = val[m][t];
-      }
+    for (int i = 0; i < n[m]; i++) h.ptr[r0 + i] = (int)(q0[m] + ptr[m][i]);
+    for (long t = 0, q = q0[m]; q < q0[m + 1]; t++, q++) {
+      h.col[q] = (int)(col[m][t] + r0);
+      h.val[q] = val[m][t];
     }
-  }
-  h.ptr[h.N] = (int)q;
+  });
+  h.ptr[h.N] = (int)nnz;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return fail(kECuda, "no CUDA device");
   mpkg_plan *p = new_plan();
@@ -4085,7 +4099,7 @@ int mpkg_plan_batch(int nmat, const int *n, const int *const *ptr, const int *co
     // batches and more on small ones); where its windows miss a fourth of the
     // columns, or it cannot be made, the CSR kernel
     if (best.staged) {
-      laid = batch_build_layout(h, nrhs, best, &lay) == kOk && 4 * lay.far <= nnz &&
+      laid = batch_build_layout(h, nrhs, best, &lay, nnz / 4) == kOk && lay.far <= nnz / 4 &&
              batch_configure(p, h, best, lay) == kOk;
       clear_error();
     }

@@ -42,8 +42,9 @@
 #include <atomic>
 #include <cstring>
 #include <map>
-#include <thread>
+#include <string>
 #include <type_traits>
+#include <unordered_map>
 #include <vector>
 
 #include "diag.cuh"
@@ -454,15 +455,6 @@ int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int
   };
   const bool near = !pair || reach <= own;
   if (!(near && consider(1, 0)) && !(pair && consider(1, 1)) && !consider(1, 0)) return kOk;  // too large
-  for (int i = 0; i < n; i++)
-    if (ptr[i + 1] - ptr[i] > 65535) return kOk;  // refused by the general wavefront
-  // patterns
-  l.pat.assign(nslice, 0);
-  std::map<std::vector<unsigned short>, int> known;
-  const unsigned short all = (unsigned short)((1 << W) - 1);
-  std::vector<unsigned short> m(32);
-  known[std::vector<unsigned short>(32, all)] = 0;
-  l.mask.assign(32, all);
   // Rows of irregular slices run one entry after another, from the CSR, where
   // the general wavefront has 8 entries in flight.  That costs 350 cycles an
   // entry for these 8 (double-float 650, and 250 for each further one, which
@@ -478,55 +470,88 @@ int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int
   // double-float 110^3 212 / 116 / 116, 188 / 924 / 188, 197 / 295 / 197.
   const double spare = fp64 ? std::max(std::min(8000.0, 1900 + 130.0 * ns_max), 0.25 * per_slice * ns_max)
                             : std::max(std::min(12000.0, 2500 + 200.0 * ns_max), 0.45 * per_slice * ns_max);
-  int cta = 0;
-  long loads = 0, worst = 0;  // of CTA `cta`, of all
-  bool wide = false;
-  long &irregular = l.irregular = 0;
-  for (int sl = 0; sl < nslice; sl++) {
-    bool ok = true;
-    std::fill(m.begin(), m.end(), 0);
-    bool full = sl * 32 + 32 <= n;
-    for (int i = sl * 32; i < std::min(n, sl * 32 + 32) && ok; i++) {
-      int u = 0;
-      unsigned bits = 0;
-      for (int q = ptr[i]; q < ptr[i + 1]; q++) {
-        while (u < W && l.d[u] != col[q] - i) u++;
-        if (u == W) { ok = false; break; }
-        bits |= 1u << u++;
+  // every CTA's rows, on all host threads: the diagonals of each row, the
+  // slices off them, the CTAs whose rows they read
+  constexpr unsigned short kPartly = 1;  // for now: a slice that lacks some diagonals
+  const unsigned short all = (unsigned short)((1 << W) - 1);
+  std::vector<unsigned short> bits(n);
+  l.pat.assign(nslice, 0);
+  std::vector<std::vector<int>> waits(grid);
+  auto owner = [&](int c) {
+    int b = (int)((long)(c / 32) * grid / nslice);
+    while (l.lo[b + 1] <= c) b++;
+    while (l.lo[b] > c) b--;
+    return b;
+  };
+  std::atomic<long> irregular{0}, worst{0};
+  std::atomic<bool> wide{false}, refused{false};
+  const bool scanned = host_parallel(grid, ptr[n], 50000, [&](int b) {
+    const int r0 = l.lo[b], r1 = l.lo[b + 1];
+    std::vector<char> seen(grid, 0);
+    long loads = 0;
+    for (int sl = r0 / 32; sl * 32 < r1 && !refused; sl++) {
+      const int end = std::min(r1, sl * 32 + 32);
+      bool ok = true, full = sl * 32 + 32 <= n;
+      for (int i = sl * 32; i < end; i++) {
+        if (ptr[i + 1] - ptr[i] > 65535) refused = true;  // by the general wavefront
+        int u = 0;
+        unsigned m = 0;
+        for (int q = ptr[i]; q < ptr[i + 1]; q++) {
+          const int c = col[q];
+          if (c < r0 || c >= r1) {
+            const int o = owner(c);
+            if (!seen[o]) {
+              seen[o] = 1;
+              waits[b].push_back(o);
+            }
+          }
+          while (u < W && l.d[u] != c - i) u++;
+          if (u < W) m |= 1u << u++;
+          else ok = false;
+        }
+        bits[i] = (unsigned short)m;
+        full &= m == all;
       }
-      m[i & 31] = (unsigned short)bits;
-      full &= bits == all;
-    }
-    if (!ok) {
+      if (ok) {
+        l.pat[sl] = full ? 0 : kPartly;
+        continue;
+      }
       l.pat[sl] = kDiagIrregular;
-      if (++irregular * 20 > nslice) return kOk;
-      while (l.lo[cta + 1] <= sl * 32) {
-        cta++;
-        loads = 0;
-      }
-      for (int i = sl * 32; i < std::min(n, sl * 32 + 32); i++) {
+      if (20 * ++irregular > nslice) refused = true;
+      for (int i = sl * 32; i < end; i++) {
         const int len = ptr[i + 1] - ptr[i], ahead = std::min(len, 8);
         loads += ahead;
         for (int q = ptr[i]; q < ptr[i + 1]; q++) {
-          if (q < ptr[i] + ahead && (col[q] < l.lo[cta] - l.halo || col[q] >= l.lo[cta + 1] + l.halo)) loads += 5;
-          wide |= std::abs(col[q] - i) > 32767;
+          if (q < ptr[i] + ahead && (col[q] < r0 - l.halo || col[q] >= r1 + l.halo)) loads += 5;
+          if (std::abs(col[q] - i) > 32767) wide = true;
         }
-        worst = std::max({worst, loads, ahead * (ring ? 650L : 350L) + (ring ? (len - ahead) * 250L : 0L)});
+        const long cost = std::max(loads, ahead * (ring ? 650L : 350L) + (ring ? (len - ahead) * 250L : 0L));
+        for (long w = worst; cost > w && !worst.compare_exchange_weak(w, cost);) {
+        }
       }
-      continue;
     }
-    if (full) continue;
-    const auto f = known.find(m);
-    if (f != known.end()) {
-      l.pat[sl] = (unsigned short)f->second;
-      continue;
-    }
-    if (known.size() == kDiagIrregular) return kOk;
-    l.pat[sl] = (unsigned short)known.size();
-    known[m] = l.pat[sl];
-    l.mask.insert(l.mask.end(), m.begin(), m.end());
-  }
+  });
+  if (!scanned) return fail(kENoMem, "diagonal layout");
+  l.irregular = irregular;
+  if (refused) return kOk;
   if (worst > (wide ? 1.6 : 1.0) * spare) return kOk;
+  // patterns
+  std::unordered_map<std::string, int> known;
+  std::string m(64, 0);
+  l.mask.assign(32, all);
+  for (int sl = 0; sl < nslice; sl++) {
+    if (l.pat[sl] != kPartly) continue;
+    const int rows = std::min(32, n - sl * 32);
+    std::fill(m.begin(), m.end(), 0);
+    std::memcpy(&m[0], &bits[(size_t)sl * 32], 2 * rows);
+    const auto f = known.emplace(m, (int)known.size() + 1);
+    if (f.first->second >= kDiagIrregular) return kOk;
+    l.pat[sl] = (unsigned short)f.first->second;
+    if (f.second) {
+      l.mask.resize(l.mask.size() + 32, 0);
+      std::memcpy(&l.mask[l.mask.size() - 32], m.data(), 64);
+    }
+  }
   if (!irregular)  // more levels per exchange
     for (int depth = 2; depth <= std::min(nlevel, kDiagMaxDepth) && consider(depth, 0); depth++) {
     }
@@ -534,8 +559,6 @@ int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int
   l.own.assign(grid, make_int2(0, 0));
   l.nres.assign(grid, 0);
   long used = 0;  // bytes below the windows
-  std::vector<std::vector<int>> waits(grid);
-  auto owner = [&](int c) { return (int)(std::upper_bound(l.lo.begin(), l.lo.end() - 1, c) - l.lo.begin()) - 1; };
   for (int b = 0; b < grid; b++) {
     const int r0 = l.lo[b], r1 = l.lo[b + 1], ns = (r1 - r0 + 31) / 32;
     const int reach_lo = std::max(0, -l.d[0]), reach_hi = std::max(0, l.d[W - 1]);
@@ -555,14 +578,6 @@ int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int
     if (vb) l.nres[b] = (int)std::min<long>(all, room / (vb * W * 32));
     used = std::max(used, pats + l.nres[b] * vb * W * 32);
     std::vector<int> &wt = waits[b];
-    int last = -1;
-    for (int q = ptr[r0]; q < ptr[r1]; q++) {
-      const int c = col[q];
-      if (c >= r0 && c < r1) continue;
-      if (last >= 0 && c >= l.lo[last] && c < l.lo[last + 1]) continue;
-      last = owner(c);
-      wt.push_back(last);
-    }
     if (l.depth > 1)  // the rows of the halo
       for (const int end : {0, 1}) {
         const int c0 = end ? r1 : std::max(0, r0 - l.halo), c1 = end ? std::min(n, r1 + l.halo) : r0;

@@ -8,6 +8,8 @@
 #include <memory>
 #include <vector>
 
+#include "host.h"
+
 namespace mpkg {
 
 // Arithmetic of the rows.
@@ -80,18 +82,25 @@ struct DiagLayout {
 int diag_layout(int n, const int *ptr, const int *col, int nlevel, int form, int nsm, int smem, DiagLayout *out);
 
 // Values along the layout's diagonals, [slice][diagonal][lane], zero where a
-// row has no entry (and in irregular slices): conv(entry) in type T.
+// row has no entry (and in irregular slices): conv(entry) in type T.  False
+// for want of memory.
 template <typename T, typename F>
-void diag_values(int n, const int *ptr, const int *col, const DiagLayout &l, F &&conv, T *out) {
-  for (int i = 0; i < n; i++) {
-    T *o = out + ((size_t)(i / 32) * l.w * 32 + i % 32);
-    if (l.pat[i / 32] == kDiagIrregular) continue;
-    int u = 0;
-    for (int q = ptr[i]; q < ptr[i + 1]; q++) {
-      while (l.d[u] != col[q] - i) u++;
-      o[32 * u] = conv(q);
+bool diag_values(int n, const int *ptr, const int *col, const DiagLayout &l, T zero, F &&conv, T *out) {
+  const int ns = (int)l.pat.size(), part = 256;  // slices a task
+  return host_parallel((ns + part - 1) / part, ptr[n], 50000, [&](int t) {
+    for (int sl = t * part; sl < std::min(ns, (t + 1) * part); sl++) {
+      T *o = out + (size_t)sl * l.w * 32;
+      std::fill(o, o + (size_t)l.w * 32, zero);
+      if (l.pat[sl] == kDiagIrregular) continue;
+      for (int i = sl * 32; i < std::min(n, sl * 32 + 32); i++) {
+        int u = 0;
+        for (int q = ptr[i]; q < ptr[i + 1]; q++) {
+          while (l.d[u] != col[q] - i) u++;
+          o[32 * u + i % 32] = conv(q);
+        }
+      }
     }
-  }
+  });
 }
 
 const void *diag_kernel_ptr(int form, int w, int mode);

@@ -3,8 +3,12 @@
 // CUDA side (device.cu) consumes the plans built here.
 #pragma once
 
+#include <algorithm>
+#include <atomic>
 #include <cstdint>
+#include <exception>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/pdmpk_gb300.h"
@@ -28,6 +32,31 @@ enum Status : int {
 int fail(int code, const std::string &msg);
 const char *last_error();
 void clear_error();
+
+// Runs fn(0..count-1) on host threads, the caller's among them, one more for
+// every `grain` of `work` (some 100 us of it pay for a thread); false when a
+// call threw (out of memory).
+template <typename F>
+bool host_parallel(int count, long work, long grain, F &&fn) {
+  const long most = std::min<long>(std::max(1u, std::min(16u, std::thread::hardware_concurrency())), 1 + work / grain);
+  std::atomic<int> next{0};
+  std::atomic<bool> ok{true};
+  auto run = [&] {
+    try {
+      for (int q; ok && (q = next.fetch_add(1)) < count;) fn(q);
+    } catch (const std::exception &) {
+      ok = false;
+    }
+  };
+  std::vector<std::thread> pool;
+  try {
+    for (long t = 1; t < most && t < count; t++) pool.emplace_back(run);
+  } catch (const std::exception &) {  // no more threads: the caller's thread does the rest
+  }
+  run();
+  for (auto &th : pool) th.join();
+  return ok;
+}
 
 // Compressed sparse rows, 0-based, int32 indices (the reference's crs0_t
 // plus optional values).
