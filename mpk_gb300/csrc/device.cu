@@ -1847,7 +1847,6 @@ __global__ void __launch_bounds__(1024) batch_pack_kernel(BatchArgs a) {
 #pragma unroll
     for (int c = 0; c < kBpRing; c++) fetch(c, c);
     for (int l = 1; l <= a.nlevel; l++) {
-      const float *src = a.vb + (size_t)(l - 1) * a.N * nrhs;
       if (l > 1) {  // the CTAs owning this range's columns have published level l-1 of group g
         for (int k = dlo + (int)threadIdx.x; k < dhi; k += blockDim.x) {
           const int c = a.dep_idx[k];
@@ -1868,13 +1867,14 @@ __global__ void __launch_bounds__(1024) batch_pack_kernel(BatchArgs a) {
           // complete it
           if (un.iv1 > un.iv0) {
             if (warp == 0)
-              for (int k = un.ivh + lane; k < un.iv1; k += 32) copy(src, a.iv[k]);
+              for (int k = un.ivh + lane; k < un.iv1; k += 32) copy(a.vb + (size_t)(l - 1) * a.N * nrhs, a.iv[k]);
             tr_wait(&s_bar_w, phase_w, a.err);
           }
           cp_async_wait_all();
           return;
         }
       }
+      const float *src = a.vb + (size_t)(l - 1) * a.N * nrhs;
       if (un.iv1 > un.iv0) {
         if (warp == 0) {
           // the CTA's reads of the window and the acquired rows come before
