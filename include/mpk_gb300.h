@@ -225,10 +225,11 @@ typedef struct {
 int mpkg_cg(int n, const int *ptr, const int *col, const double *val, const double *b, double *x, double tol,
             int max_iter, mpkg_cg_info_t *info);
 /* Accumulation of the s-step Gram matrix for the calling thread's later
- * mpkg_sstep_cg calls: MPKG_GRAM_FP64 (default; FP64 FMAs over the exact
- * FP64 products of the FP32 basis) or MPKG_GRAM_DF64 (the same products
- * split exactly and summed in double-float on the FP32 pipes, about
- * 2^-46 relative to the sum of |products|; faster on GB300). */
+ * mpkg_sstep_cg calls: MPKG_GRAM_FP64 (default; FP64 sums of the exact
+ * products of the FP32 basis, 64 rows at a time from FP32 sums that keep the
+ * errors of every addition) or MPKG_GRAM_DF64 (the same products split
+ * exactly and summed in double-float on the FP32 pipes, about 2^-46 relative
+ * to the sum of |products|; faster on GB300). */
 #define MPKG_GRAM_FP64 0
 #define MPKG_GRAM_DF64 1
 int mpkg_sstep_gram(int mode);

@@ -1777,11 +1777,11 @@ __global__ void __launch_bounds__(256, VW == 4 ? 6 : 8) batch_kernel(BatchArgs a
 // the entry words, 8 for the vector rows (more where two rows of a quarter
 // warp meet in their banks, which the plan keeps rare) and 1 for the copy in.
 // 48 matrices (stencils and random banded, 375 K rows, 4.8 M entries), 16
-// right-hand sides, 6 levels: 138 us at four CTAs per SM, 134 at one or two,
+// right-hand sides, 6 levels: 144 us at four CTAs per SM, 135 at one or two,
 // against 220 for the CSR rows read from L2 into the same window; 6 matrices
-// of 300-3000 rows, 4 right-hand sides, 4 levels (resident): 21 against 47.
-// Two ring chunks measure as three do (139 and 142 us at two CTAs per SM)
-// and leave room for one group instead of two at four CTAs (142 and 167).
+// of 300-3000 rows, 4 right-hand sides, 4 levels (resident): 21 against 45.
+// Two ring chunks measure as three do at two CTAs per SM and leave room for
+// one group instead of two at four CTAs (142 and 167 us).
 constexpr int kBpRing = 2;  // chunks in flight per warp
 __host__ __device__ constexpr int bp_chunk_pairs(int lpr) { return lpr == 1 ? 2 : lpr == 2 ? 4 : lpr; }
 __host__ __device__ constexpr int bp_chunk_bytes(int lpr) { return bp_chunk_pairs(lpr) * (32 / lpr) * 16; }

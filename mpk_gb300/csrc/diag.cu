@@ -35,9 +35,9 @@
 // hand-over (release after the barrier 1.5-3 K, the neighbours' flags 1-2 K,
 // the halo 1 K).  Against the general wavefront, which reads every index and
 // its columns through L1 (us): 128^3 1/deg k = 8 228 / 249; 100^2 1/deg k = 4
-// 8.2 / 15.1; 9-point FP64 1400 x 1300 k = 8 266 / 293; double-float 1/deg
-// 101 x 97 x 89 k = 8 79 / 105; mixed FP32 120 x 110 x 100 k = 8 68 / 141, BF16
-// 9-point 701 x 699 k = 4 17.7 / 40.9.
+// 8.2 / 15.2; 9-point FP64 1400 x 1300 k = 8 266 / 293; double-float 1/deg
+// 101 x 97 x 89 k = 8 79 / 105; mixed FP32 120 x 110 x 100 k = 8 68 / 140, BF16
+// 9-point 701 x 699 k = 4 17.4 / 40.8.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
