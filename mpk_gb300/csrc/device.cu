@@ -741,6 +741,10 @@ __device__ __forceinline__ int ld_off(const short *p) {
   return (int)__ldg(p);
 }
 
+// How fused multiply-adds go over a matrix's rows (plan_wave_impl chooses):
+// without integer products; with them, most rows of up to 8 entries; longer.
+enum RowKind { kRowsPlain, kRowsShort, kRowsLong };
+
 // One row's sum over its entries (CSR order): the row's int16 offsets are
 // RS apart (32: per-lane layout, a constant after inlining; 1: a slice's
 // shared list), values and int32 columns 32 apart.  The first 8 entries have
@@ -748,14 +752,31 @@ __device__ __forceinline__ int ld_off(const short *p) {
 // product runs on the integer pipes (128^3 1/deg, 8 levels: 270 -> 249 us;
 // 9-point diffusion 1400 x 1300 in FP64, whose rows of 9 used to load entry by
 // entry: 360 -> 293 us).  The others go four at a time: written out for fused
-// multiply-adds with values, where the compiler's own unrolling spills, and
-// left to the compiler otherwise, where it is the faster (us before this loop
-// was unrolled / 8 loads in flight only / so, 6 levels: 27-point 31^3 with
-// values 67 / 76 / 65, 40 entries a row, 5000 rows 61 / 63 / 47; 1/deg 27-point
-// 40^3, separate rounding, 85 / 88 / 76, 64^3 244 / 227 / 171).
-template <int ARITH, bool VALUED, bool REL, bool STAGE>
+// multiply-adds with values in matrices of longer rows, where the compiler's
+// own unrolling spills, and left to the compiler otherwise, unrolled with
+// separate rounding (us before this loop was written so / 8 loads in flight
+// only / so, 6 levels: 27-point 31^3 with values 67 / 76 / 65, 40 entries a row,
+// 5000 rows 61 / 63 / 47; 1/deg 27-point 40^3, separate rounding, 85 / 88 / 76,
+// 64^3 244 / 227 / 171; for 7-point rows written out costs 3 %).
+// KIND: RowKind.
+template <int ARITH, bool VALUED, bool REL, bool STAGE, int KIND>
 __device__ __forceinline__ double fp_row(int len, int RS, double cf, const short *cr, const int *cc,
                                          const double *cv, const double *xb, const double *src) {
+  constexpr bool INT = KIND != kRowsPlain;
+  if (!INT && !VALUED && len <= 8) {
+    double x[8], v[8], s = 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      if (u < len) {
+        x[u] = REL ? xb[ld_off<STAGE>(cr + RS * u)] : src[__ldg(cc + 32 * u)];
+        v[u] = cf;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+      if (u < len) s = row_term<ARITH>(s, v[u], x[u]);
+    return s;
+  }
   double x[8], v[8];
 #pragma unroll
   for (int u = 0; u < 8; u++) {
@@ -765,13 +786,13 @@ __device__ __forceinline__ double fp_row(int len, int RS, double cf, const short
     }
   }
   double s = 0.0;
-  if (len > 0) s = row_first<ARITH>(v[0], x[0]);
+  if (len > 0) s = INT ? row_first<ARITH>(v[0], x[0]) : row_term<ARITH>(0.0, v[0], x[0]);
 #pragma unroll
   for (int u = 1; u < 8; u++)
     if (u < len) s = u < kIntTerms ? row_next<ARITH>(s, v[u], x[u]) : row_term<ARITH>(s, v[u], x[u]);
   auto x_at = [&](int t) { return REL ? xb[ld_off<STAGE>(cr + RS * t)] : src[__ldg(cc + 32L * t)]; };
   int t = 8;
-  if (VALUED && ARITH != MPKG_ARITH_SEPARATE) {
+  if (VALUED && ARITH != MPKG_ARITH_SEPARATE && KIND != kRowsShort) {
     for (; t + 4 <= len; t += 4) {
       double y[4], w[4];
 #pragma unroll
@@ -784,8 +805,10 @@ __device__ __forceinline__ double fp_row(int len, int RS, double cf, const short
     }
 #pragma unroll 1
     for (; t < len; t++) s = row_term<ARITH>(s, __ldg(cv + 32L * t), x_at(t));
-  } else {
+  } else if (ARITH == MPKG_ARITH_SEPARATE) {
 #pragma unroll 4
+    for (; t < len; t++) s = row_term<ARITH>(s, VALUED ? __ldg(cv + 32L * t) : cf, x_at(t));
+  } else {
     for (; t < len; t++) s = row_term<ARITH>(s, VALUED ? __ldg(cv + 32L * t) : cf, x_at(t));
   }
   return s;
@@ -853,7 +876,7 @@ constexpr int kWaveXGroups = 8;  // host execution: CTA groups that copy x in tu
 // A warp computes one 32-row slice; CTA row ranges start on slices.  The
 // previous level is read from vv: every address of it is fresh in this
 // launch, so L1 holds no stale copy.
-template <int ARITH, bool VALUED, bool REL, bool STAGE, bool UNI>
+template <int ARITH, bool VALUED, bool REL, bool STAGE, bool UNI, int KIND>
 __global__ void __launch_bounds__(256, 4) wave_kernel(WaveArgs a) {
   extern __shared__ __align__(16) unsigned char wave_smem[];
   __shared__ int s_abort;
@@ -912,7 +935,7 @@ __global__ void __launch_bounds__(256, 4) wave_kernel(WaveArgs a) {
       const double *cv = a.sval + e0;
       const double *xb = src + i;
       // the stride is the constant 32 unless the plan compresses offsets
-      const double s = fp_row<ARITH, VALUED, REL, STAGE>(len, UNI ? (uni ? 1 : 32) : 32, cf, cr, cc, cv, xb, src);
+      const double s = fp_row<ARITH, VALUED, REL, STAGE, KIND>(len, UNI ? (uni ? 1 : 32) : 32, cf, cr, cc, cv, xb, src);
       __stcs(dst + i, s);
       if (hdst) hdst[i] = s;
     }
@@ -2110,6 +2133,7 @@ struct mpkg_plan {
   int wave_grid = 0;
   bool wave_rel = false;
   bool wave_uni = false;  // pattern-compressed offsets (plans with matrix values)
+  int wave_kind = kRowsShort;  // RowKind
   DiagArgs dg{};          // rows on a few diagonals: the diagonal wavefront
   bool dg_on = false;
   int dg_form = 0, dg_w = 0, dg_mode = 0, dg_threads = 0, dg_irregular = 0;
@@ -2393,10 +2417,15 @@ void *wave_kernel_ptr(const mpkg_plan *p) {
   if (p->arith == MPKG_ARITH_DF64)                                                                            \
     return p->valued ? (void *)wave_df_kernel<true, REL, ST, UN> : (void *)wave_df_kernel<false, REL, ST, UN>; \
   if (p->arith == MPKG_ARITH_SEPARATE)                                                                        \
-    return p->valued ? (void *)wave_kernel<MPKG_ARITH_SEPARATE, true, REL, ST, UN>                            \
-                     : (void *)wave_kernel<MPKG_ARITH_SEPARATE, false, REL, ST, UN>;                          \
-  return p->valued ? (void *)wave_kernel<MPKG_ARITH_FMA, true, REL, ST, UN>                                   \
-                   : (void *)wave_kernel<MPKG_ARITH_FMA, false, REL, ST, UN>;
+    return p->valued ? (void *)wave_kernel<MPKG_ARITH_SEPARATE, true, REL, ST, UN, kRowsShort>                \
+                     : (void *)wave_kernel<MPKG_ARITH_SEPARATE, false, REL, ST, UN, kRowsShort>;              \
+  if (!ST && p->wave_kind == kRowsPlain)                                                                      \
+    return p->valued ? (void *)wave_kernel<MPKG_ARITH_FMA, true, REL, ST, UN, ST ? kRowsShort : kRowsPlain>   \
+                     : (void *)wave_kernel<MPKG_ARITH_FMA, false, REL, ST, UN, ST ? kRowsShort : kRowsPlain>; \
+  if (p->valued && p->wave_kind == kRowsLong)                                                                 \
+    return (void *)wave_kernel<MPKG_ARITH_FMA, true, REL, ST, UN, kRowsLong>;                                 \
+  return p->valued ? (void *)wave_kernel<MPKG_ARITH_FMA, true, REL, ST, UN, kRowsShort>                       \
+                   : (void *)wave_kernel<MPKG_ARITH_FMA, false, REL, ST, UN, kRowsShort>;
   if (rel && stage && uni) { MPKG_WK(true, true, true) }
   if (rel && stage) { MPKG_WK(true, true, false) }
   if (rel && uni) { MPKG_WK(true, false, true) }
@@ -3692,6 +3721,20 @@ int plan_wave_impl(int n, const int *ptr, const int *col, const double *val, int
     // shared offset lists pay where values dominate the bytes; the pattern
     // operator keeps the per-lane layout (fewer instructions per entry)
     p->wave_uni = rel && val != nullptr;
+    // Fused multiply-adds of short rows: the first product of a row on the
+    // integer pipes relieves the FP64 pipe while the columns are near (16-bit
+    // offsets) and two levels, the offsets and the values stay in L2.  Else
+    // (and unless the offsets are staged) the rows wait for their gathers or
+    // for memory, and its instructions only lengthen that (us, 5 levels, with /
+    // without: 1/deg 140^3 214 / 224, 150^3 287 / 279, 160^3 388 / 352, 180^3
+    // 549 / 516; 256 x 256 x 64 with values 475 / 430; 80^3 in random order 142 /
+    // 135, with values 167 / 158).  Rows of more than 8 entries keep it (9-point
+    // 2048^2 389 / 415).
+    int l2 = 0;
+    if (!rc && cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, p->device) != cudaSuccess)
+      rc = fail(kECuda, "device query failed");
+    const double bytes = 16.0 * n + (double)ptr[n] * ((rel ? 2 : 4) + (val ? 8 : 0));
+    p->wave_kind = ptr[n] > 8L * n ? kRowsLong : !rel || bytes > 0.7 * l2 ? kRowsPlain : kRowsShort;
   }
   int grid = 0;
   if (!rc)

@@ -39,3 +39,21 @@ def test_every_row_length(plan, n, uniform, valued, arith, gpu):
     p.exec_host(vv)
     want = O.mpk(a.ptr, a.col, a.val, x, k, O.MODE_FMA if arith == M.ARITH_FMA else O.MODE_SEPARATE)
     assert vv.tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("valued", [False, True])
+@pytest.mark.parametrize("order", ["beyond_l2", "random"])
+def test_rows_without_integer_products(order, valued, gpu):
+    """The general wavefront where rows wait for memory: levels beyond L2, and columns anywhere."""
+    if order == "random":
+        a = _matrix(70001, False, 4)
+        a = M.Csr(np.arange(0, 4 * a.n + 1, 4, dtype=np.int32), np.random.default_rng(1).integers(0, a.n, 4 * a.n).astype(np.int32))
+    else:
+        a = M.Csr.laplacian(150, 150, 151)
+    a = M.Csr(a.ptr, a.col, M.uniform(3, a.nnz) if valued else None)
+    k = 2
+    x = M.uniform(5, a.n)
+    vv = np.zeros((k + 1) * a.n)
+    vv[:a.n] = x
+    M.Plan.wave(a, k, ctas_per_sm=32).exec_host(vv)
+    assert vv.tobytes() == O.mpk(a.ptr, a.col, a.val, x, k, O.MODE_FMA).tobytes()

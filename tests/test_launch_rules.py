@@ -52,3 +52,19 @@ for mode in (M.BATCH_DEFAULT, M.BATCH_STAGED, M.BATCH_STAGED4):
     assert [(w[1], w[3]) for w in got] == info
     for kernel, blocks, threads, smem, _ in got:
         assert smem <= threads * 150  # of about 225 bytes a thread
+
+
+@pytest.mark.parametrize("make,kind", [
+    ("M.Csr.laplacian(140, 140, 138)", 1),  # columns near, the levels in L2
+    ("M.Csr.laplacian(150, 150, 151)", 0),  # beyond L2
+    ("M.Csr.laplacian(240, 240, 3)", 0),    # columns beyond 16 bits
+    ("M.Csr.diffusion(300, 301, 1, sigma=0.5, seed=1)", 1),
+])
+def test_general_wavefront_takes_integer_products_where_the_fp64_pipe_is_busy(make, kind, tmp_path):
+    log = fake_cudart.run(str(tmp_path), f"""
+a = {make}.pattern()
+p = M.Plan.wave(a, 1, ctas_per_sm=32)
+p.exec_device(1 << 20)
+""")
+    (kernel, *_), = _kernels(log, "wave_kernel")
+    assert f"Li{kind}EEEv" in kernel, kernel
