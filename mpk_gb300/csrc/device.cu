@@ -741,9 +741,9 @@ __device__ __forceinline__ int ld_off(const short *p) {
   return (int)__ldg(p);
 }
 
-// How fused multiply-adds go over a matrix's rows (plan_wave_impl chooses):
-// without integer products; with them, most rows of up to 8 entries; longer.
-enum RowKind { kRowsPlain, kRowsShort, kRowsLong };
+// How the row sums go over a matrix's rows (plan_wave_impl chooses): without
+// integer products; rows of up to 8 entries on average; of up to 28; longer.
+enum RowKind { kRowsPlain, kRowsShort, kRowsMid, kRowsLong };
 
 // One row's sum over its entries (CSR order): the row's int16 offsets are
 // RS apart (32: per-lane layout, a constant after inlining; 1: a slice's
@@ -751,13 +751,16 @@ enum RowKind { kRowsPlain, kRowsShort, kRowsLong };
 // all their loads in flight together, whatever the row's length; the first
 // product runs on the integer pipes (128^3 1/deg, 8 levels: 270 -> 249 us;
 // 9-point diffusion 1400 x 1300 in FP64, whose rows of 9 used to load entry by
-// entry: 360 -> 293 us).  The others go four at a time: written out for fused
-// multiply-adds with values in matrices of longer rows, where the compiler's
-// own unrolling spills, and left to the compiler otherwise, unrolled with
-// separate rounding (us before this loop was written so / 8 loads in flight
-// only / so, 6 levels: 27-point 31^3 with values 67 / 76 / 65, 40 entries a row,
-// 5000 rows 61 / 63 / 47; 1/deg 27-point 40^3, separate rounding, 85 / 88 / 76,
-// 64^3 244 / 227 / 171; for 7-point rows written out costs 3 %).
+// entry: 360 -> 293 us).  The others go as the kind of matrix has them fastest:
+// four at a time, written out, for fused multiply-adds with values in rows of
+// more than 8, where the compiler's own unrolling spills, and for separate
+// rounding with values in the longest; unrolled by four for separate rounding
+// in shorter ones; else as the compiler has it (us before the 8 loads ahead /
+// with them only / so, 6 levels: FMA with values, 27-point 31^3 67 / 76 / 65, 40
+// entries a row, 5000 rows 61 / 63 / 47; separate rounding, 1/deg 27-point 40^3
+// 85 / 88 / 76, 64^3 244 / 227 / 171.  40 entries a row, 5000 rows, separate
+// rounding, before / unrolled by four / so: with values 64 / 71 / 50, 1/deg 69 /
+// 47 / 44; left to the compiler, 7-point rows cost 2 %: 160^3 567 -> 579).
 // KIND: RowKind.
 template <int ARITH, bool VALUED, bool REL, bool STAGE, int KIND>
 __device__ __forceinline__ double fp_row(int len, int RS, double cf, const short *cr, const int *cc,
@@ -792,7 +795,8 @@ __device__ __forceinline__ double fp_row(int len, int RS, double cf, const short
     if (u < len) s = u < kIntTerms ? row_next<ARITH>(s, v[u], x[u]) : row_term<ARITH>(s, v[u], x[u]);
   auto x_at = [&](int t) { return REL ? xb[ld_off<STAGE>(cr + RS * t)] : src[__ldg(cc + 32L * t)]; };
   int t = 8;
-  if (VALUED && ARITH != MPKG_ARITH_SEPARATE && KIND != kRowsShort) {
+  constexpr bool kFours = VALUED && (ARITH == MPKG_ARITH_SEPARATE ? KIND == kRowsLong : KIND != kRowsShort);
+  if (kFours) {
     for (; t + 4 <= len; t += 4) {
       double y[4], w[4];
 #pragma unroll
@@ -805,7 +809,7 @@ __device__ __forceinline__ double fp_row(int len, int RS, double cf, const short
     }
 #pragma unroll 1
     for (; t < len; t++) s = row_term<ARITH>(s, __ldg(cv + 32L * t), x_at(t));
-  } else if (ARITH == MPKG_ARITH_SEPARATE) {
+  } else if (ARITH == MPKG_ARITH_SEPARATE && KIND == kRowsMid) {
 #pragma unroll 4
     for (; t < len; t++) s = row_term<ARITH>(s, VALUED ? __ldg(cv + 32L * t) : cf, x_at(t));
   } else {
@@ -2419,12 +2423,15 @@ void *wave_kernel_ptr(const mpkg_plan *p) {
   if (p->arith == MPKG_ARITH_DF64)                                                                            \
     return p->valued ? (void *)wave_df_kernel<true, REL, ST, UN> : (void *)wave_df_kernel<false, REL, ST, UN>; \
   if (p->arith == MPKG_ARITH_SEPARATE)                                                                        \
-    return p->valued ? (void *)wave_kernel<MPKG_ARITH_SEPARATE, true, REL, ST, UN, kRowsShort>                \
-                     : (void *)wave_kernel<MPKG_ARITH_SEPARATE, false, REL, ST, UN, kRowsShort>;              \
+    return p->wave_kind != kRowsLong                                                                          \
+               ? (p->valued ? (void *)wave_kernel<MPKG_ARITH_SEPARATE, true, REL, ST, UN, kRowsMid>           \
+                            : (void *)wave_kernel<MPKG_ARITH_SEPARATE, false, REL, ST, UN, kRowsMid>)         \
+           : !p->valued ? (void *)wave_kernel<MPKG_ARITH_SEPARATE, false, REL, ST, UN, kRowsShort>            \
+           : (void *)wave_kernel<MPKG_ARITH_SEPARATE, true, REL, ST, UN, kRowsLong>;                          \
   if (!ST && p->wave_kind == kRowsPlain)                                                                      \
     return p->valued ? (void *)wave_kernel<MPKG_ARITH_FMA, true, REL, ST, UN, ST ? kRowsShort : kRowsPlain>   \
                      : (void *)wave_kernel<MPKG_ARITH_FMA, false, REL, ST, UN, ST ? kRowsShort : kRowsPlain>; \
-  if (p->valued && p->wave_kind == kRowsLong)                                                                 \
+  if (p->valued && p->wave_kind >= kRowsMid)                                                                  \
     return (void *)wave_kernel<MPKG_ARITH_FMA, true, REL, ST, UN, kRowsLong>;                                 \
   return p->valued ? (void *)wave_kernel<MPKG_ARITH_FMA, true, REL, ST, UN, kRowsShort>                       \
                    : (void *)wave_kernel<MPKG_ARITH_FMA, false, REL, ST, UN, kRowsShort>;
@@ -3736,7 +3743,9 @@ int plan_wave_impl(int n, const int *ptr, const int *col, const double *val, int
     if (!rc && cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, p->device) != cudaSuccess)
       rc = fail(kECuda, "device query failed");
     const double bytes = 16.0 * n + (double)ptr[n] * ((rel ? 2 : 4) + (val ? 8 : 0));
-    p->wave_kind = ptr[n] > 8L * n ? kRowsLong : !rel || bytes > 0.7 * l2 ? kRowsPlain : kRowsShort;
+    p->wave_kind = ptr[n] > 28L * n ? kRowsLong
+                   : ptr[n] > 8L * n ? kRowsMid
+                   : arith == MPKG_ARITH_FMA && (!rel || bytes > 0.7 * l2) ? kRowsPlain : kRowsShort;
   }
   int grid = 0;
   if (!rc)

@@ -57,3 +57,25 @@ def test_rows_without_integer_products(order, valued, gpu):
     vv[:a.n] = x
     M.Plan.wave(a, k, ctas_per_sm=32).exec_host(vv)
     assert vv.tobytes() == O.mpk(a.ptr, a.col, a.val, x, k, O.MODE_FMA).tobytes()
+
+
+@pytest.mark.parametrize("n,uniform", [(3001, False), (20011, True)])
+@pytest.mark.parametrize("valued", [False, True])
+@pytest.mark.parametrize("arith", [M.ARITH_FMA, M.ARITH_SEPARATE])
+def test_longest_rows(n, uniform, valued, arith, gpu):
+    """The general wavefront where rows have more than 28 entries on average: every length from 20 to 65."""
+    i = np.arange(n)
+    length = 20 + (i // 32 % 46 if uniform else i % 46)
+    ptr = np.concatenate([[0], np.cumsum(length)]).astype(np.int32)
+    row = np.repeat(i, length)
+    first = np.clip(i - 3 * (length // 2), 0, n - 3 * 65)
+    col = (first[row] + 3 * (np.arange(ptr[-1]) - ptr[row])).astype(np.int32)
+    assert ptr[-1] > 28 * n
+    a = M.Csr(ptr, col, np.random.default_rng(6).normal(size=int(ptr[-1])) if valued else None)
+    k = 3
+    x = M.uniform(5, n)
+    vv = np.zeros((k + 1) * n)
+    vv[:n] = x
+    M.Plan.wave(a, k, arith=arith).exec_host(vv)
+    want = O.mpk(a.ptr, a.col, a.val, x, k, O.MODE_FMA if arith == M.ARITH_FMA else O.MODE_SEPARATE)
+    assert vv.tobytes() == want.tobytes()

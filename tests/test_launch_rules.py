@@ -68,3 +68,17 @@ p.exec_device(1 << 20)
 """)
     (kernel, *_), = _kernels(log, "wave_kernel")
     assert f"Li{kind}EEEv" in kernel, kernel
+
+
+@pytest.mark.parametrize("entries,valued,arith,code,kind", [
+    (8, True, "FMA", 0, 1), (9, True, "FMA", 0, 3), (28, True, "SEPARATE", 1, 2), (29, True, "SEPARATE", 1, 3),
+    (29, False, "SEPARATE", 1, 1), (28, False, "SEPARATE", 1, 2), (8, True, "SEPARATE", 1, 2), (29, True, "FMA", 0, 3),
+])
+def test_general_wavefront_goes_over_rows_by_their_average_length(entries, valued, arith, code, kind, tmp_path):
+    log = fake_cudart.run(str(tmp_path), f"""
+a = M.Csr.banded(5000, 128, {entries}, {entries}, seed=1)
+p = M.Plan.wave(a if {valued} else a.pattern(), 1, arith=M.ARITH_{arith})
+p.exec_device(1 << 20)
+""")
+    (kernel, *_), = _kernels(log, "wave_kernel")
+    assert f"wave_kernelILi{code}ELb{int(valued)}E" in kernel and f"Li{kind}EEEv" in kernel, kernel
