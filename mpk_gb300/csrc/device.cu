@@ -742,7 +742,8 @@ __device__ __forceinline__ int ld_off(const short *p) {
 }
 
 // How the row sums go over a matrix's rows (plan_wave_impl chooses): without
-// integer products; rows of up to 8 entries on average; of up to 28; longer.
+// integer products; rows of up to 8 entries on average; of up to 28; longer,
+// or one row that the level waits for.
 enum RowKind { kRowsPlain, kRowsShort, kRowsMid, kRowsLong };
 
 // One row's sum over its entries (CSR order): the row's int16 offsets are
@@ -3743,7 +3744,13 @@ int plan_wave_impl(int n, const int *ptr, const int *col, const double *val, int
     if (!rc && cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, p->device) != cudaSuccess)
       rc = fail(kECuda, "device query failed");
     const double bytes = 16.0 * n + (double)ptr[n] * ((rel ? 2 : 4) + (val ? 8 : 0));
-    p->wave_kind = ptr[n] > 28L * n ? kRowsLong
+    // One row of hundreds of entries holds up a level by about 0.1 us an entry,
+    // in which the others do 50000: its lane's loop decides then (100^2 mesh
+    // with one row of 200, 5 levels, by the average / so: FMA with values 196 /
+    // 115, separate rounding with values 223 / 130, 1/deg 122 / 114).
+    long longest = 0;
+    for (int i = 0; i < n; i++) longest = std::max<long>(longest, ptr[i + 1] - ptr[i]);
+    p->wave_kind = ptr[n] > 28L * n || (longest > 64 && longest * 50000 > ptr[n]) ? kRowsLong
                    : ptr[n] > 8L * n ? kRowsMid
                    : arith == MPKG_ARITH_FMA && (!rel || bytes > 0.7 * l2) ? kRowsPlain : kRowsShort;
   }

@@ -79,3 +79,24 @@ def test_longest_rows(n, uniform, valued, arith, gpu):
     M.Plan.wave(a, k, arith=arith).exec_host(vv)
     want = O.mpk(a.ptr, a.col, a.val, x, k, O.MODE_FMA if arith == M.ARITH_FMA else O.MODE_SEPARATE)
     assert vv.tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("length", [65, 203, 2000])
+@pytest.mark.parametrize("valued", [False, True])
+@pytest.mark.parametrize("arith", [M.ARITH_FMA, M.ARITH_SEPARATE])
+def test_one_long_row(length, valued, arith, gpu):
+    """The general wavefront over a mesh whose level waits for one row."""
+    a = M.Csr.laplacian(100, 100)
+    i = 5000
+    lo, hi = int(a.ptr[i]), int(a.ptr[i + 1])
+    ptr = a.ptr.astype(np.int64)
+    ptr[i + 1:] += length - (hi - lo)
+    col = np.concatenate([a.col[:lo], i - 30 + np.arange(length), a.col[hi:]])
+    a = M.Csr(ptr.astype(np.int32), col.astype(np.int32), np.random.default_rng(8).normal(size=len(col)) if valued else None)
+    k = 3
+    x = M.uniform(5, a.n)
+    vv = np.zeros((k + 1) * a.n)
+    vv[:a.n] = x
+    M.Plan.wave(a, k, arith=arith, ctas_per_sm=32).exec_host(vv)
+    want = O.mpk(a.ptr, a.col, a.val, x, k, O.MODE_FMA if arith == M.ARITH_FMA else O.MODE_SEPARATE)
+    assert vv.tobytes() == want.tobytes()

@@ -82,3 +82,20 @@ p.exec_device(1 << 20)
 """)
     (kernel, *_), = _kernels(log, "wave_kernel")
     assert f"wave_kernelILi{code}ELb{int(valued)}E" in kernel and f"Li{kind}EEEv" in kernel, kernel
+
+
+@pytest.mark.parametrize("nx,length,long", [(100, 64, False), (100, 65, True), (300, 200, True), (2000, 65, False)])
+@pytest.mark.parametrize("arith,code", [("SEPARATE", 1), ("FMA", 0)])
+def test_general_wavefront_with_one_long_row(nx, length, long, arith, code, tmp_path):
+    log = fake_cudart.run(str(tmp_path), f"""
+a = M.Csr.laplacian({nx}, {nx})
+i = a.n // 2
+ptr, cut = a.ptr.astype(np.int64), slice(a.ptr[i], a.ptr[i + 1])
+col = np.concatenate([a.col[:cut.start], np.arange(i - 30, i - 30 + {length}), a.col[cut.stop:]])
+ptr[i + 1:] += {length} - (cut.stop - cut.start)
+a = M.Csr(ptr.astype(np.int32), col.astype(np.int32), np.ones(len(col)))
+p = M.Plan.wave(a, 1, arith=M.ARITH_{arith}, ctas_per_sm=32)
+p.exec_device(1 << 20)
+""")
+    (kernel, *_), = _kernels(log, "wave_kernel")
+    assert f"wave_kernelILi{code}ELb1E" in kernel and ("Li3EEEv" in kernel) == long, kernel
